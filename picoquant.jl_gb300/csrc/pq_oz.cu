@@ -7,27 +7,40 @@
 // Scaling.  Every row m of A (over K, per batch index) gets the power of two
 // 2^ea[m] with every |Re|, |Im| of the row below it (frexp exponent of the row
 // maximum); likewise every column n of B gets 2^eb[n].  A scaled value
-// x = a 2^-ea in (-1, 1) is cut into five slices on fixed grids
+// x = a 2^-ea in (-1, 1) is cut into slices, and the products of A's slice i
+// and B's slice j are accumulated by level i + j into three FP32 accumulators
+// per real output (Cr, Ci): level 0, level 1 and the rest.
+//
+// Complex64 results of PQ_PREC_OZAKI (kHalf): three fp16 slices, s0 on a grid of
+// 2^-8 (or 2^-7, below), s1 on one 12 bits finer, s2 the rest with 11 bits, so
+// x - (s0 + s1 + s2) is below 2^-33 (2^-32); 8 of the 9 products (all but the
+// 2^-40-sized s2 t2).  Level 0 sums 2K products of multiples of 2^-16 of size at
+// most 1: with 8 bits in s0 and t0 it fits the 24-bit significand exactly for K
+// <= 128, with 7 and 8 for K <= 256, with 7 and 7 for K <= 512, so the tensor
+// core never drops a bit of it.  Level 1 is on a grid of 2^-28 .. 2^-26 and
+// about 2^-5 in size for rows without structure, exact as well; where it is
+// larger its truncation is below 2^-28 of the level-0 sums that come with it.
+// The split's error, at most 2^-31 K of the scales and near 2^-32 of the result
+// on random pairs, is far below the complex64 rounding (3.5e-8 of max |C|
+// either way), so 8 products give what five bf16 slices gave with 15: the pair
+// M = 2^18, N = K = 256 takes 1.0 ms instead of 1.47.
+//
+// Complex128 results keep five bf16 slices
 //   s0 = rint(x 2^7) 2^-7,  s_i = rint((x - s0 - .. - s_{i-1}) 2^{7(i+1)}) 2^{-7(i+1)}
 // (|s0| <= 1, |s_i| <= 2^{-7i-1}), each an integer of at most 8 bits times a
 // power of two, hence exact in bf16; x - (s0 + .. + s4) is below 2^-36, so a
-// value 2^-10 below its row maximum still keeps 26 significant bits.
-//
-// Products.  s_i t_j is an integer multiple of 2^{-7(i+j+2)} of magnitude at
-// most 2^{-7(i+j)}.  The 15 slice pairs with i + j <= 4 are accumulated by
-// level l = i + j into three accumulators per real output (Cr, Ci):
+// value 2^-10 below its row maximum still keeps 26 significant bits.  s_i t_j is
+// an integer multiple of 2^{-7(i+j+2)} of magnitude at most 2^{-7(i+j)}; the 15
+// slice pairs with i + j <= 4 are accumulated:
 //   level 0   (0,0)             multiples of 2^-14, |sum| <= 2K
 //   level 1   (0,1) (1,0)       multiples of 2^-21, |sum| <= 4K 2^-8
 //   levels 2-4 (the other 12)   |sum| <= 2^-14 relative
-// For K <= 512 the level-0 and level-1 sums fit the 24-bit FP32 significand
-// on their grids, so the tensor core accumulates them EXACTLY (its rounding
-// of an accumulation never drops a bit); only the small levels 2-4 round
-// (truncation, about 2^-30 relative after K).  The result is
+// For K <= 512 the level-0 and level-1 sums are exact in FP32; only the small
+// levels 2-4 round (truncation, about 2^-30 relative after K).  The result is
 // (L0 + L1 + L2) 2^(ea+eb) rounded once to the output type, so the error is
 // the output rounding plus the dropped pairs and slice residuals, at most
-// 2^-33 K 2^(ea+eb) per component.  (Dropping level 4 -- four slices, ten
-// pairs -- was measured to double the amplitude error of deep circuits:
-// their rows span many binades.)
+// 2^-33 K 2^(ea+eb) per component.  (Four 7-bit slices, ten pairs, double the
+// amplitude error of deep circuits: their rows span many binades.)
 //   Cr = Ar.Br + (-Ai).Bi   (the negation is the MMA's negate-A bit)
 //   Ci = Ar.Bi + Ai.Br
 //
@@ -50,16 +63,16 @@
 //   k_oz_gemm       persistent, one CTA per SM over 64 x TN complex output
 //                   tiles (TN = 128, or 64 / 32 / 16 for narrow pairs; a pair
 //                   whose A side is the narrow one runs as B x A):
-//     warp 0       producer: cp.async.bulk of B's 10 plane tiles of one
+//     warp 0       producer: cp.async.bulk of B's plane tiles of one
 //                  16-deep K tile into the shared-memory ring;
-//     warp 1       TMEM owner and MMA issuer: 30 tcgen05.mma (kind::f16,
-//                  bf16) per K tile into three TN-column accumulators (levels
-//                  0, 1, 2-4); narrow tiles (TN <= 64) alternate between two
-//                  such sets, so a tile's MMAs do not wait for the epilogue
-//                  of the one before; 16-wide tiles issue one MMA per A slice
-//                  i against B's slices 0 .. 4-i side by side (N = 16 (5-i),
-//                  10 MMAs per K tile), each slice pair into its own exact
-//                  16-column region;
+//     warp 1       TMEM owner and MMA issuer: 16 tcgen05.mma (kind::f16; 30
+//                  for five slices) per K tile into three TN-column
+//                  accumulators (levels 0, 1, rest); narrow tiles (TN <= 64)
+//                  alternate between two such sets, so a tile's MMAs do not
+//                  wait for the epilogue of the one before; 16-wide tiles
+//                  issue one MMA per A slice i against the B slices it meets
+//                  side by side, each slice pair into its own 16-column
+//                  region;
 //     warps 2-9    A converters: gather A's 64 x 16 complex values of the K
 //                  tile through its index map straight from HBM (the group's
 //                  next K tile in flight while this one is sliced), slice
@@ -75,6 +88,7 @@
 // Every mbarrier wait is bounded; on expiry the kernel records an error in the
 // context's status word and runs to the end (TMEM is always released).
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -98,28 +112,42 @@ constexpr int kExpZero = -4096;                  // exponent of an all-zero row
 constexpr int64_t kMaxK = 512;                   // exact level-0/1 sums up to this K
 
 // Tile width N: 128 for general pairs, 64 / 32 / 16 for narrow ones.
-// Slices per real value: 5 for PQ_PREC_OZAKI (15 slice pairs, i + j <= 4),
-// 4 for PQ_PREC_OZAKI4 (10 pairs, i + j <= 3), 3 for PQ_PREC_3XBF16 (6
-// pairs, i + j <= 2).
-template <int NSL>
+// Split of a real value: kHalf for PQ_PREC_OZAKI with complex64 results (three
+// fp16 slices, the 8 pairs but (2,2)); bf16 slices for the others: 5 for
+// PQ_PREC_OZAKI with complex128 results (15 slice pairs, i + j <= 4), 4 for
+// PQ_PREC_OZAKI4 (10 pairs, i + j <= 3), 3 for PQ_PREC_3XBF16 (6 pairs,
+// i + j <= 2).
+constexpr int kHalf = 8;
+template <int S>
 struct Sl {
-  static_assert(NSL == 5 || NSL == 4 || NSL == 3, "slice count");
-  static constexpr int planes = 2 * NSL;  // per operand: Re s0.., Im s0..
-  static constexpr int pairs = NSL == 5 ? 15 : (NSL == 4 ? 10 : 6);
+  static_assert(S == kHalf || S == 5 || S == 4 || S == 3, "split");
+  static constexpr bool half = S == kHalf;
+  static constexpr int n = half ? 3 : S;      // slices
+  static constexpr int planes = 2 * n;        // per operand: Re s0.., Im s0..
+  static constexpr int pairs = half ? 8 : (S == 5 ? 15 : (S == 4 ? 10 : 6));
+  // slices 0 .. met(i) - 1 of B meet slice i of A
+  __host__ __device__ static constexpr int met(int i) { return half ? (i < 2 ? 3 : 2) : n - i; }
 };
+// kHalf: scaled values are held times 2^kHalfUp, so that the lowest bits of
+// the third slice stay in fp16's range.
+constexpr int kHalfUp = 15;
+// Bits of the first slice (a grid of 2^-bits): with a + b bits and K terms of
+// two real products, a level-0 sum is at most 2K on a grid of 2^-(a+b), which
+// fits the 24-bit significand while a + b + 1 + log2 K <= 24.
+__host__ __device__ constexpr int first_bits(int64_t k, int side) { return k <= (side == 0 ? 128 : 256) ? 8 : 7; }
 
-template <int TN, int NSL>
+template <int TN, int S>
 struct OzCfg {
-  static constexpr int kBTile = TN * TK;                                   // bf16 per B plane tile
-  static constexpr uint32_t b_bytes = Sl<NSL>::planes * kBTile * 2;        // B planes of one K tile
-  static constexpr uint32_t stage_bytes = NSL * kStackBytes + b_bytes;
-  static constexpr int stages = (TN == 128 && NSL >= 4) ? 3 : 4;
-  // 16-wide tiles: one MMA per A slice i against B slices 0 .. NSL-1-i side
-  // by side (N = 16 (NSL - i)), every slice pair in its own TMEM region
+  static constexpr int kBTile = TN * TK;                                   // 16-bit values per B plane tile
+  static constexpr uint32_t b_bytes = Sl<S>::planes * kBTile * 2;          // B planes of one K tile
+  static constexpr uint32_t stage_bytes = Sl<S>::n * kStackBytes + b_bytes;
+  static constexpr int stages = Sl<S>::half ? (TN == 128 ? 5 : 6) : ((TN == 128 && S >= 4) ? 3 : 4);
+  // 16-wide tiles: one MMA per A slice i against B slices 0 .. met(i)-1 side
+  // by side (N = 16 met(i)), every slice pair in its own TMEM region
   static constexpr bool narrow = TN == 16;
-  // accumulator columns of one tile: three levels of TN columns, or the
-  // NSL (NSL + 1) / 2 pair regions of 16 columns
-  static constexpr int set_cols = narrow ? 8 * NSL * (NSL + 1) : 3 * TN;
+  // accumulator columns of one tile: three levels of TN columns, or the pair
+  // regions of 16 columns
+  static constexpr int set_cols = narrow ? 16 * Sl<S>::pairs : 3 * TN;
   // accumulator sets: two for TN <= 64, so that the MMAs of the next tile
   // run while the epilogue drains this one
   static constexpr int acc_sets = TN <= 64 ? 2 : 1;
@@ -129,31 +157,12 @@ struct OzCfg {
   static_assert(acc_sets * set_cols <= (int)tmem_cols && cw % 8 == 0 && stage_bytes % 1024 == 0, "tile width");
 };
 
-// First TMEM column of A slice i's region in a narrow tile: the regions of
-// slices 0 .. i-1 hold NSL, NSL - 1, ... pair blocks of 16 columns.
-template <int NSL>
+// First TMEM column of A slice i's region in a narrow tile.
+template <int S>
 __host__ __device__ constexpr int narrow_col(int i) {
-  return 16 * (i * NSL - i * (i - 1) / 2);
-}
-// The slice pairs of level >= 2, smallest level first: the p-th is
-// (rest_i, rest_level - rest_i); level l holds the l + 1 pairs i = 0 .. l.
-template <int NSL>
-__host__ __device__ constexpr int rest_level(int p) {
-  int l = NSL - 1;
-  while (p > l) {
-    p -= l + 1;
-    --l;
-  }
-  return l;
-}
-template <int NSL>
-__host__ __device__ constexpr int rest_i(int p) {
-  int l = NSL - 1;
-  while (p > l) {
-    p -= l + 1;
-    --l;
-  }
-  return p;
+  int c = 0;
+  for (int q = 0; q < i; ++q) c += 16 * Sl<S>::met(q);
+  return c;
 }
 
 // slice pairs, level 0 first, then level 1, then the higher levels (the
@@ -166,18 +175,24 @@ __host__ __device__ constexpr int rest_i(int p) {
 // three slices:
 //   i: 0 0 1 0 1 2
 //   j: 0 1 0 2 1 0
+// kHalf:
+//   i: 0 0 1 1 2 0 2 1
+//   j: 0 1 0 2 1 2 0 1
 // (4-bit fields, pair p in bits [4p, 4p + 4))
-template <int NSL>
+template <int S>
 __host__ __device__ constexpr int pair_i(int p) {
-  return (int)((NSL == 5 ? 0x210321043210100ull : (NSL == 4 ? 0x2103210100ull : 0x210100ull)) >> (4 * p)) & 15;
+  return (int)((S == kHalf ? 0x12021100ull
+                           : (S == 5 ? 0x210321043210100ull : (S == 4 ? 0x2103210100ull : 0x210100ull))) >>
+               (4 * p)) &
+         15;
 }
-template <int NSL>
+template <int S>
 __host__ __device__ constexpr int pair_j(int p) {
-  return (int)((NSL == 5 ? 0x12012301234010ull : (NSL == 4 ? 0x0120123010ull : 0x12010ull)) >> (4 * p)) & 15;
+  return (int)((S == kHalf ? 0x10212010ull
+                           : (S == 5 ? 0x12012301234010ull : (S == 4 ? 0x0120123010ull : 0x12010ull))) >>
+               (4 * p)) &
+         15;
 }
-
-__host__ __device__ constexpr int level_of(int p) { return p == 0 ? 0 : (p < 3 ? 1 : 2); }
-__host__ __device__ constexpr bool first_of_level(int p) { return p == 0 || p == 1 || p == 3; }
 
 template <typename T>
 struct Real;
@@ -321,7 +336,7 @@ void row_exponents(const T* A, const GemmDesc& d, int* ea, cudaStream_t s) {
   }
 }
 
-// The slices of x (|x| < 1 after scaling); every step is exact in R.
+// The bf16 slices of x (|x| < 1 after scaling); every step is exact in R.
 template <typename R, int NSL>
 __device__ __forceinline__ void slices(R x, float* s) {
   R r = x;
@@ -334,6 +349,33 @@ __device__ __forceinline__ void slices(R x, float* s) {
     g *= (R)128.0;
     gi *= (R)(1.0 / 128.0);
   }
+}
+// x rounded to a multiple of 2^e for |x| < 2^(e + 21), by adding and taking
+// off c = 1.5 2^(23 + e).
+__device__ __forceinline__ float round_grid(float x, float c) { return __fadd_rn(__fadd_rn(x, c), -c); }
+// The fp16 slices of x 2^kHalfUp (|x| < 1): s0 on the grid of c0, s1 on a grid
+// 2^-12 of it, s2 the rest (rounded to fp16's 11 bits when it is stored).
+// Exact but for that last rounding; |s1| is half a grid step of s0 (11 bits).
+__device__ __forceinline__ void half_slices(float x, float c0, float c1, float* s) {
+  s[0] = round_grid(x, c0);
+  const float r = x - s[0];
+  s[1] = round_grid(r, c1);
+  s[2] = r - s[1];
+}
+__device__ __forceinline__ void half_slices(double x, float c0, float c1, float* s) {
+  s[0] = round_grid((float)x, c0);
+  const double r = x - (double)s[0];
+  s[1] = round_grid((float)r, c1);
+  s[2] = (float)(r - (double)s[1]);
+}
+// The rounding constants of the first two slices for a first slice of `bits`.
+__device__ __forceinline__ float half_c0(int bits) { return 1.5f * __int_as_float((23 + kHalfUp - bits + 127) << 23); }
+__device__ __forceinline__ float half_c1(int bits) { return half_c0(bits) * (1.f / 4096.f); }
+// A slice as the 16-bit operand value (exact, kHalf's last slice rounded).
+template <int S>
+__device__ __forceinline__ uint16_t slice_bits(float v) {
+  if constexpr (Sl<S>::half) return __half_as_ushort(__float2half_rn(v));
+  return __bfloat16_as_ushort(__float2bfloat16_rn(v));
 }
 
 // 2^k as a float for -126 <= k <= 127.
@@ -352,15 +394,15 @@ __device__ __forceinline__ double scale_row(double x, int e, float2) { return ld
 // One plane tile (ROWS x 16) is shared by PARTS blocks (blockIdx.x = kt PARTS
 // + part), each slicing TILE / PARTS values: complex128 B is sliced in FP64,
 // whose GB300 rate is low, so the work is spread over many SMs.
-template <typename T, int ROWS, int NSL>
+template <int ROWS>
 __host__ __device__ constexpr int pack_parts() {
   return ROWS * TK / 256 > 0 ? ROWS * TK / 256 : 1;
 }
-template <typename T, int ROWS, int NSL>
-__global__ void __launch_bounds__(256) k_oz_pack(const T* __restrict__ X, __nv_bfloat16* __restrict__ planes,
+template <typename T, int ROWS, int S>
+__global__ void __launch_bounds__(256) k_oz_pack(const T* __restrict__ X, uint16_t* __restrict__ planes,
                                                  const __grid_constant__ GemmDesc d, int side, int64_t rows,
                                                  int64_t rtiles, int64_t ktiles, const int* __restrict__ e_in) {
-  constexpr int TILE = ROWS * TK, GROUPS = ROWS / 8, PARTS = pack_parts<T, ROWS, NSL>(), PER = TILE / PARTS;
+  constexpr int TILE = ROWS * TK, GROUPS = ROWS / 8, PARTS = pack_parts<ROWS>(), PER = TILE / PARTS, NSL = Sl<S>::n;
   __shared__ int64_t roff[ROWS];
   __shared__ int rexp[ROWS];
   __shared__ int64_t koff[TK];
@@ -384,7 +426,8 @@ __global__ void __launch_bounds__(256) k_oz_pack(const T* __restrict__ X, __nv_b
   __syncthreads();
   const int64_t zo = decode(z, d.nz, d.zdim, zstr);
   using R = typename Real<T>::R;
-  __nv_bfloat16* tile = planes + (((z * rtiles + rt) * ktiles + kt) * Sl<NSL>::planes) * (int64_t)TILE;
+  uint16_t* tile = planes + (((z * rtiles + rt) * ktiles + kt) * Sl<S>::planes) * (int64_t)TILE;
+  const float c0 = half_c0(first_bits(d.K, side)), c1 = half_c1(first_bits(d.K, side));
   for (int o = part * PER + threadIdx.x; o < (part + 1) * PER; o += blockDim.x) {
     // o = ((kc * GROUPS + g) * 8 + r8) * 8 + k8: core matrix (kc, g), row r8, K k8
     const int core = o >> 6, within = o & 63;
@@ -395,8 +438,13 @@ __global__ void __launch_bounds__(256) k_oz_pack(const T* __restrict__ X, __nv_b
     for (int i = 0; i < NSL; ++i) re[i] = im[i] = 0.f;
     if (roff[r] >= 0 && koff[k] >= 0 && rexp[r] != kExpZero) {
       const T v = X[zo + roff[r] + koff[k]];
-      slices<R, NSL>(scale2((R)v.x, -rexp[r]), re);
-      slices<R, NSL>(scale2((R)v.y, -rexp[r]), im);
+      if constexpr (Sl<S>::half) {
+        half_slices(scale2((R)v.x, kHalfUp - rexp[r]), c0, c1, re);
+        half_slices(scale2((R)v.y, kHalfUp - rexp[r]), c0, c1, im);
+      } else {
+        slices<R, NSL>(scale2((R)v.x, -rexp[r]), re);
+        slices<R, NSL>(scale2((R)v.y, -rexp[r]), im);
+      }
     }
     if constexpr (ROWS == 16) {
       // 16-wide tiles: per part (Re, Im) one block of the NSL slices side by
@@ -406,25 +454,25 @@ __global__ void __launch_bounds__(256) k_oz_pack(const T* __restrict__ X, __nv_b
 #pragma unroll
       for (int i = 0; i < NSL; ++i) {
         const int q = ((kc * (NSL * GROUPS) + i * GROUPS + g) * 8 + r8) * 8 + k8;
-        tile[0 * NSL * TILE + q] = __float2bfloat16_rn(re[i]);
-        tile[1 * NSL * TILE + q] = __float2bfloat16_rn(im[i]);
+        tile[0 * NSL * TILE + q] = slice_bits<S>(re[i]);
+        tile[1 * NSL * TILE + q] = slice_bits<S>(im[i]);
       }
     } else {
 #pragma unroll
       for (int i = 0; i < NSL; ++i) {
-        tile[(0 * NSL + i) * TILE + o] = __float2bfloat16_rn(re[i]);
-        tile[(1 * NSL + i) * TILE + o] = __float2bfloat16_rn(im[i]);
+        tile[(0 * NSL + i) * TILE + o] = slice_bits<S>(re[i]);
+        tile[(1 * NSL + i) * TILE + o] = slice_bits<S>(im[i]);
       }
     }
   }
 }
 
-template <int TN, int NSL>
+template <int TN, int S>
 struct alignas(1024) OzSmem {
-  unsigned char stage[OzCfg<TN, NSL>::stages][OzCfg<TN, NSL>::stage_bytes];  // A stacks, then B planes
+  unsigned char stage[OzCfg<TN, S>::stages][OzCfg<TN, S>::stage_bytes];  // A stacks, then B planes
   int64_t koff[kMaxK];                                                        // A's K offsets
-  uint64_t full[OzCfg<TN, NSL>::stages];
-  uint64_t empty[OzCfg<TN, NSL>::stages];
+  uint64_t full[OzCfg<TN, S>::stages];
+  uint64_t empty[OzCfg<TN, S>::stages];
   uint64_t accf[2];  // accumulator set b holds a finished tile
   uint64_t acce[2];  // the epilogue has read accumulator set b
   uint64_t drain;
@@ -457,15 +505,29 @@ __device__ __forceinline__ double combine(float l0, float l1, float l2, int ex, 
   return ldexp(((double)l0 + (double)l1) + (double)l2, ex);
 }
 
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);  // exact: slices have <= 8 bits
-  return *reinterpret_cast<const uint32_t*>(&v);
+// Two slice values (k, k + 1) as one 32-bit word of 16-bit operands.
+template <int S>
+__device__ __forceinline__ uint32_t pack_x2(float lo, float hi) {
+  if constexpr (Sl<S>::half) {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  } else {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);  // exact: slices have <= 8 bits
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
 }
 __device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
   asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// Four complex64 values (32 bytes, 32-byte aligned) of a read-only operand.
+__device__ __forceinline__ void ldg256(const void* p, float* v) {
+  asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+      : "l"(p));
 }
 
 // A values per converter thread and K tile: 8 for complex64 A (whole 16-byte
@@ -478,19 +540,29 @@ __host__ __device__ constexpr int conv_values() {
 // Generic-proxy shared-memory writes made visible to the tensor core's reads.
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-template <typename TA, typename TC, int TN, int NSL>
+// The ring position `by` stages on (by <= kStages), with its phase.
+template <int kStages>
+__device__ __forceinline__ void next_stage(int& s, uint32_t& ph, int by = 1) {
+  s += by;
+  if (s >= kStages) {
+    s -= kStages;
+    ph ^= 1u;
+  }
+}
+
+template <typename TA, typename TC, int TN, int S>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_oz_gemm(const TA* __restrict__ A, const __nv_bfloat16* __restrict__ pb, TC* __restrict__ C,
+    k_oz_gemm(const TA* __restrict__ A, const uint16_t* __restrict__ pb, TC* __restrict__ C,
               const __grid_constant__ GemmDesc d, const int64_t* __restrict__ cm_tab,
               const int64_t* __restrict__ cn_tab, const int* __restrict__ ea, const int* __restrict__ eb,
-              int64_t mtiles, int64_t ntiles, int64_t ktiles, int* status) {
-  using CF = OzCfg<TN, NSL>;
-  constexpr int kSlices = NSL, kPlanes = Sl<NSL>::planes, kPairs = Sl<NSL>::pairs;
+              int64_t mtiles, int64_t ntiles, int64_t ktiles, int kvec, int* status) {
+  using CF = OzCfg<TN, S>;
+  constexpr int kSlices = Sl<S>::n, kPlanes = Sl<S>::planes, kPairs = Sl<S>::pairs;
   constexpr int kStages = CF::stages;
   constexpr uint32_t kTmemCols = CF::tmem_cols;
   constexpr int kSets = CF::acc_sets;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  OzSmem<TN, NSL>& sm = *reinterpret_cast<OzSmem<TN, NSL>*>(smem_raw);
+  OzSmem<TN, S>& sm = *reinterpret_cast<OzSmem<TN, S>*>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t ntot = ntiles * mtiles * d.Z;
 
@@ -520,7 +592,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       int64_t g = 0;  // K tiles issued so far (all tiles)
       for (int64_t tile = blockIdx.x; tile < ntot && ok; tile += gridDim.x) {
         const int64_t nt = tile % ntiles, z = tile / (ntiles * mtiles);
-        const __nv_bfloat16* btile = pb + ((z * ntiles + nt) * ktiles) * (int64_t)(kPlanes * CF::kBTile);
+        const uint16_t* btile = pb + ((z * ntiles + nt) * ktiles) * (int64_t)(kPlanes * CF::kBTile);
         for (int64_t kt = 0; kt < ktiles; ++kt, ++g) {
           const int s = (int)(g % kStages);
           const uint32_t ph = (uint32_t)((g / kStages) & 1);
@@ -539,67 +611,93 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (!mbar_wait(&sm.full[i % kStages], (uint32_t)((i / kStages) & 1))) ok = false;
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_bf16(128, TN), idesc_neg = idesc_bf16(128, TN, true);
-      constexpr uint32_t ALBO = 24 * 128, BLBO = (TN / 8) * 128, SBO = 128;
-      int64_t g = 0;  // K tiles consumed so far
-      int64_t t = 0;  // tiles of this CTA
-      for (int64_t tile = blockIdx.x; tile < ntot && ok; tile += gridDim.x, ++t) {
-        // the epilogue has read this accumulator set's previous tile
-        const int b = (int)(t % kSets);
-        if (!mbar_wait(&sm.acce[b], (uint32_t)(((t / kSets) & 1) ^ 1))) {
+    // The whole warp runs the loop and waits, and one elected thread issues a
+    // K tile's MMAs and its commit, so that descriptors and predicates stay
+    // uniform: one MMA takes 64 cycles of the tensor core, and issued from a
+    // lane-0 branch with 64-bit descriptor sums they came 79-81 cycles apart
+    // (69 with this form).
+    constexpr uint32_t idesc = idesc_f16(Sl<S>::half, 128, TN), idesc_neg = idesc_f16(Sl<S>::half, 128, TN, true);
+    constexpr uint32_t ALBO = 24 * 128, BLBO = (TN / 8) * 128, SBO = 128;
+    int s = 0;       // ring stage and its phase
+    uint32_t ph = 0;
+    int64_t t = 0;   // tiles of this CTA
+    for (int64_t tile = blockIdx.x; tile < ntot && ok; tile += gridDim.x, ++t) {
+      // the epilogue has read this accumulator set's previous tile
+      const int b = (int)(t % kSets);
+      if (!__all_sync(0xffffffffu, mbar_wait(&sm.acce[b], (uint32_t)(((t / kSets) & 1) ^ 1)))) {
+        ok = false;
+        break;
+      }
+      fence_after();
+      for (int kt = 0; kt < (int)ktiles; ++kt) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&sm.full[s], ph))) {
           ok = false;
           break;
         }
         fence_after();
-        for (int64_t kt = 0; kt < ktiles; ++kt, ++g) {
-          const int s = (int)(g % kStages);
-          const uint32_t ph = (uint32_t)((g / kStages) & 1);
-          if (!mbar_wait(&sm.full[s], ph)) {
-            ok = false;
-            break;
-          }
-          fence_after();
-          const uint32_t sa = smem_u32(sm.stage[s]);
-          const uint64_t a0 = smem_desc(sa, ALBO, SBO);
-          if constexpr (CF::narrow) {
-            // B block per part: NSL slices x 2 row groups per K half
-            const uint64_t bn = smem_desc(sa + kSlices * kStackBytes, NSL * 2 * 128, SBO);
+        // shared-memory descriptors: the address field is in the low word, the
+        // rest is constant
+        const uint32_t sa = smem_u32(sm.stage[s]) >> 4;
+        constexpr uint32_t BOFF = (kSlices * kStackBytes) >> 4;
+        if constexpr (CF::narrow) {
+          // B block per part: the slices x 2 row groups per K half
+          constexpr uint32_t NLBO = kSlices * 2 * 128;
+          if (elect_one()) {
 #pragma unroll
-            for (int i = 0; i < NSL; ++i) {
-              const uint32_t dl = tmem + (uint32_t)(b * CF::set_cols + narrow_col<NSL>(i));
-              const uint64_t x1 = a0 + (uint64_t)((i * kStackBytes) >> 4);            // [Ar; Ai]
-              const uint64_t x2 = a0 + (uint64_t)((i * kStackBytes + 8 * 128) >> 4);  // [Ai; -Ar]
-              const uint64_t bi = bn + (uint64_t)((NSL * CF::kBTile * 2) >> 4);       // the Im block
-              const uint32_t acc = kt == 0 ? 0u : 1u;
-              mma_bf16(dl, x1, bn, idesc_bf16(128, 16 * (NSL - i)), acc);   // [Ar.Br ; Ai.Br], slices 0..NSL-1-i
-              mma_bf16(dl, x2, bi, idesc_bf16(128, 16 * (NSL - i), true), 1u);
+            for (int i = 0; i < kSlices; ++i) {
+              const uint32_t dl = tmem + (uint32_t)(b * CF::set_cols + narrow_col<S>(i));
+              const uint64_t x1 = desc_at(sa + ((i * kStackBytes) >> 4), ALBO, SBO);            // [Ar; Ai]
+              const uint64_t x2 = desc_at(sa + ((i * kStackBytes + 8 * 128) >> 4), ALBO, SBO);  // [Ai; -Ar]
+              const uint64_t br = desc_at(sa + BOFF, NLBO, SBO);
+              const uint64_t bi = desc_at(sa + BOFF + ((kSlices * CF::kBTile * 2) >> 4), NLBO, SBO);
+              // [Ar.Br ; Ai.Br], then [-Ai.Bi ; Ar.Bi], slices 0 .. met(i)-1 of B
+              mma_f16(dl, x1, br, idesc_f16(Sl<S>::half, 128, 16 * Sl<S>::met(i)), kt == 0 ? 0u : 1u);
+              mma_f16(dl, x2, bi, idesc_f16(Sl<S>::half, 128, 16 * Sl<S>::met(i), true), 1u);
             }
             mma_commit(&sm.empty[s]);
-            continue;
           }
-          const uint64_t b0 = smem_desc(sa + kSlices * kStackBytes, BLBO, SBO);
+          next_stage<kStages>(s, ph);
+          continue;
+        }
+        // The MMAs of one A operand follow each other: the first fills the
+        // tensor core's A buffer from shared memory, the others use it (an
+        // M = N = 128 MMA reads 8 KB in its 64 cycles, all of the SM's
+        // shared-memory bandwidth; with A kept, kHalf reads 88 KB per K tile
+        // instead of 128 KB: 7 % of the wide pair's time).
+        if (elect_one()) {
 #pragma unroll
-          for (int p = 0; p < kPairs; ++p) {
-            const int i = pair_i<NSL>(p), j = pair_j<NSL>(p);
-            const uint32_t acc = (kt == 0 && first_of_level(p)) ? 0u : 1u;
-            const uint32_t dl = tmem + (uint32_t)((b * 3 + level_of(p)) * TN);
-            const uint64_t x1 = a0 + (uint64_t)((i * kStackBytes) >> 4);             // [Ar; Ai]
-            const uint64_t x2 = a0 + (uint64_t)((i * kStackBytes + 8 * 128) >> 4);   // [Ai; -Ar]
-            const uint64_t br = b0 + (uint64_t)(((0 * kSlices + j) * CF::kBTile * 2) >> 4);
-            const uint64_t bi = b0 + (uint64_t)(((1 * kSlices + j) * CF::kBTile * 2) >> 4);
-            mma_bf16(dl, x1, br, idesc, acc);     // [Ar.Br ; Ai.Br]
-            mma_bf16(dl, x2, bi, idesc_neg, 1u);  // [-Ai.Bi ; Ar.Bi]
+          for (int i = 0; i < kSlices; ++i) {
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+              // part 0: [Ar; Ai] . Br = [Ar.Br ; Ai.Br]; part 1: [Ai; -Ar]
+              // with A negated . Bi = [-Ai.Bi ; Ar.Bi]
+              const uint64_t x = desc_at(sa + ((i * kStackBytes + part * 8 * 128) >> 4), ALBO, SBO);
+#pragma unroll
+              for (int j = 0; j < Sl<S>::met(i); ++j) {
+                // the first MMA into each level overwrites it
+                const uint32_t acc = (kt == 0 && i == 0 && part == 0 && j <= 2) ? 0u : 1u;
+                const uint32_t dl = tmem + (uint32_t)((b * 3 + (i + j < 2 ? i + j : 2)) * TN);
+                const uint64_t y = desc_at(sa + BOFF + (((part * kSlices + j) * CF::kBTile * 2) >> 4), BLBO, SBO);
+                const uint32_t id = part ? idesc_neg : idesc;
+                if (j == 0)
+                  mma_f16_a_fill(dl, x, y, id, acc);
+                else if (j + 1 < Sl<S>::met(i))
+                  mma_f16_a_use(dl, x, y, id, acc);
+                else
+                  mma_f16_a_lastuse(dl, x, y, id, acc);
+              }
+            }
           }
           mma_commit(&sm.empty[s]);  // smem stage free once these MMAs finish
         }
-        if (!ok) break;
-        mma_commit(&sm.accf[b]);  // tile accumulators ready for the epilogue
+        next_stage<kStages>(s, ph);
       }
-      // every MMA issued has finished once this arrives (TMEM is freed below)
-      mma_commit(&sm.drain);
-      if (!mbar_wait(&sm.drain, 0)) ok = false;
+      if (!ok) break;
+      if (elect_one()) mma_commit(&sm.accf[b]);  // tile accumulators ready for the epilogue
     }
+    // every MMA issued has finished once this arrives (TMEM is freed below)
+    if (elect_one()) mma_commit(&sm.drain);
+    if (!mbar_wait(&sm.drain, 0)) ok = false;
   } else if (warp < 2 + kConvWarps) {
     // converters: with NV values per thread and K tile, the converter warps
     // form NV / 4 groups that take alternate K tiles; thread ch of a group
@@ -614,13 +712,13 @@ __global__ void __launch_bounds__(kThreads, 1)
     using R = typename Real<TA>::R;
     // byte offset of (slice 0, block 0, row r, K value kq) in the stacks
     const uint32_t row_off = (uint32_t)((((kq >> 3) * 24 + (r >> 3)) * 8 + (r & 7)) * 16 + (kq & 7) * 2);
+    const float hc0 = half_c0(first_bits(d.K, 0)), hc1 = half_c1(first_bits(d.K, 0));
     // This CTA's K tiles form one sequence g = tile number * ktiles + kt; the
     // group takes g = grp, grp + H, ...  The next one's A values and row
     // exponent are loaded while this one is sliced, across tile boundaries
     // (a tile's rows and exponent are looked up once per tile).
     const int64_t ntl = blockIdx.x < ntot ? (ntot - 1 - blockIdx.x) / gridDim.x + 1 : 0;
     const int64_t items = ntl * ktiles;
-    int64_t ptl = -1;  // tile (number within this CTA) whose row pointer and exponent are cached
     const TA* prow = A;
     bool pm = false;
     int en = kExpZero;  // exponent of the prefetched K tile's row (a load in flight)
@@ -631,11 +729,25 @@ __global__ void __launch_bounds__(kThreads, 1)
       pm = m < d.M;
       en = pm ? ea[z * d.M + m] : kExpZero;
       prow = A + (pm ? decode(z, d.nz, d.zdim, d.zsa) + decode(m, d.nm, d.mdim, d.msa) : 0);
-      ptl = tl;
     };
     // zeros past the operand (and for rows outside it); an all-zero row's
     // values are zeros themselves, whatever its exponent
     auto load = [&](int64_t kt, TA* v) {
+      if constexpr (NV == 8) {
+        if (kvec) {  // every four values from a multiple of 4 are 32 aligned bytes
+          const int64_t k = kt * TK + kq;
+#pragma unroll
+          for (int q = 0; q < NV; q += 4) {
+            if (pm && k + q < d.K) {
+              ldg256(prow + sm.koff[k + q], reinterpret_cast<float*>(v + q));
+            } else {
+#pragma unroll
+              for (int u = 0; u < 4; ++u) v[q + u].x = v[q + u].y = 0;
+            }
+          }
+          return;
+        }
+      }
 #pragma unroll
       for (int q = 0; q < NV; ++q) {
         const int64_t k = kt * TK + kq + q;
@@ -648,36 +760,58 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     };
     TA nxt[NV];
+    // the next K tile to load: tile ptl (number within this CTA) and its K
+    // tile pkt, stepped without divisions
+    int64_t ptl = 0;
+    int pkt = grp;
+    auto settle = [&]() {
+      bool moved = false;
+      while (pkt >= (int)ktiles) {
+        pkt -= (int)ktiles;
+        ++ptl;
+        moved = true;
+      }
+      return moved;
+    };
     if (grp < items) {
-      row_info(grp / ktiles);
-      load(grp % ktiles, nxt);
+      settle();
+      row_info(ptl);
+      load(pkt, nxt);
     }
+    int s = grp;  // H <= 2 <= kStages
+    uint32_t ph = 0;
     for (int64_t gk = grp; gk < items && ok; gk += H) {
       const int e = en;
       TA cur[NV];
 #pragma unroll
       for (int q = 0; q < NV; ++q) cur[q] = nxt[q];
       if (gk + H < items) {  // in flight while this K tile is sliced
-        const int64_t gp = gk + H, tl = gp / ktiles;
-        if (tl != ptl) row_info(tl);
-        load(gp - tl * ktiles, nxt);
+        pkt += H;
+        if (settle()) row_info(ptl);
+        load(pkt, nxt);
       }
-      const float2 f = inv_scale(e != kExpZero ? e : 0);
+      const int up = Sl<S>::half ? kHalfUp : 0;
+      const float2 f = inv_scale((e != kExpZero ? e : 0) - up);
       {
-        const int s = (int)(gk % kStages);
-        const uint32_t ph = (uint32_t)((gk / kStages) & 1);
         uint32_t pr[kSlices][NV / 2], pim[kSlices][NV / 2];  // bf16 pairs (k, k + 1) of Ar, Ai
 #pragma unroll
         for (int q = 0; q < NV; q += 2) {
           float a0[kSlices], b0[kSlices], a1[kSlices], b1[kSlices];
-          slices<R, NSL>(scale_row((R)cur[q].x, e, f), a0);
-          slices<R, NSL>(scale_row((R)cur[q].y, e, f), b0);
-          slices<R, NSL>(scale_row((R)cur[q + 1].x, e, f), a1);
-          slices<R, NSL>(scale_row((R)cur[q + 1].y, e, f), b1);
+          if constexpr (Sl<S>::half) {
+            half_slices(scale_row((R)cur[q].x, e - up, f), hc0, hc1, a0);
+            half_slices(scale_row((R)cur[q].y, e - up, f), hc0, hc1, b0);
+            half_slices(scale_row((R)cur[q + 1].x, e - up, f), hc0, hc1, a1);
+            half_slices(scale_row((R)cur[q + 1].y, e - up, f), hc0, hc1, b1);
+          } else {
+            slices<R, kSlices>(scale_row((R)cur[q].x, e, f), a0);
+            slices<R, kSlices>(scale_row((R)cur[q].y, e, f), b0);
+            slices<R, kSlices>(scale_row((R)cur[q + 1].x, e, f), a1);
+            slices<R, kSlices>(scale_row((R)cur[q + 1].y, e, f), b1);
+          }
 #pragma unroll
           for (int i = 0; i < kSlices; ++i) {
-            pr[i][q / 2] = pack_bf16x2(a0[i], a1[i]);
-            pim[i][q / 2] = pack_bf16x2(b0[i], b1[i]);
+            pr[i][q / 2] = pack_x2<S>(a0[i], a1[i]);
+            pim[i][q / 2] = pack_x2<S>(b0[i], b1[i]);
           }
         }
         bool got = mbar_wait(&sm.empty[s], ph ^ 1);
@@ -704,6 +838,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.full[s]);
+        next_stage<kStages>(s, ph, H);
       }
     }
   } else {
@@ -756,6 +891,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const bool mrow = M.mrow;
       const int64_t base = M.base, c0 = M.c0;
       const int exa = M.exa;
+      constexpr int kDown = Sl<S>::half ? 2 * kHalfUp : 0;  // both operands' factor, taken off
       const int b = (int)(t % kSets);
       bool got = mbar_wait(&sm.accf[b], (uint32_t)((t / kSets) & 1));
       got = __all_sync(0xffffffffu, got);  // the TMEM loads below are warp-collective
@@ -799,7 +935,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int ebj = __shfl_sync(0xffffffffu, M.ebl[cc / 32], cc % 32);
             const long long cnj = __shfl_sync(0xffffffffu, M.cnl[cc / 32], cc % 32);
             if (mrow && c0 + cc < d.N) {
-              const int ex = exa + ebj;
+              const int ex = exa + ebj - kDown;
               const R val = (exa == kExpZero || ex < -2 * 1100) ? (R)0 : (R)scale_pow2(v[j], ex);
               Cr[2 * (base + cnj) + part] = val;
             }
@@ -813,35 +949,31 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t col = (uint32_t)(b * 3 * TN + h * CW + piece * PW);
         float l0[PW], l1[PW], l2[PW];
         if constexpr (CF::narrow) {
-          // the slice-pair regions (each an exact sum over K): level 0 =
-          // (0,0); level 1 = (0,1) + (1,0), exact; levels 2 .. NSL-1 summed
-          // in FP32, the smallest first, four regions per TMEM wait
+          // the slice-pair regions (each a sum over K of one pair): level 0 =
+          // (0,0); level 1 = (0,1) + (1,0); the others summed in FP32, the
+          // smallest first, four regions per TMEM wait
           static_assert(PW == 8, "narrow tiles: 8 columns per epilogue warp");
           const uint32_t rb = lane_base + (uint32_t)(b * CF::set_cols + h * CW + piece * PW);
           float t0[PW], t1[PW];
-          tmem_ld8(rb + narrow_col<NSL>(0), l0);
-          tmem_ld8(rb + narrow_col<NSL>(0) + 16, t0);
-          tmem_ld8(rb + narrow_col<NSL>(1), t1);
+          tmem_ld8(rb + narrow_col<S>(0), l0);
+          tmem_ld8(rb + narrow_col<S>(0) + 16, t0);
+          tmem_ld8(rb + narrow_col<S>(1), t1);
           tmem_wait_ld();
 #pragma unroll
           for (int q = 0; q < PW; ++q) {
             l1[q] = t0[q] + t1[q];
             l2[q] = 0.f;
           }
-          constexpr int NR = NSL * (NSL + 1) / 2 - 3;
 #pragma unroll
-          for (int p0 = 0; p0 < NR; p0 += 4) {
+          for (int p0 = 3; p0 < kPairs; p0 += 4) {
             float tb[4][PW];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-              if (p0 + u < NR)
-                tmem_ld8(rb + narrow_col<NSL>(rest_i<NSL>(p0 + u)) +
-                             16 * (rest_level<NSL>(p0 + u) - rest_i<NSL>(p0 + u)),
-                         tb[u]);
+              if (p0 + u < kPairs) tmem_ld8(rb + narrow_col<S>(pair_i<S>(p0 + u)) + 16 * pair_j<S>(p0 + u), tb[u]);
             tmem_wait_ld();
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-              if (p0 + u < NR)
+              if (p0 + u < kPairs)
 #pragma unroll
                 for (int q = 0; q < PW; ++q) l2[q] += tb[u][q];
           }
@@ -866,7 +998,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           const int ebj = __shfl_sync(0xffffffffu, M.ebl[cc / 32], cc % 32);
           const long long cnj = __shfl_sync(0xffffffffu, M.cnl[cc / 32], cc % 32);
           if (mrow && c0 + cc < d.N) {
-            const int ex = exa + ebj;
+            const int ex = exa + ebj - kDown;
             const R v = (exa == kExpZero || ex < -2 * 1100) ? (R)0 : combine(l0[j], l1[j], l2[j], ex, R());
             Cr[2 * (base + cnj) + part] = v;
           }
@@ -944,52 +1076,68 @@ bool needs_swap(const GemmDesc& d) {
 
 // B's column exponents (16 columns per block, 16 threads on each: B is the
 // small side, so its pass needs many blocks to be short), then its slices.
-template <typename T, int ROWS, int NSL>
-void prep_b(const void* X, __nv_bfloat16* planes, int* e, const GemmDesc& d, int64_t rtiles, int64_t kt,
+template <typename T, int ROWS, int S>
+void prep_b(const void* X, uint16_t* planes, int* e, const GemmDesc& d, int64_t rtiles, int64_t kt,
             cudaStream_t s) {
   k_oz_exp<T, 16><<<dim3((unsigned)ceil_div(d.N, 16), (unsigned)d.Z), 256, 0, s>>>((const T*)X, d, 1, d.N, e);
-  constexpr int parts = pack_parts<T, ROWS, NSL>();
-  k_oz_pack<T, ROWS, NSL><<<dim3((unsigned)(kt * parts), (unsigned)rtiles, (unsigned)d.Z), 256, 0, s>>>(
+  constexpr int parts = pack_parts<ROWS>();
+  k_oz_pack<T, ROWS, S><<<dim3((unsigned)(kt * parts), (unsigned)rtiles, (unsigned)d.Z), 256, 0, s>>>(
       (const T*)X, planes, d, 1, d.N, rtiles, kt, e);
 }
 
-template <typename T, int NSL>
-void prep_b_tn(const void* X, int tn, __nv_bfloat16* planes, int* e, const GemmDesc& d, int64_t rtiles, int64_t kt,
+template <typename T, int S>
+void prep_b_tn(const void* X, int tn, uint16_t* planes, int* e, const GemmDesc& d, int64_t rtiles, int64_t kt,
                cudaStream_t s) {
-  if (tn == 128) prep_b<T, 128, NSL>(X, planes, e, d, rtiles, kt, s);
-  else if (tn == 64) prep_b<T, 64, NSL>(X, planes, e, d, rtiles, kt, s);
-  else if (tn == 32) prep_b<T, 32, NSL>(X, planes, e, d, rtiles, kt, s);
-  else prep_b<T, 16, NSL>(X, planes, e, d, rtiles, kt, s);
+  if (tn == 128) prep_b<T, 128, S>(X, planes, e, d, rtiles, kt, s);
+  else if (tn == 64) prep_b<T, 64, S>(X, planes, e, d, rtiles, kt, s);
+  else if (tn == 32) prep_b<T, 32, S>(X, planes, e, d, rtiles, kt, s);
+  else prep_b<T, 16, S>(X, planes, e, d, rtiles, kt, s);
 }
 
-template <typename TA, typename TC, int TN, int NSL>
-cudaError_t oz_gemm_launch(const void* A, const __nv_bfloat16* pb, void* C, const GemmDesc& d, const int64_t* cm,
+// Whether the converters may read complex64 A as aligned 32-byte runs of four
+// K values: the fastest K mode has stride 1 and an extent that is a multiple of
+// 4 (so runs of 4 from a multiple of 4 never cross it), and every other stride
+// and the base keep the alignment.  Otherwise they read value by value, which
+// coalesces over rows when A's first M mode has stride 1.
+bool k_vector(const void* A, const GemmDesc& d) {
+  if (((uintptr_t)A & 31) || d.nk < 1 || d.ksa[0] != 1 || d.kdim[0] % 4) return false;
+  for (int i = 1; i < d.nk; ++i)
+    if (d.ksa[i] % 4) return false;
+  for (int i = 0; i < d.nm; ++i)
+    if (d.msa[i] % 4) return false;
+  for (int i = 0; i < d.nz; ++i)
+    if (d.zsa[i] % 4) return false;
+  return true;
+}
+
+template <typename TA, typename TC, int TN, int S>
+cudaError_t oz_gemm_launch(const void* A, const uint16_t* pb, void* C, const GemmDesc& d, const int64_t* cm,
                            const int64_t* cn, const int* ea, const int* eb, const OzLayout& L, int* status,
                            cudaStream_t s) {
-  static_assert(sizeof(OzSmem<TN, NSL>) + 1024 <= 232448, "shared memory layout exceeds 227 KiB");
-  const size_t smem = sizeof(OzSmem<TN, NSL>) + 1024;
+  static_assert(sizeof(OzSmem<TN, S>) + 1024 <= 232448, "shared memory layout exceeds 227 KiB");
+  const size_t smem = sizeof(OzSmem<TN, S>) + 1024;
   static bool attr = false;
   if (!attr) {
     cudaError_t e =
-        cudaFuncSetAttribute(k_oz_gemm<TA, TC, TN, NSL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_oz_gemm<TA, TC, TN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     attr = true;
   }
   const int64_t tiles = L.mt * L.nt * d.Z;
   const unsigned grid = (unsigned)std::min<int64_t>(tiles, sm_count());
-  k_oz_gemm<TA, TC, TN, NSL><<<grid, kThreads, smem, s>>>((const TA*)A, pb, (TC*)C, d, cm, cn, ea, eb, L.mt, L.nt, L.kt,
-                                                     status);
+  k_oz_gemm<TA, TC, TN, S><<<grid, kThreads, smem, s>>>((const TA*)A, pb, (TC*)C, d, cm, cn, ea, eb, L.mt, L.nt, L.kt,
+                                                        k_vector(A, d) ? 1 : 0, status);
   return cudaGetLastError();
 }
 
-template <typename TA, typename TC, int NSL>
-cudaError_t oz_gemm_tn(const void* A, const __nv_bfloat16* pb, void* C, const GemmDesc& d, const int64_t* cm,
+template <typename TA, typename TC, int S>
+cudaError_t oz_gemm_tn(const void* A, const uint16_t* pb, void* C, const GemmDesc& d, const int64_t* cm,
                        const int64_t* cn, const int* ea, const int* eb, const OzLayout& L, int* status,
                        cudaStream_t s) {
-  if (L.tn == 128) return oz_gemm_launch<TA, TC, 128, NSL>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
-  if (L.tn == 64) return oz_gemm_launch<TA, TC, 64, NSL>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
-  if (L.tn == 32) return oz_gemm_launch<TA, TC, 32, NSL>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
-  return oz_gemm_launch<TA, TC, 16, NSL>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+  if (L.tn == 128) return oz_gemm_launch<TA, TC, 128, S>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+  if (L.tn == 64) return oz_gemm_launch<TA, TC, 64, S>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+  if (L.tn == 32) return oz_gemm_launch<TA, TC, 32, S>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+  return oz_gemm_launch<TA, TC, 16, S>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
 }
 
 bool eligible_oriented(const GemmDesc& d) {
@@ -1008,10 +1156,10 @@ bool oz_eligible(const GemmDesc& d) { return eligible_oriented(needs_swap(d) ? s
 
 size_t oz_scratch_bytes(int slices, const GemmDesc& d) { return layout(needs_swap(d) ? swapped(d) : d, slices).total; }
 
-template <int NSL>
-static cudaError_t launch_oz_n(int ta, int tb, int tc, const void* A, const void* B, void* C, const GemmDesc& d,
+template <int S, typename TC>
+static cudaError_t launch_oz_n(int ta, int tb, const void* A, const void* B, void* C, const GemmDesc& d,
                                char* base, const OzLayout& L, int* status, cudaStream_t stream) {
-  auto* pb = (__nv_bfloat16*)(base + L.pb);
+  auto* pb = (uint16_t*)(base + L.pb);
   auto* cm = (int64_t*)(base + L.cm);
   auto* cn = (int64_t*)(base + L.cn);
   auto* ea = (int*)(base + L.ea);
@@ -1021,18 +1169,15 @@ static cudaError_t launch_oz_n(int ta, int tb, int tc, const void* A, const void
   else
     row_exponents((const float2*)A, d, ea, stream);
   if (tb == PQ_C128)
-    prep_b_tn<double2, NSL>(B, L.tn, pb, eb, d, L.nt, L.kt, stream);
+    prep_b_tn<double2, S>(B, L.tn, pb, eb, d, L.nt, L.kt, stream);
   else
-    prep_b_tn<float2, NSL>(B, L.tn, pb, eb, d, L.nt, L.kt, stream);
+    prep_b_tn<float2, S>(B, L.tn, pb, eb, d, L.nt, L.kt, stream);
   const int64_t idx_blocks = std::min<int64_t>(ceil_div(d.M + d.N, 256), 152 * 8);
   k_result_index<<<(unsigned)idx_blocks, 256, 0, stream>>>(d, cm, cn);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  if (ta == PQ_C128)
-    return tc == PQ_C128 ? oz_gemm_tn<double2, double2, NSL>(A, pb, C, d, cm, cn, ea, eb, L, status, stream)
-                         : oz_gemm_tn<double2, float2, NSL>(A, pb, C, d, cm, cn, ea, eb, L, status, stream);
-  return tc == PQ_C128 ? oz_gemm_tn<float2, double2, NSL>(A, pb, C, d, cm, cn, ea, eb, L, status, stream)
-                       : oz_gemm_tn<float2, float2, NSL>(A, pb, C, d, cm, cn, ea, eb, L, status, stream);
+  return ta == PQ_C128 ? oz_gemm_tn<double2, TC, S>(A, pb, C, d, cm, cn, ea, eb, L, status, stream)
+                       : oz_gemm_tn<float2, TC, S>(A, pb, C, d, cm, cn, ea, eb, L, status, stream);
 }
 
 cudaError_t launch_oz(int slices, int ta, int tb, int tc, const void* A, const void* B, void* C,
@@ -1047,9 +1192,19 @@ cudaError_t launch_oz(int slices, int ta, int tb, int tc, const void* A, const v
   const OzLayout L = layout(d, slices);
   if (!scratch || scratch_bytes < L.total) return cudaErrorInvalidValue;
   char* base = (char*)(((uintptr_t)scratch + 255) & ~(uintptr_t)255);
-  if (slices == 5) return launch_oz_n<5>(ta, tb, tc, A, B, C, d, base, L, status, stream);
-  if (slices == 4) return launch_oz_n<4>(ta, tb, tc, A, B, C, d, base, L, status, stream);
-  return launch_oz_n<3>(ta, tb, tc, A, B, C, d, base, L, status, stream);
+  // Five slices stay for complex128 results, where the split's own error (about
+  // 2^-34 of the scales) is what the caller sees; in a complex64 result it is
+  // far below the 2^-25 of the storage rounding with either split, and kHalf
+  // takes 8 slice products instead of 15.
+  const bool c128 = tc == PQ_C128;
+  if (slices == 5)
+    return c128 ? launch_oz_n<5, double2>(ta, tb, A, B, C, d, base, L, status, stream)
+                : launch_oz_n<kHalf, float2>(ta, tb, A, B, C, d, base, L, status, stream);
+  if (slices == 4)
+    return c128 ? launch_oz_n<4, double2>(ta, tb, A, B, C, d, base, L, status, stream)
+                : launch_oz_n<4, float2>(ta, tb, A, B, C, d, base, L, status, stream);
+  return c128 ? launch_oz_n<3, double2>(ta, tb, A, B, C, d, base, L, status, stream)
+              : launch_oz_n<3, float2>(ta, tb, A, B, C, d, base, L, status, stream);
 }
 
 }  // namespace pq

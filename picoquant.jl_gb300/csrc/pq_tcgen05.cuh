@@ -84,14 +84,28 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
   d |= (uint64_t)1 << 46;  // descriptor version for sm_100-family tcgen05
   return d;                // base offset 0, no swizzle (layout type 0)
 }
+// The same from an address in 16-byte units, for the low word alone.
+__device__ __forceinline__ uint64_t desc_at(uint32_t addr16, uint32_t lbo, uint32_t sbo) {
+  const uint32_t lo = addr16 | (lbo >> 4) << 16, hi = (sbo >> 4) | 1u << 14;
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+// One thread of a converged warp (the same one every time).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+  return e != 0;
+}
 // Instruction descriptors, FP32 accumulation, both operands K-major; bit 13
-// negates A.  kind::tf32: A/B format 2; kind::f16 with bf16 operands: 1.
+// negates A.  kind::tf32: A/B format 2; kind::f16: 0 for fp16 operands, 1 for
+// bf16 (both operands of one MMA alike).
 __host__ __device__ constexpr uint32_t idesc_tf32(int m, int n, bool neg_a = false) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((neg_a ? 1u : 0u) << 13) | ((uint32_t)(n >> 3) << 17) |
          ((uint32_t)(m >> 4) << 24);
 }
-__host__ __device__ constexpr uint32_t idesc_bf16(int m, int n, bool neg_a = false) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((neg_a ? 1u : 0u) << 13) | ((uint32_t)(n >> 3) << 17) |
+__host__ __device__ constexpr uint32_t idesc_f16(bool half, int m, int n, bool neg_a = false) {
+  return (1u << 4) | ((half ? 0u : 1u) << 7) | ((half ? 0u : 1u) << 10) | ((neg_a ? 1u : 0u) << 13) | ((uint32_t)(n >> 3) << 17) |
          ((uint32_t)(m >> 4) << 24);
 }
 __device__ __forceinline__ void mma_tf32(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -101,11 +115,35 @@ __device__ __forceinline__ void mma_tf32(uint32_t dtmem, uint64_t adesc, uint64_
           dtmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
-__device__ __forceinline__ void mma_bf16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                        uint32_t accumulate) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
-          dtmem),
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dtmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+// The same MMA, keeping A in the tensor core's buffer (fill), taking it from
+// there and keeping it (use), or taking it for the last time (lastuse): for
+// consecutive MMAs with the same A operand.
+__device__ __forceinline__ void mma_f16_a_fill(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                        uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16.collector::a::fill [%0], %1, %2, %3, p;\n}\n" ::"r"(dtmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+__device__ __forceinline__ void mma_f16_a_use(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                        uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16.collector::a::use [%0], %1, %2, %3, p;\n}\n" ::"r"(dtmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+__device__ __forceinline__ void mma_f16_a_lastuse(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                        uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16.collector::a::lastuse [%0], %1, %2, %3, p;\n}\n" ::"r"(dtmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 // Arrives on `bar` once every tcgen05 operation issued so far by this thread

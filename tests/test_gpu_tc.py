@@ -464,3 +464,42 @@ def test_ozaki4_c128_plan_amplitude(pq, O):
     assert abs(amp - ref) / 2.0 ** -8 < 1e-7
     plan.close()
     be.close()
+
+
+@pytest.mark.parametrize("order", ["mk", "km", "k4", "k6"])
+@pytest.mark.parametrize("k,n", [(24, 128), (96, 8), (144, 136), (264, 72), (504, 24)])
+def test_ozaki_half_split(pq, O, order, k, n):
+    """Complex64 results (three fp16 slices): the first slice's 8 or 7 bits on
+    either side of K = 128 and 256, ragged K tiles, 16- to 128-wide tiles, A
+    contiguous along M, along all of K, and in K runs of 4 (32-byte loads) and 6
+    (value by value).  Random rows spanning 12 binades: the scheme's bound.
+    Equal entries c (1 + i): every level-0 sum is at its largest, 2K c^2, and
+    must be exact; level 1 is 2^-7 of it at most and is truncated at most
+    4 ceil(K / 16) <= 128 times by 2^-24 of itself, 2^-24 in all, so with the
+    final rounding (2^-24) the result is within 2^-23 of the product."""
+    rng = np.random.default_rng(k + n)
+    m = 1400  # at least 2^20 multiply-adds in every case
+    for data in ("rows", "equal"):
+        if data == "rows":
+            A = (rand(rng, (m, k)) * np.exp2(-rng.integers(0, 13, size=(m, k)))).astype(np.complex64)
+            B = rand(rng, (k, n)).astype(np.complex64)
+        else:
+            A = np.full((m, k), (1 + 1j) * (1 - 2.0 ** -13), dtype=np.complex64)
+            B = np.full((k, n), (1 + 1j) * (1 - 2.0 ** -12), dtype=np.complex64)
+        be = ozaki_backend(pq)
+        if order == "mk":
+            got, nl = run(be, A, [-1, 1], B, [1, -2])
+        elif order == "km":
+            got, nl = run(be, A.T, [1, -1], B, [1, -2])
+        else:
+            r = 4 if order == "k4" else 6
+            T = A.reshape(m, k // r, r).transpose(2, 0, 1)  # fastest K run first, then M
+            got, nl = run(be, T, [2, -1, 1], B.reshape(k // r, r, n), [1, 2, -2])
+        be.close()
+        assert nl == OZ_LAUNCHES
+        A, B = A.astype(np.complex128), B.astype(np.complex128)
+        ref = A @ B
+        if data == "rows":
+            assert np.all(np.abs(got - ref) <= ozaki_bound(A, B, ref))
+        else:
+            assert np.max(np.abs(got - ref)) <= 2.0 ** -23 * np.max(np.abs(ref))

@@ -86,6 +86,46 @@ __device__ __forceinline__ void cfma(float2& acc, float2 a, float2 b) {
   acc.y = fmaf(a.y, b.x, acc.y);
 }
 
+// Programmatic dependent launch: a kernel launched with launch_pdl may start
+// while the kernel before it in the stream still runs.  pdl_wait() returns once
+// that kernel has finished and its writes are visible; every thread of such a
+// kernel calls it before it reads anything a kernel writes, or writes anything.
+// pdl_trigger() lets the next launch_pdl kernel start (it still waits).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... KA, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, KA(args)...);
+}
+
+// Two FP32 values in one 64-bit register pair, and the multiply-add on both.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2_dup(float x) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float2 f2_get(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+
 // Kahan-compensated complex accumulator: partial sums of short K chunks are
 // accumulated in FP32 and folded into (s, c) here, so the accumulation error
 // grows with the chunk length rather than with K.

@@ -212,3 +212,35 @@ def test_block_fused_amplitudes_4x5(pq, O, prec):
     ref = O.statevector(n, gates)[[O.amplitude_index(b) for b in bits]]
     scale = np.sqrt(np.mean(np.abs(ref) ** 2))
     assert np.max(np.abs(got - ref)) / scale < (2e-5 if prec == 1 else 1e-11)
+
+
+@pytest.mark.parametrize("first,m,last,n", [(4, 4099, 1, 5), (2, 4099, 3, 16), (6, 4099, 2, 7), (3, 4100, 5, 1),
+                                            (8, 5000, 2, 9), (16, 4096, 1, 16), (12, 40000, 1, 3), (1, 4097, 16, 2)])
+def test_skinny_complex64_runs(pq, first, m, last, n):
+    """Complex64 operands, the large one's fastest mode contracted in runs of
+    ``first``: 32-, 16- and 8-byte loads, odd rows and columns, K = first *
+    last up to 16, in both operand orders.  Every real part is the difference
+    and every imaginary part the sum of K-term FP32 dot products, so each is
+    within (K + 2) 2^-24 of the sum of absolute products, a complex result
+    within twice that of sum |x||w|."""
+    rng = np.random.default_rng(first * 100 + last)
+    k = first * last
+
+    def crand(*s):
+        return (rng.standard_normal(s) + 1j * rng.standard_normal(s)).astype(np.complex64)
+
+    X, W = crand(first, m, last), crand(first, last, n)
+    ref = np.einsum("fml,fln->mn", X.astype(np.complex128), W.astype(np.complex128))
+    bound = 2 * (k + 2) * 2.0 ** -24 * np.einsum("fml,fln->mn", np.abs(X), np.abs(W))
+    be = pq.GB300Backend(pq.PREC_C64, small_elems=0)
+    for swap in (False, True):
+        be.save_tensor_data("x", X)
+        be.save_tensor_data("w", W)
+        if swap:
+            be.contract_tensors("w", [1, 2, -2], "x", [1, -1, 2], "c")
+        else:
+            be.contract_tensors("x", [1, -1, 2], "w", [1, 2, -2], "c")
+        got = be.load_tensor_data("c")
+        got = got.T if swap else got
+        assert np.all(np.abs(got - ref) <= bound)
+    be.close()

@@ -36,108 +36,186 @@ using namespace pq;
 
 namespace {
 
-constexpr int kSvThreads = 256;
+constexpr int kSvThreads = 128;
 constexpr int kSvMaxQ = 4;
 constexpr int kSvMaxDim = 1 << kSvMaxQ;
-constexpr int64_t kSvFibersPerThread = 2;  // fibers per thread per block (on average)
+// Blocks of one launch: as many as fit the SMs at once (6 of 128 threads at 80
+// registers), so that the table lookups at a block's start are paid once.  With
+// a block per 512 fibers (11 rounds of blocks) they were half the time of a
+// launch over 2^23.6 amplitudes.
+constexpr int64_t kSvBlocks = 152 * 6;
 
 struct SvOp {
   float2* state;      // the circuit's state, 2^n complex64
   const float2* mat;  // 2^k x 2^k complex64, element (out, in) at out + in 2^k
   int64_t rows;       // 2^(n - k) fibers
   int k;
-  int q[kSvMaxQ];     // bit positions of the block's qubits, bit i of a fiber index <-> q[i]
-  int qs[kSvMaxQ];    // the same positions in ascending order
+  int q[kSvMaxQ];     // bit positions of the block's qubits, ascending; bit i of a fiber index <-> q[i]
 };
 
 // The fibers [first, rows) step `stride` of one block pass with D = 2^k
 // amplitudes per fiber (specialised per k: every thread of a CUDA block works
 // on the same table entry, so the branch on k is uniform).
 struct SvQubits {
-  int q[kSvMaxQ], qs[kSvMaxQ];
+  int q[kSvMaxQ];
 };
 
-template <int D>
-__device__ __forceinline__ void sv_pass(float2* __restrict__ S, const float2* __restrict__ U, const SvQubits Q,
-                                        int64_t first, int64_t rows, int64_t stride) {
+// V adjacent amplitudes (V * 8 bytes, aligned to them).
+template <int V>
+__device__ __forceinline__ void load_adj(const float2* p, float2* a) {
+  if constexpr (V == 4) {
+    float* f = reinterpret_cast<float*>(a);
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7])
+                 : "l"(p));
+  } else if constexpr (V == 2) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    a[0] = make_float2(v.x, v.y);
+    a[1] = make_float2(v.z, v.w);
+  } else {
+    a[0] = *p;
+  }
+}
+template <int V>
+__device__ __forceinline__ void store_adj(float2* p, const float2* a) {
+  if constexpr (V == 4)
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(a[0].x), "f"(a[0].y), "f"(a[1].x),
+                 "f"(a[1].y), "f"(a[2].x), "f"(a[2].y), "f"(a[3].x), "f"(a[3].y)
+                 : "memory");
+  else if constexpr (V == 2)
+    *reinterpret_cast<float4*>(p) = make_float4(a[0].x, a[0].y, a[1].x, a[1].y);
+  else
+    *p = a[0];
+}
+
+// U: columns of the block's matrix, entries (out, out + 1) of input c as (re,
+// re', im, im') at U[c * D / 2 + out / 2].  Two outputs per multiply-add
+// (fma.rn.f32x2): with one, the issue slots bound the 4-qubit passes.
+// V amplitudes of a fiber are adjacent in memory: 2 with qubit 0 in the block, 4
+// with qubits 0 and 1 (loaded one by one, every 8 bytes of such a fiber are a
+// sector of their own: 83 us against 45 for a launch over the same amplitudes).
+template <int D, int V>
+__device__ __forceinline__ void sv_pass(float2* __restrict__ S, const ulonglong2* __restrict__ U, const SvQubits Q,
+                                        uint32_t first, uint32_t rows, uint32_t stride) {
   constexpr int k = D == 2 ? 1 : (D == 4 ? 2 : (D == 8 ? 3 : 4));
-  constexpr int G = D < 4 ? D : 4;  // outputs per group (the matrix is read a group of rows at a time)
+  constexpr int G = D < 4 ? D / 2 : 2;  // output pairs per group (the matrix is read a group of rows at a time)
   // offset of amplitude c of a fiber relative to its base (states have at
-  // most 2^31 amplitudes, so offsets fit 32 bits)
+  // most 2^31 amplitudes, so indices fit 32 bits)
   auto off = [&](int c) {
-    int o = 0;
+    uint32_t o = 0;
 #pragma unroll
-    for (int i = 0; i < k; ++i) o += ((c >> i) & 1) << Q.q[i];
+    for (int i = 0; i < k; ++i) o += (uint32_t)((c >> i) & 1) << Q.q[i];
     return o;
   };
-  for (int64_t r = first; r < rows; r += stride) {
+  for (uint32_t r = first; r < rows; r += stride) {
     // base index: r with a zero bit inserted at each block position (ascending)
-    int64_t base = r;
+    uint32_t base = r;
 #pragma unroll
     for (int i = 0; i < k; ++i) {
-      const int p = Q.qs[i];
-      base = ((base >> p) << (p + 1)) | (base & ((int64_t(1) << p) - 1));
+      const int p = Q.q[i];
+      const uint32_t lo = base & ((1u << p) - 1);
+      base = ((base - lo) << 1) | lo;
     }
+    float2* P = S + base;
     float2 a[D];
 #pragma unroll
-    for (int c = 0; c < D; ++c) a[c] = S[base + off(c)];
+    for (int c = 0; c < D; c += V) load_adj<V>(P + off(c), a + c);
+    F2 ax[D], ay[D];
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+      ax[c] = f2_dup(a[c].x);
+      ay[c] = f2_dup(a[c].y);
+    }
     // not unrolled: the matrix entries are read from shared memory per group
     // instead of being hoisted into registers
 #pragma unroll 1
-    for (int c0 = 0; c0 < D; c0 += G) {
-      float2 acc[G];
+    for (int c0 = 0; c0 < D; c0 += 2 * G) {
+      F2 rr[G], ii[G], ri[G];  // sums of re re, im im and re im + im re
 #pragma unroll
-      for (int j = 0; j < G; ++j) acc[j] = make_float2(0.f, 0.f);
+      for (int q = 0; q < G; ++q) rr[q] = ii[q] = ri[q] = 0;
 #pragma unroll
       for (int ci = 0; ci < D; ++ci) {
 #pragma unroll
-        for (int j = 0; j < G; ++j) cfma(acc[j], a[ci], U[c0 + j + ci * D]);
+        for (int q = 0; q < G; ++q) {
+          const ulonglong2 u = U[ci * (D / 2) + c0 / 2 + q];
+          rr[q] = f2_fma(ax[ci], u.x, rr[q]);
+          ii[q] = f2_fma(ay[ci], u.y, ii[q]);
+          ri[q] = f2_fma(ax[ci], u.y, ri[q]);
+          ri[q] = f2_fma(ay[ci], u.x, ri[q]);
+        }
+      }
+      float2 o[2 * G];
+#pragma unroll
+      for (int q = 0; q < G; ++q) {
+        const float2 p = f2_get(rr[q]), m = f2_get(ii[q]), y = f2_get(ri[q]);
+        o[2 * q] = make_float2(p.x - m.x, y.x);
+        o[2 * q + 1] = make_float2(p.y - m.y, y.y);
       }
 #pragma unroll
-      for (int j = 0; j < G; ++j) S[base + off(c0 + j)] = acc[j];
+      for (int q = 0; q < 2 * G; q += V) store_adj<V>(P + off(c0 + q), o + q);
     }
   }
 }
 
-__global__ void __launch_bounds__(kSvThreads)
+__global__ void __launch_bounds__(kSvThreads, 6)
     k_sv_group(const SvOp* __restrict__ ops, const int64_t* __restrict__ blk, int nops) {
-  __shared__ float2 U[kSvMaxDim * kSvMaxDim];
-  __shared__ int s_op;
-  if (threadIdx.x == 0) {
-    // the entry owning this block: the last one with blk[entry] <= blockIdx.x
-    int lo = 0, hi = nops - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) / 2;
-      if (blk[mid] <= (int64_t)blockIdx.x)
-        lo = mid;
-      else
-        hi = mid - 1;
+  __shared__ __align__(16) float U[kSvMaxDim * kSvMaxDim / 2][4];
+  __shared__ SvOp s_op;
+  __shared__ int64_t s_blk[2];
+  // the entry owning this block: the one with blk[entry] <= blockIdx.x <
+  // blk[entry + 1], looked at by all threads at once
+  for (int t = threadIdx.x; t < nops; t += blockDim.x) {
+    const int64_t b0 = blk[t], b1 = blk[t + 1];
+    if (b0 <= (int64_t)blockIdx.x && (int64_t)blockIdx.x < b1) {
+      s_op = ops[t];
+      s_blk[0] = b0;
+      s_blk[1] = b1;
     }
-    s_op = lo;
   }
   __syncthreads();
-  const int o_id = s_op;
-  const int k = ops[o_id].k;
+  const int k = s_op.k;
   const int D = 1 << k;
-  const float2* mat = ops[o_id].mat;
-  for (int t = threadIdx.x; t < D * D; t += blockDim.x) U[t] = mat[t];
-  __syncthreads();
-  float2* S = ops[o_id].state;
-  const int64_t rows = ops[o_id].rows;
+  const float2* mat = s_op.mat;
+  for (int t = threadIdx.x; t < D * D; t += blockDim.x) {
+    const float2 v = mat[t];
+    const int out = t & (D - 1), in = t >> k, e = in * (D / 2) + out / 2;
+    U[e][out & 1] = v.x;
+    U[e][2 + (out & 1)] = v.y;
+  }
   SvQubits Q;
 #pragma unroll
-  for (int i = 0; i < kSvMaxQ; ++i) {
-    Q.q[i] = ops[o_id].q[i];
-    Q.qs[i] = ops[o_id].qs[i];
-  }
-  const int64_t stride = (blk[o_id + 1] - blk[o_id]) * kSvThreads;
-  const int64_t first = ((int64_t)blockIdx.x - blk[o_id]) * kSvThreads + threadIdx.x;
+  for (int i = 0; i < kSvMaxQ; ++i) Q.q[i] = s_op.q[i];
+  __syncthreads();
+  float2* S = s_op.state;
+  const uint32_t rows = (uint32_t)s_op.rows;
+  const uint32_t stride = (uint32_t)(s_blk[1] - s_blk[0]) * kSvThreads;
+  const uint32_t first = (uint32_t)((int64_t)blockIdx.x - s_blk[0]) * kSvThreads + threadIdx.x;
+  const ulonglong2* M = reinterpret_cast<const ulonglong2*>(U);
+  // everything above reads tables that no kernel writes; the states are the
+  // previous launch's, whose blocks these may have joined on the SM
+  pdl_wait();
+  pdl_trigger();
+  const int adj = Q.q[0] != 0 ? 1 : (k >= 2 && Q.q[1] == 1 ? 4 : 2);
+#define SV_CASE(D)                                                \
+  if (adj == 4)                                                   \
+    sv_pass<D, 4>(S, M, Q, first, rows, stride);                  \
+  else if (adj == 2)                                              \
+    sv_pass<D, 2>(S, M, Q, first, rows, stride);                  \
+  else                                                            \
+    sv_pass<D, 1>(S, M, Q, first, rows, stride);                  \
+  break
   switch (k) {
-    case 1: sv_pass<2>(S, U, Q, first, rows, stride); break;
-    case 2: sv_pass<4>(S, U, Q, first, rows, stride); break;
-    case 3: sv_pass<8>(S, U, Q, first, rows, stride); break;
-    default: sv_pass<16>(S, U, Q, first, rows, stride); break;
+    case 1:
+      if (adj == 2)
+        sv_pass<2, 2>(S, M, Q, first, rows, stride);
+      else
+        sv_pass<2, 1>(S, M, Q, first, rows, stride);
+      break;
+    case 2: SV_CASE(4);
+    case 3: SV_CASE(8);
+    default: SV_CASE(16);
   }
+#undef SV_CASE
 }
 
 // |0...0> in every state of a chunk: the used arena zeroed beforehand, then
@@ -217,7 +295,9 @@ cudaError_t issue(pq_svbatch* b) {
     k_sv_init<<<(c.nstates + 255) / 256, 256, 0, s>>>(b->arena, b->d_soff + c.soff0, c.nstates);
     for (int l = c.launch0; l < c.launch0 + c.nlaunch; ++l) {
       const Launch& L = b->launches[l];
-      k_sv_group<<<(unsigned)L.blocks, kSvThreads, 0, s>>>(b->d_ops + L.op0, b->d_blk + L.blk0, L.nops);
+      if ((e = launch_pdl(k_sv_group, dim3((unsigned)L.blocks), dim3(kSvThreads), 0, s, (const SvOp*)(b->d_ops + L.op0),
+                          (const int64_t*)(b->d_blk + L.blk0), L.nops)) != cudaSuccess)
+        return e;
     }
     if (c.namp)
       k_sv_gather<<<(unsigned)((c.namp + 255) / 256), 256, 0, s>>>(b->arena, b->d_idx + c.amp0, c.namp,
@@ -306,8 +386,27 @@ int pq_svbatch_create(pq_ctx* c, int n_circ, const int32_t* n_qubits, const int3
   std::vector<SvOp> ops;
   std::vector<int64_t> blk, soff, idx;
   std::vector<float2> mats((size_t)mat_first[nblk_total]);
-  for (int64_t t = 0; t < mat_first[nblk_total]; ++t)
-    mats[t] = make_float2((float)block_mats[2 * t], (float)block_mats[2 * t + 1]);
+  // each block's qubits in ascending order, its matrix permuted to match: bit j
+  // of the new index is bit perm[j] of the given one
+  std::vector<int> sorted_q((size_t)q_first[nblk_total]);
+  for (int64_t j = 0; j < nblk_total; ++j) {
+    const int k = block_k[j], D = 1 << k;
+    const int32_t* q = block_qubits + q_first[j];
+    int perm[kSvMaxQ] = {0, 1, 2, 3};
+    std::sort(perm, perm + k, [&](int x, int y) { return q[x] < q[y]; });
+    for (int i = 0; i < k; ++i) sorted_q[q_first[j] + i] = q[perm[i]];
+    auto given = [&](int c) {
+      int g = 0;
+      for (int i = 0; i < k; ++i) g |= ((c >> i) & 1) << perm[i];
+      return g;
+    };
+    const double* src = block_mats + 2 * mat_first[j];
+    for (int in = 0; in < D; ++in)
+      for (int out = 0; out < D; ++out) {
+        const int g = given(out) + given(in) * D;
+        mats[mat_first[j] + out + in * D] = make_float2((float)src[2 * g], (float)src[2 * g + 1]);
+      }
+  }
   std::vector<int64_t> amp_pos(n_circ, 0);  // where circuit i's amplitudes land in the gathered output
   int64_t arena_elems = 0;
   size_t p = 0;
@@ -347,6 +446,11 @@ int pq_svbatch_create(pq_ctx* c, int n_circ, const int32_t* n_qubits, const int3
       L.op0 = (int)ops.size();
       L.blk0 = (int64_t)blk.size();
       int64_t nb = 0;
+      // blocks in proportion to the amplitudes an entry moves, at least one,
+      // no more than one fiber per thread needs
+      double total = 0;
+      for (int i : members)
+        if (s < n_blocks[i]) total += (double)(int64_t(1) << n_qubits[i]);
       for (size_t m = 0; m < members.size(); ++m) {
         const int i = members[m];
         if (s >= n_blocks[i]) continue;
@@ -357,13 +461,12 @@ int pq_svbatch_create(pq_ctx* c, int n_circ, const int32_t* n_qubits, const int3
         op.rows = int64_t(1) << (n_qubits[i] - op.k);
         op.state = nullptr;  // arena + base, fixed below once the arena exists
         op.mat = reinterpret_cast<const float2*>(mat_first[j]);  // element offset, fixed below
-        for (int t = 0; t < op.k; ++t) op.q[t] = op.qs[t] = block_qubits[q_first[j] + t];
-        std::sort(op.qs, op.qs + op.k);
+        for (int t = 0; t < op.k; ++t) op.q[t] = sorted_q[q_first[j] + t];
         op.state = reinterpret_cast<float2*>(base[m]);
         ops.push_back(op);
         blk.push_back(nb);
-        nb += std::max<int64_t>(1, (op.rows + kSvThreads * kSvFibersPerThread - 1) /
-                                       (kSvThreads * kSvFibersPerThread));
+        const int64_t share = (int64_t)((double)kSvBlocks * (double)(int64_t(1) << n_qubits[i]) / total);
+        nb += std::max<int64_t>(1, std::min(share, (op.rows + kSvThreads - 1) / kSvThreads));
       }
       blk.push_back(nb);
       L.nops = (int)ops.size() - L.op0;

@@ -88,3 +88,38 @@ def test_svbatch_rejects_bad_input(pq):
     assert np.allclose(got, [1 / np.sqrt(2), 1 / np.sqrt(2)], atol=1e-7)
     sb.close()
     be.close()
+
+
+@pytest.mark.parametrize("n,qs", [(1, [1]), (2, [2, 1]), (2, [2]), (5, [1]), (5, [2, 1]), (5, [1, 3]), (6, [4, 1, 2]),
+                                  (6, [3, 2, 5]), (4, [4, 2, 1, 3]), (7, [1, 7, 2, 4]), (9, [6, 1, 9, 3]),
+                                  (11, [5, 11, 2, 8])])
+def test_svbatch_block_positions(pq, n, qs):
+    """One dense block after a random product state, its qubits listed in any
+    order: qubits 1 and 2 in the block (four adjacent amplitudes per access),
+    qubit 1 alone (two), neither; the smallest states.  Every amplitude is two
+    sums of 2^k FP32 products (2^k + 2 roundings each of unit-norm rows and
+    fibers) after n one-qubit passes of the same kind with two products."""
+    from pqgb300.svbatch import StateVectorBatch
+
+    rng = np.random.default_rng(n * 100 + sum(qs))
+
+    def haar(d):
+        q, r = np.linalg.qr(rng.standard_normal((d, d)) + 1j * rng.standard_normal((d, d)))
+        return q * (np.diag(r) / np.abs(np.diag(r)))
+
+    blocks = [(haar(2), [q]) for q in range(1, n + 1)] + [(haar(1 << len(qs)), qs)]
+    psi = np.zeros((2,) * n, dtype=np.complex128)
+    psi[(0,) * n] = 1
+    for U, b in blocks:  # axis a holds qubit n - a; the first listed qubit is U's low bit
+        k = len(b)
+        axes = [n - q for q in reversed(b)]
+        psi = np.tensordot(U.reshape((2,) * (2 * k)), psi, axes=(list(range(k, 2 * k)), axes))
+        psi = np.moveaxis(psi, list(range(k)), axes)
+    bits = [format(i, f"0{n}b")[::-1] for i in range(1 << n)]
+    be = pq.GB300Backend(pq.PREC_C64)
+    sb = StateVectorBatch(be, [(n, blocks, bits)])
+    got = sb.execute()[0]
+    sb.close()
+    be.close()
+    tol = 2.0 ** -24 * (2 * (len(qs) ** 2 + 2 ** len(qs) + 2) + 8 * n)
+    assert np.linalg.norm(got - psi.reshape(-1)) <= tol

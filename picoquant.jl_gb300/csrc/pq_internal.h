@@ -53,9 +53,11 @@ struct GemmDesc {
 
 enum KernelClass : int { KC_GENERIC = 0, KC_GEMM = 1, KC_TC = 2, KC_COPY = 3, KC_SKINNY = 4 };
 // Skinny pairs (pq_skinny.cu): a large operand (>= kSkinnyMinRows rows over
-// its free modes) against a small one, K <= kSkinnyK, the small side's free
-// extent <= kSkinnyN, no batch modes.
-constexpr int kSkinnyK = 16, kSkinnyN = 16;
+// its free and batch modes, a block's worth of free ones) against a small one, K
+// <= kSkinnyK, the small side's free extent <= kSkinnyN; in complex128 contexts
+// <= kSkinnyN64 and no batch modes (FP64 multiply-adds bound those pairs on
+// every kernel).
+constexpr int kSkinnyK = 16, kSkinnyN = 128, kSkinnyN64 = 16;
 constexpr int64_t kSkinnyMinRows = 4096;
 // SIMT GEMM tile shapes: 64x64, 256x16 (narrow N), 16x256 (narrow M).
 enum GemmShape : int { GEMM_SQUARE = 0, GEMM_TALL = 1, GEMM_WIDE = 2 };
@@ -178,7 +180,7 @@ struct GenericGroup {
   void* C[kGroupMax];
 };
 cudaError_t launch_generic_group(const GenericGroup& g, const GenericDesc* d_descs, cudaStream_t stream);
-bool skinny_eligible(const GemmDesc& d);
+bool skinny_eligible(int precision, const GemmDesc& d);
 cudaError_t launch_skinny(int ta, int tb, int tc, const void* A, const void* B, void* C,
                           const GemmDesc& d, cudaStream_t stream);
 // out[c] = in[base + sum_i idx_i * stride_i] over `d` (uses csa as input

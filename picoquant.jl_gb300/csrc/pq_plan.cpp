@@ -405,10 +405,20 @@ bool compile(const Ctx* ctx, const std::vector<std::vector<int>>& leaf_labels,
     if (last) {
       lr = out_labels;
     } else {
-      for (int l : cp.labels[x])
-        if (cnt[l] > 0) lr.push_back(l);
-      for (int l : cp.labels[y])
-        if (cnt[l] > 0 && std::find(lr.begin(), lr.end(), l) == lr.end()) lr.push_back(l);
+      // x's labels, y's, then those of both (batch indices: the bitstrings of a
+      // group of amplitudes, a batch of slices).  With a batch index slowest,
+      // every member of the batch is a contiguous tensor and the kernels' rows
+      // and K runs stay adjacent; left where x had it, it drifts to the front
+      // as the labels before it are contracted, and every value of a row is a
+      // sector of its own.
+      const auto& lx = cp.labels[x];
+      const auto& ly = cp.labels[y];
+      std::vector<int> both;
+      for (int l : lx)
+        if (cnt[l] > 0) (std::find(ly.begin(), ly.end(), l) == ly.end() ? lr : both).push_back(l);
+      for (int l : ly)
+        if (cnt[l] > 0 && std::find(lx.begin(), lx.end(), l) == lx.end()) lr.push_back(l);
+      lr.insert(lr.end(), both.begin(), both.end());
     }
     if (last) {
       // everything not in the output must be summed now

@@ -1,8 +1,9 @@
 // Skinny pairs on the SIMT cores (sm_103a): a large operand X (R rows over
 // its free modes, K <= 16 contracted) against a small operand W (K x N, N <=
-// 16), C[r, n] = sum_k X[r, k] W[k, n].  This is a gate of up to four qubits
-// applied to a state vector or a boundary tensor absorbing a gate column:
-// memory-bound work whose bytes are X read once and C written once.
+// 128), C[r, n, z] = sum_k X[r, k, z] W[k, n, z].  This is a gate of up to four
+// qubits applied to a state vector or a boundary tensor absorbing a gate column
+// (with a batch index z, for every bitstring or slice): memory-bound work whose
+// bytes are X read once and C written once.
 //
 // One thread per row: it decodes the row's offsets in X and C (the modes are
 // merged, so a state-vector row has at most a few), loads its K values of X
@@ -11,7 +12,9 @@
 // consecutive rows, so each load and store of a warp is coalesced whenever the
 // row's first mode has unit stride; when X's unit-stride mode is contracted
 // (runs of KV values), a thread reads 16 or 32 aligned bytes at a time instead.
-// The offsets of k and n are decoded on the host and come with the launch.
+// The offsets of k and n are decoded on the host and come with the launch.  The
+// batch is the grid's y: one z and its W per block.  Where the small operand's
+// fastest mode is the result's, four columns are one aligned store.
 //
 // What bounds it: a 16 x 16 row needs 1024 FP32 multiply-adds for 256 bytes,
 // 28 us of the FP32 pipes per 2^20 rows against 39 us of HBM, and the broadcast
@@ -35,13 +38,29 @@ namespace {
 constexpr int kSkThreads = 128;
 
 struct SkinnyDesc {
-  int64_t R;
-  int K, N, nr, w64;        // w64: W is complex128
+  int64_t R, Z;
+  int K, N, nr, nz;
+  int w64;                  // W is complex128
+  int cvec;                 // columns 4i .. 4i + 3 are 32 aligned bytes of C (complex64)
   int64_t rdim[kMaxModes], rsx[kMaxModes], rsc[kMaxModes];
   int32_t rlog[kMaxModes];  // log2 of rdim, or -1
+  int64_t zdim[kMaxModes], zsx[kMaxModes], zsw[kMaxModes], zsc[kMaxModes];
   int64_t kx[kSkinnyK], cn[kSkinnyN];    // offsets of k in X and of n in C
   int64_t kw[kSkinnyK], nw[kSkinnyN];    // offsets of k and n in W
 };
+static_assert(sizeof(SkinnyDesc) + 64 <= 32764, "kernel parameters");
+
+// Offsets of batch index z in X, W and C.
+__device__ __forceinline__ void batch_offsets(const SkinnyDesc& d, int64_t z, int64_t& zx, int64_t& zw, int64_t& zc) {
+  zx = zw = zc = 0;
+  for (int i = 0; i < d.nz; ++i) {
+    const int64_t q = z / d.zdim[i], rem = z - q * d.zdim[i];
+    zx += rem * d.zsx[i];
+    zw += rem * d.zsw[i];
+    zc += rem * d.zsc[i];
+    z = q;
+  }
+}
 
 // KV consecutive complex64 values (KV * 8 bytes, aligned to them), or one value.
 template <int KV, typename TX>
@@ -79,69 +98,128 @@ __device__ __forceinline__ void row_offsets(const SkinnyDesc& d, int64_t x, int6
 }
 
 template <typename R>
-__device__ __forceinline__ typename Acc<R>::C w_value(const SkinnyDesc& d, const void* W, int k, int n) {
+__device__ __forceinline__ typename Acc<R>::C w_value(const SkinnyDesc& d, const void* W, int64_t zw, int k, int n) {
   if (k >= d.K || n >= d.N) return czero(R());
-  const int64_t o = d.kw[k] + d.nw[n];
+  const int64_t o = zw + d.kw[k] + d.nw[n];
   return d.w64 ? cvt<R>(static_cast<const double2*>(W)[o]) : cvt<R>(static_cast<const float2*>(W)[o]);
 }
 
-// Complex64 X and C.
+// One row of complex64 X: its K values (zero past K) and its products with W's
+// columns n0 .. n0 + 3 (columns n, n + 1 of W[k] as (re, re', im, im') at
+// w[(k * np + n / 2) * 4]).
+template <int KMAX, int KV>
+__device__ __forceinline__ void load_row(const SkinnyDesc& d, const float2* x, F2* ax, F2* ay) {
+  float2 a[KMAX];
+#pragma unroll
+  for (int k = 0; k < KMAX; k += KV) {
+    if (k < d.K) {
+      load_run<KV>(x + d.kx[k], &a[k]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < KV; ++u) a[k + u] = make_float2(0.f, 0.f);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < KMAX; ++k) {
+    ax[k] = f2_dup(a[k].x);
+    ay[k] = f2_dup(a[k].y);
+  }
+}
+template <int KMAX>
+__device__ __forceinline__ void four_columns(const F2* ax, const F2* ay, const float* w, int np, int n0, float2* o) {
+  F2 rr[2], ii[2], ri[2];  // sums of re re, im im and re im + im re for two column pairs
+#pragma unroll
+  for (int q = 0; q < 2; ++q) rr[q] = ii[q] = ri[q] = 0;
+#pragma unroll
+  for (int k = 0; k < KMAX; ++k) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(w + (k * np + n0 / 2 + q) * 4);
+      rr[q] = f2_fma(ax[k], b.x, rr[q]);
+      ii[q] = f2_fma(ay[k], b.y, ii[q]);
+      ri[q] = f2_fma(ax[k], b.y, ri[q]);
+      ri[q] = f2_fma(ay[k], b.x, ri[q]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const float2 p = f2_get(rr[q]), m = f2_get(ii[q]), y = f2_get(ri[q]);
+    o[2 * q] = make_float2(p.x - m.x, y.x);
+    o[2 * q + 1] = make_float2(p.y - m.y, y.y);
+  }
+}
+__device__ __forceinline__ void w_store(float* w, int np, int k, int n, float2 v) {
+  float* e = w + (k * np + n / 2) * 4 + (n & 1);
+  e[0] = v.x;
+  e[2] = v.y;
+}
+
+// Complex64 X and C, up to 16 columns, no batch.
 template <int KMAX, int KV>
 __global__ void __launch_bounds__(kSkThreads)
     k_skinny_f(const float2* __restrict__ X, const void* __restrict__ W, float2* __restrict__ C,
                const __grid_constant__ SkinnyDesc d) {
-  // columns n, n + 1 of W[k] as (re, re', im, im'), zero past K and N
-  __shared__ __align__(16) float w[KMAX][kSkinnyN / 2][4];
-  for (int t = threadIdx.x; t < KMAX * kSkinnyN; t += kSkThreads) {
-    const int k = t / kSkinnyN, n = t % kSkinnyN;
-    const float2 v = w_value<float>(d, W, k, n);
-    w[k][n / 2][n & 1] = v.x;
-    w[k][n / 2][2 + (n & 1)] = v.y;
-  }
+  constexpr int NP = 8;
+  __shared__ __align__(16) float w[KMAX * NP * 4];  // zero past K and N
+  for (int t = threadIdx.x; t < KMAX * 2 * NP; t += kSkThreads)
+    w_store(w, NP, t / (2 * NP), t % (2 * NP), w_value<float>(d, W, 0, t / (2 * NP), t % (2 * NP)));
   __syncthreads();
   const int64_t step = (int64_t)gridDim.x * kSkThreads;
   for (int64_t r = (int64_t)blockIdx.x * kSkThreads + threadIdx.x; r < d.R; r += step) {
     int64_t xo, co;
     row_offsets(d, r, xo, co);
-    float2 a[KMAX];
-#pragma unroll
-    for (int k = 0; k < KMAX; k += KV) {
-      if (k < d.K) {
-        load_run<KV>(X + xo + d.kx[k], &a[k]);
-      } else {
-#pragma unroll
-        for (int u = 0; u < KV; ++u) a[k + u] = make_float2(0.f, 0.f);
-      }
-    }
     F2 ax[KMAX], ay[KMAX];
-#pragma unroll
-    for (int k = 0; k < KMAX; ++k) {
-      ax[k] = f2_dup(a[k].x);
-      ay[k] = f2_dup(a[k].y);
-    }
+    load_row<KMAX, KV>(d, X + xo, ax, ay);
     // not unrolled: W is read per group of four columns instead of being kept
     // in registers
 #pragma unroll 1
     for (int n0 = 0; n0 < d.N; n0 += 4) {
-      F2 rr[2], ii[2], ri[2];  // sums of re re, im im and re im + im re for two column pairs
+      float2 o[4];
+      four_columns<KMAX>(ax, ay, w, NP, n0, o);
 #pragma unroll
-      for (int q = 0; q < 2; ++q) rr[q] = ii[q] = ri[q] = 0;
+      for (int n = 0; n < 4; ++n)
+        if (n0 + n < d.N) C[co + d.cn[n0 + n]] = o[n];
+    }
+  }
+}
+
+// Complex64 X and C, any number of columns up to 128, batched, or with whole
+// columns adjacent in C.
+template <int KMAX, int KV>
+__global__ void __launch_bounds__(kSkThreads)
+    k_skinny_w(const float2* __restrict__ X, const void* __restrict__ W, float2* __restrict__ C,
+               const __grid_constant__ SkinnyDesc d) {
+  extern __shared__ __align__(16) float w[];  // KMAX * np * 4, zero past K and N
+  const int np = (d.N + 3) / 4 * 2;
+  const int64_t step = (int64_t)gridDim.x * kSkThreads;
+  for (int64_t z = blockIdx.y; z < d.Z; z += gridDim.y) {
+    int64_t zx, zw, zc;
+    batch_offsets(d, z, zx, zw, zc);
+    if (z != blockIdx.y) __syncthreads();  // the previous W has been read
+    for (int t = threadIdx.x; t < KMAX * 2 * np; t += kSkThreads) {
+      const int k = t / (2 * np), n = t - k * (2 * np);
+      w_store(w, np, k, n, w_value<float>(d, W, zw, k, n));
+    }
+    __syncthreads();
+    for (int64_t r = (int64_t)blockIdx.x * kSkThreads + threadIdx.x; r < d.R; r += step) {
+      int64_t xo, co;
+      row_offsets(d, r, xo, co);
+      F2 ax[KMAX], ay[KMAX];
+      load_row<KMAX, KV>(d, X + zx + xo, ax, ay);
+      float2* c = C + zc + co;
+#pragma unroll 1
+      for (int n0 = 0; n0 < d.N; n0 += 4) {
+        float2 o[4];
+        four_columns<KMAX>(ax, ay, w, np, n0, o);
+        if (d.cvec) {
+          asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(c + d.cn[n0]), "f"(o[0].x), "f"(o[0].y),
+                       "f"(o[1].x), "f"(o[1].y), "f"(o[2].x), "f"(o[2].y), "f"(o[3].x), "f"(o[3].y)
+                       : "memory");
+        } else {
 #pragma unroll
-      for (int k = 0; k < KMAX; ++k) {
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(w[k][n0 / 2 + q]);
-          rr[q] = f2_fma(ax[k], b.x, rr[q]);
-          ii[q] = f2_fma(ay[k], b.y, ii[q]);
-          ri[q] = f2_fma(ax[k], b.y, ri[q]);
-          ri[q] = f2_fma(ay[k], b.x, ri[q]);
+          for (int n = 0; n < 4; ++n)
+            if (n0 + n < d.N) c[d.cn[n0 + n]] = o[n];
         }
-      }
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const float2 p = f2_get(rr[q]), m = f2_get(ii[q]), y = f2_get(ri[q]);
-        if (n0 + 2 * q < d.N) C[co + d.cn[n0 + 2 * q]] = make_float2(p.x - m.x, y.x);
-        if (n0 + 2 * q + 1 < d.N) C[co + d.cn[n0 + 2 * q + 1]] = make_float2(p.y - m.y, y.y);
       }
     }
   }
@@ -154,60 +232,77 @@ __global__ void __launch_bounds__(kSkThreads)
              const __grid_constant__ SkinnyDesc d) {
   using R = typename std::conditional<std::is_same<TC, double2>::value, double, float>::type;
   using R2 = typename Acc<R>::C;
-  __shared__ __align__(16) R2 w[KMAX][kSkinnyN];  // W[k][n], zero past K and N
-  for (int t = threadIdx.x; t < KMAX * kSkinnyN; t += kSkThreads)
-    w[t / kSkinnyN][t % kSkinnyN] = w_value<R>(d, W, t / kSkinnyN, t % kSkinnyN);
-  __syncthreads();
+  // W[k][n] at w[k * nw + n], zero past K and N (nw a multiple of four)
+  extern __shared__ __align__(16) unsigned char w_raw[];
+  R2* w = reinterpret_cast<R2*>(w_raw);
+  const int nw = (d.N + 3) / 4 * 4;
   const int64_t step = (int64_t)gridDim.x * kSkThreads;
-  for (int64_t r = (int64_t)blockIdx.x * kSkThreads + threadIdx.x; r < d.R; r += step) {
-    int64_t xo, co;
-    row_offsets(d, r, xo, co);
-    R2 a[KMAX];
+  for (int64_t z = blockIdx.y; z < d.Z; z += gridDim.y) {
+    int64_t zx, zw, zc;
+    batch_offsets(d, z, zx, zw, zc);
+    if (z != blockIdx.y) __syncthreads();  // the previous W has been read
+    for (int t = threadIdx.x; t < KMAX * nw; t += kSkThreads) w[t] = w_value<R>(d, W, zw, t / nw, t % nw);
+    __syncthreads();
+    for (int64_t r = (int64_t)blockIdx.x * kSkThreads + threadIdx.x; r < d.R; r += step) {
+      int64_t xo, co;
+      row_offsets(d, r, xo, co);
+      xo += zx;
+      co += zc;
+      R2 a[KMAX];
 #pragma unroll
-    for (int k = 0; k < KMAX; ++k) a[k] = k < d.K ? cvt<R>(__ldg(X + xo + d.kx[k])) : czero(R());
+      for (int k = 0; k < KMAX; ++k) a[k] = k < d.K ? cvt<R>(__ldg(X + xo + d.kx[k])) : czero(R());
 #pragma unroll 1
-    for (int n0 = 0; n0 < d.N; n0 += 4) {
-      R2 acc[4];
+      for (int n0 = 0; n0 < d.N; n0 += 4) {
+        R2 acc[4];
 #pragma unroll
-      for (int n = 0; n < 4; ++n) acc[n] = czero(R());
+        for (int n = 0; n < 4; ++n) acc[n] = czero(R());
 #pragma unroll
-      for (int k = 0; k < KMAX; ++k) {
+        for (int k = 0; k < KMAX; ++k) {
 #pragma unroll
-        for (int n = 0; n < 4; ++n) cfma(acc[n], a[k], w[k][n0 + n]);
+          for (int n = 0; n < 4; ++n) cfma(acc[n], a[k], w[k * nw + n0 + n]);
+        }
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+          if (n0 + n < d.N) C[co + d.cn[n0 + n]] = store_as<TC>(acc[n]);
       }
-#pragma unroll
-      for (int n = 0; n < 4; ++n)
-        if (n0 + n < d.N) C[co + d.cn[n0 + n]] = store_as<TC>(acc[n]);
     }
   }
 }
 
-// Persistent-style grids of the blocks that fit an SM at the kernels' register
-// counts (complex64: 64 registers at K <= 16, 46 or fewer below; FP64: 96).
-int sk_grid(int64_t rows, int per_sm) {
-  return (int)std::min<int64_t>((rows + kSkThreads - 1) / kSkThreads, 152 * per_sm);
+// Row blocks by batch index; persistent-style over the blocks that fit an SM at
+// the kernels' register counts (complex64: 64 registers at K <= 16, 46 or fewer
+// below; FP64: 96).
+dim3 sk_grid(const SkinnyDesc& d, int per_sm) {
+  const int64_t y = std::min<int64_t>(d.Z, 65535);
+  const int64_t x = std::max<int64_t>(1, 152 * per_sm / y);
+  return dim3((unsigned)std::min<int64_t>((d.R + kSkThreads - 1) / kSkThreads, x), (unsigned)y);
 }
 
 template <typename TX, typename TC>
 cudaError_t launch_mixed(const void* X, const void* W, void* C, const SkinnyDesc& d, cudaStream_t s) {
+  const size_t col = (size_t)((d.N + 3) / 4 * 4) * (std::is_same<TC, double2>::value ? 16 : 8);
   if (d.K <= 4)
-    k_skinny<TX, TC, 4><<<sk_grid(d.R, 10), kSkThreads, 0, s>>>((const TX*)X, W, (TC*)C, d);
+    k_skinny<TX, TC, 4><<<sk_grid(d, 10), kSkThreads, 4 * col, s>>>((const TX*)X, W, (TC*)C, d);
   else
-    k_skinny<TX, TC, 16><<<sk_grid(d.R, 5), kSkThreads, 0, s>>>((const TX*)X, W, (TC*)C, d);
+    k_skinny<TX, TC, 16><<<sk_grid(d, 5), kSkThreads, 16 * col, s>>>((const TX*)X, W, (TC*)C, d);
   return cudaGetLastError();
 }
 
-template <int KMAX>
-cudaError_t launch_f(int kv, const void* X, const void* W, void* C, const SkinnyDesc& d, cudaStream_t s) {
-  const int grid = sk_grid(d.R, KMAX == 16 ? 8 : 10);
-  const float2* x = (const float2*)X;
-  if (kv == 4)
-    k_skinny_f<KMAX, 4><<<grid, kSkThreads, 0, s>>>(x, W, (float2*)C, d);
-  else if (kv == 2)
-    k_skinny_f<KMAX, 2><<<grid, kSkThreads, 0, s>>>(x, W, (float2*)C, d);
+template <int KMAX, int KV>
+cudaError_t launch_kv(const void* X, const void* W, void* C, const SkinnyDesc& d, cudaStream_t s) {
+  const dim3 grid = sk_grid(d, KMAX == 16 ? 8 : 10);
+  if (d.N <= 16 && d.Z == 1 && !d.cvec)
+    k_skinny_f<KMAX, KV><<<grid, kSkThreads, 0, s>>>((const float2*)X, W, (float2*)C, d);
   else
-    k_skinny_f<KMAX, 1><<<grid, kSkThreads, 0, s>>>(x, W, (float2*)C, d);
+    k_skinny_w<KMAX, KV><<<grid, kSkThreads, (size_t)KMAX * ((d.N + 3) / 4 * 2) * 16, s>>>((const float2*)X, W,
+                                                                                             (float2*)C, d);
   return cudaGetLastError();
+}
+template <int KMAX>
+cudaError_t launch_k(int kv, const void* X, const void* W, void* C, const SkinnyDesc& d, cudaStream_t s) {
+  if (kv == 4) return launch_kv<KMAX, 4>(X, W, C, d, s);
+  if (kv == 2) return launch_kv<KMAX, 2>(X, W, C, d, s);
+  return launch_kv<KMAX, 1>(X, W, C, d, s);
 }
 
 int log2_exact(int64_t v) {
@@ -228,13 +323,19 @@ int64_t offset_of(int64_t x, int n, const int64_t* dim, const int64_t* s) {
 
 }  // namespace
 
-bool skinny_eligible(const GemmDesc& g) {
-  return g.Z == 1 && std::max(g.M, g.N) >= kSkinnyMinRows && std::min(g.M, g.N) <= kSkinnyN && g.K <= kSkinnyK;
+static bool skinny_shape(const GemmDesc& g) {
+  const int64_t rows = std::max(g.M, g.N);
+  return rows >= kSkThreads && rows * g.Z >= kSkinnyMinRows && std::min(g.M, g.N) <= kSkinnyN && g.K <= kSkinnyK;
+}
+
+bool skinny_eligible(int precision, const GemmDesc& g) {
+  if (precision == PQ_PREC_C128 && (g.Z > 1 || std::min(g.M, g.N) > kSkinnyN64)) return false;
+  return skinny_shape(g);
 }
 
 cudaError_t launch_skinny(int ta, int tb, int tc, const void* A, const void* B, void* C, const GemmDesc& g,
                           cudaStream_t stream) {
-  if (!skinny_eligible(g)) return cudaErrorInvalidValue;
+  if (!skinny_shape(g)) return cudaErrorInvalidValue;
   // the large side is X (rows), the small side W
   const bool a_big = g.M >= g.N;
   const void* X = a_big ? A : B;
@@ -243,10 +344,11 @@ cudaError_t launch_skinny(int ta, int tb, int tc, const void* A, const void* B, 
   SkinnyDesc d;
   std::memset(&d, 0, sizeof(d));
   d.R = a_big ? g.M : g.N;
+  d.Z = g.Z;
   d.N = (int)(a_big ? g.N : g.M);
   d.K = (int)g.K;
   d.w64 = (a_big ? tb : ta) == PQ_C128;
-  if (d.R == 0) return cudaSuccess;
+  if (d.R * d.Z == 0) return cudaSuccess;
   d.nr = a_big ? g.nm : g.nn;
   const int64_t* ksx = a_big ? g.ksa : g.ksb;
   // runs of KV contracted values that are KV * 8 aligned bytes in X: the first
@@ -268,19 +370,35 @@ cudaError_t launch_skinny(int ta, int tb, int tc, const void* A, const void* B, 
     d.rlog[i] = log2_exact(d.rdim[i]);
     limit(d.rsx[i]);
   }
+  const int64_t* nsc = a_big ? g.nsc : g.msc;
+  const int64_t* ndim = a_big ? g.ndim : g.mdim;
+  const int nn = a_big ? g.nn : g.nm;
+  bool cvec = nn > 0 && nsc[0] == 1 && ndim[0] % 4 == 0 && (uintptr_t)C % 32 == 0;
+  for (int i = 1; i < nn; ++i) cvec = cvec && nsc[i] % 4 == 0;
+  for (int i = 0; i < d.nr; ++i) cvec = cvec && d.rsc[i] % 4 == 0;
+  d.nz = g.nz;
+  for (int i = 0; i < g.nz; ++i) {
+    d.zdim[i] = g.zdim[i];
+    d.zsx[i] = a_big ? g.zsa[i] : g.zsb[i];
+    d.zsw[i] = a_big ? g.zsb[i] : g.zsa[i];
+    d.zsc[i] = g.zsc[i];
+    limit(d.zsx[i]);
+    cvec = cvec && d.zsc[i] % 4 == 0;
+  }
+  d.cvec = cvec;
   for (int k = 0; k < d.K; ++k) {
     d.kx[k] = offset_of(k, g.nk, g.kdim, ksx);
     d.kw[k] = offset_of(k, g.nk, g.kdim, a_big ? g.ksb : g.ksa);
   }
   for (int n = 0; n < d.N; ++n) {
-    d.nw[n] = offset_of(n, a_big ? g.nn : g.nm, a_big ? g.ndim : g.mdim, a_big ? g.nsb : g.msa);
-    d.cn[n] = offset_of(n, a_big ? g.nn : g.nm, a_big ? g.ndim : g.mdim, a_big ? g.nsc : g.msc);
+    d.nw[n] = offset_of(n, nn, ndim, a_big ? g.nsb : g.msa);
+    d.cn[n] = offset_of(n, nn, ndim, nsc);
   }
   if (c64) return x64 ? launch_mixed<double2, double2>(X, W, C, d, stream) : launch_mixed<float2, double2>(X, W, C, d, stream);
   if (x64) return launch_mixed<double2, float2>(X, W, C, d, stream);
-  if (d.K <= 4) return launch_f<4>(kv, X, W, C, d, stream);
-  if (d.K <= 8) return launch_f<8>(kv, X, W, C, d, stream);
-  return launch_f<16>(kv, X, W, C, d, stream);
+  if (d.K <= 4) return launch_k<4>(kv, X, W, C, d, stream);
+  if (d.K <= 8) return launch_k<8>(kv, X, W, C, d, stream);
+  return launch_k<16>(kv, X, W, C, d, stream);
 }
 
 }  // namespace pq

@@ -61,7 +61,7 @@ bool choice_eligible(int precision, const PairPlan& p, const TuneChoice& c) {
       return tc_eligible(precision, g);
     }
     case KC_SKINNY:
-      return skinny_eligible(p.m);
+      return skinny_eligible(precision, p.m);
     case KC_GEMM:
       return p.gemm_shape || (p.ksize > kGenericKTab && p.M >= 8 && p.N >= 8);
     case KC_GENERIC:

@@ -244,3 +244,46 @@ def test_skinny_complex64_runs(pq, first, m, last, n):
         got = got.T if swap else got
         assert np.all(np.abs(got - ref) <= bound)
     be.close()
+
+
+@pytest.mark.parametrize("m,k,n,z,order", [(130, 8, 128, 64, "mkz"), (4097, 3, 33, 2, "mkz"), (1000, 16, 17, 5, "kmz"),
+                                           (513, 1, 100, 9, "zkm"), (2049, 12, 7, 3, "kmz"), (140, 4, 2, 31, "mzk"),
+                                           (5000, 5, 128, 1, "mkz")])
+@pytest.mark.parametrize("swap", [False, True], ids=["large-first", "small-first"])
+def test_skinny_wide_and_batched(pq, m, k, n, z, order, swap):
+    """More than 16 columns and batch modes in a complex64 context (one W per
+    batch index), in several mode orders, either operand first (the small
+    operand's modes then lead the result: whole-sector stores where its
+    extent is a multiple of four).  Bound as for single pairs."""
+    from pqgb300 import _lib as L
+
+    rng = np.random.default_rng(m + n)
+    ext = {"m": m, "k": k, "z": z}
+
+    def crand(*s):
+        return (rng.standard_normal(s) + 1j * rng.standard_normal(s)).astype(np.complex64)
+
+    X = crand(*[ext[c] for c in order])
+    W = crand(k, n, z)
+    xs, ws = (order, "knz")
+    ops, out = ([(W, ws), (X, xs)], "nmz") if swap else ([(X, xs), (W, ws)], "mnz")
+    ids = {"m": 0, "k": 1, "n": 2, "z": 3}
+    be = pq.GB300Backend(pq.PREC_C64, small_elems=0)
+    for name, (T, _) in zip("ab", ops):
+        be.save_tensor_data(name, T)
+    h = C.c_void_p()
+    labs = [ids[c] for _, s in ops for c in s]
+    L.check(be.lib.pq_plan_create(be.ctx, 2, L.arr(C.c_int32, [3, 3]), L.arr(C.c_int32, labs), 4,
+                                  L.arr(C.c_int64, [m, k, n, z]), 1, L.arr(C.c_int32, [0, 1]), 3,
+                                  L.arr(C.c_int32, [ids[c] for c in out]), C.byref(h)), be.ctx, "plan_create")
+    f = (C.c_double * 8)()
+    L.check(be.lib.pq_plan_step_features(h, f), be.ctx, "features")
+    assert int(f[6]) == KC_SKINNY
+    L.check(be.lib.pq_plan_execute(h, L.arr(C.c_int64, [be.id_of("a"), be.id_of("b")]), be.id_of("r")), be.ctx, "run")
+    got = be.load_tensor_data("r")
+    be.lib.pq_plan_destroy(h)
+    be.close()
+    expr = f"{xs},{ws}->{out}"
+    ref = np.einsum(expr, X.astype(np.complex128), W.astype(np.complex128))
+    bound = 2 * (k + 2) * 2.0 ** -24 * np.einsum(expr, np.abs(X), np.abs(W))
+    assert np.all(np.abs(got - ref) <= bound)

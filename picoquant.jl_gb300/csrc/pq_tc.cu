@@ -222,27 +222,28 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (!mbar_wait(&sm.full[i % S], (uint32_t)((i / S) & 1))) ok = false;
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_tf32(TM, TN), idesc_neg = idesc_tf32(TM, TN, true);
-      constexpr uint32_t ALBO = (TM / 8) * 128, BLBO = (TN / 8) * 128, SBO = 128;
-      int64_t g = 0;  // K tiles (= chunks) consumed so far
-      for (int64_t tile = blockIdx.x; tile < ntot && ok; tile += gridDim.x) {
-        for (int64_t kt = 0; kt < ktiles; ++kt, ++g) {
-          const int s = (int)(g % S);
-          const uint32_t ph = (uint32_t)((g / S) & 1);
-          const int b = (int)(g % kSets);
-          const uint32_t use = (uint32_t)((g / kSets) & 1);
-          if (!mbar_wait(&sm.full[s], ph) || !mbar_wait(&sm.acce[b], use ^ 1)) {
-            ok = false;
-            break;
-          }
-          fence_after();
-          const uint32_t sa = smem_u32(sm.stage[s]);
-          const uint32_t sb = sa + P * kATile * 4;
-          const uint32_t dr = tmem + (uint32_t)b * (2 * TN), di = dr + TN;
-          // The tensor core rounds an accumulation toward zero.  The small
-          // correction products go in first (the first one overwrites), the
-          // large hi x hi products last.
+    // The whole warp runs the loop and waits, one elected thread issues a K
+    // tile's MMAs and commits, so that descriptors stay uniform.  An N = 48 MMA
+    // takes 24 cycles of the tensor core and reads 5.5 KB of operands (43 cycles
+    // of shared memory).
+    constexpr uint32_t idesc = idesc_tf32(TM, TN), idesc_neg = idesc_tf32(TM, TN, true);
+    constexpr uint32_t ALBO = (TM / 8) * 128, BLBO = (TN / 8) * 128, SBO = 128;
+    int s = 0, b = 0;  // ring stage and accumulator set, with their phases
+    uint32_t ph = 0, use = 0;
+    for (int64_t tile = blockIdx.x; tile < ntot && ok; tile += gridDim.x) {
+      for (int64_t kt = 0; kt < ktiles; ++kt) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&sm.full[s], ph) && mbar_wait(&sm.acce[b], use ^ 1))) {
+          ok = false;
+          break;
+        }
+        fence_after();
+        const uint32_t sa = smem_u32(sm.stage[s]) >> 4;
+        const uint32_t sb = sa + ((P * kATile * 4) >> 4);
+        const uint32_t dr = tmem + (uint32_t)b * (2 * TN), di = dr + TN;
+        // The tensor core rounds an accumulation toward zero.  The small
+        // correction products go in first (the first one overwrites), the
+        // large hi x hi products last.
+        if (elect_one()) {
 #pragma unroll
           for (int q = 1; q <= CF::products; ++q) {
             const int qq = q == CF::products ? 0 : q;  // hi x hi last
@@ -253,10 +254,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int j = 0; j < TK / 8; ++j) {  // the two 8-deep halves of the tile
               const uint32_t acc = (q == 1 && j == 0) ? 0u : 1u;
               const uint32_t oa = (uint32_t)j * 2 * ALBO, ob = (uint32_t)j * 2 * BLBO;
-              const uint64_t ar = smem_desc(sa + (0 * NS + ti) * kATile * 4 + oa, ALBO, SBO);
-              const uint64_t ai = smem_desc(sa + (1 * NS + ti) * kATile * 4 + oa, ALBO, SBO);
-              const uint64_t br = smem_desc(sb + (0 * NS + tj) * kBTile * 4 + ob, BLBO, SBO);
-              const uint64_t bi = smem_desc(sb + (1 * NS + tj) * kBTile * 4 + ob, BLBO, SBO);
+              const uint64_t ar = desc_at(sa + (((0 * NS + ti) * kATile * 4 + oa) >> 4), ALBO, SBO);
+              const uint64_t ai = desc_at(sa + (((1 * NS + ti) * kATile * 4 + oa) >> 4), ALBO, SBO);
+              const uint64_t br = desc_at(sb + (((0 * NS + tj) * kBTile * 4 + ob) >> 4), BLBO, SBO);
+              const uint64_t bi = desc_at(sb + (((1 * NS + tj) * kBTile * 4 + ob) >> 4), BLBO, SBO);
               mma_tf32(dr, ar, br, idesc, acc);     // + Ar.Br
               mma_tf32(di, ar, bi, idesc, acc);     // + Ar.Bi
               mma_tf32(dr, ai, bi, idesc_neg, 1u);  // - Ai.Bi
@@ -266,11 +267,19 @@ __global__ void __launch_bounds__(kThreads, 1)
           mma_commit(&sm.accf[b]);   // chunk accumulators ready for the epilogue
           mma_commit(&sm.empty[s]);  // smem stage free once these MMAs finish
         }
+        if (++s == S) {
+          s = 0;
+          ph ^= 1u;
+        }
+        if (++b == kSets) {
+          b = 0;
+          use ^= 1u;
+        }
       }
-      // every MMA issued has finished once this arrives (TMEM is freed below)
-      mma_commit(&sm.drain);
-      if (!mbar_wait(&sm.drain, 0)) ok = false;
     }
+    // every MMA issued has finished once this arrives (TMEM is freed below)
+    if (elect_one()) mma_commit(&sm.drain);
+    if (!mbar_wait(&sm.drain, 0)) ok = false;
   } else {
     // epilogue: warp w reads TMEM lanes of quadrant w % 4, columns [16h, 16h+16)
     constexpr int CW = TN / (kEpiWarps / 4);  // columns per epilogue warp

@@ -5,8 +5,9 @@
 // results accumulate each 16-deep K tile in FP32 and fold the tile sums into a
 // Kahan-compensated accumulator, so the rounding error does not grow with K.
 //
-// Three tile shapes (256 threads, each owning R x S results):
-//   square  BM=64,  BN=64,  R=4,  S=4   general pairs
+// Tile shapes (256 threads, each owning R x S results):
+//   square  BM=64,  BN=64,  R=4,  S=4   general pairs (complex128 results also
+//                                        32 x 32 and 16 x 16)
 //   tall    BM=256, BN=16,  R=16, S=1   narrow N (e.g. a big boundary absorbing
 //                                        a qubit with few open bonds)
 //   wide    BM=16,  BN=256, R=1,  S=16  narrow M
@@ -223,10 +224,23 @@ static cudaError_t gemm_launch(const void* A, const void* B, void* C, const Gemm
 template <typename TA, typename TB, typename TC>
 static cudaError_t gemm_shape(int shape, const void* A, const void* B, void* C, const GemmDesc& d, cudaStream_t s) {
   // the narrow tiles need 32 KiB of complex64 staging; complex128 results
-  // (FP64 accumulation, twice the tile bytes) always use the square tile
+  // (FP64 accumulation, twice the tile bytes) use square tiles
   if constexpr (std::is_same<TC, float2>::value) {
     if (shape == GEMM_TALL) return gemm_launch<TA, TB, TC, 256, 16, 16, 1>(A, B, C, d, s);
     if (shape == GEMM_WIDE) return gemm_launch<TA, TB, TC, 16, 256, 1, 16>(A, B, C, d, s);
+  }
+  // Complex128 results: FP64 multiply-adds (2 per clock and SM) bound every
+  // tile, so the tile is the one with the least work on the busiest SM, tiles
+  // there times tile area, the larger at a tie.  M = 1024, N = 16, K = 128: 16
+  // tiles of 64 x 64 took 544 us, 64 of 16 x 16 take 39.
+  if constexpr (std::is_same<TC, double2>::value) {
+    auto load = [&](int64_t t) {
+      const int64_t tiles = ((d.M + t - 1) / t) * ((d.N + t - 1) / t) * d.Z;
+      return (tiles + 151) / 152 * t * t;
+    };
+    const int64_t l64 = load(64), l32 = load(32), l16 = load(16);
+    if (l16 < l32 && l16 < l64) return gemm_launch<TA, TB, TC, 16, 16, 1, 1>(A, B, C, d, s);
+    if (l32 < l64) return gemm_launch<TA, TB, TC, 32, 32, 2, 2>(A, B, C, d, s);
   }
   return gemm_launch<TA, TB, TC, 64, 64, 4, 4>(A, B, C, d, s);
 }

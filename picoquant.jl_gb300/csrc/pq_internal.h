@@ -175,10 +175,12 @@ struct GenericGroup {
   int n;
   int blk[kGroupMax + 1];
   int desc[kGroupMax];
+  int lsub[kGroupMax];  // log2 of the lanes that share a result element
   const void* A[kGroupMax];
   const void* B[kGroupMax];
   void* C[kGroupMax];
 };
+int generic_lanes(int64_t csize, int64_t ksize);
 cudaError_t launch_generic_group(const GenericGroup& g, const GenericDesc* d_descs, cudaStream_t stream);
 bool skinny_eligible(int precision, const GemmDesc& d);
 cudaError_t launch_skinny(int ta, int tb, int tc, const void* A, const void* B, void* C,

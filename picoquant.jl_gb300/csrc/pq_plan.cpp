@@ -588,7 +588,8 @@ int launch_all(pq_plan* p, const Compiled& cp, const std::vector<const void*>& l
         g.A[g.n] = vptr[t.x];
         g.B[g.n] = vptr[t.y];
         g.C[g.n] = (char*)p->arena + t.off;
-        blocks += (int)std::min<int64_t>((t.pp.csize + 255) / 256, 64);
+        g.lsub[g.n] = generic_lanes(t.pp.csize, t.pp.g.ksize);
+        blocks += (int)std::min<int64_t>(((t.pp.csize << g.lsub[g.n]) + 255) / 256, 64);
         g.n++;
       }
       g.blk[g.n] = blocks;

@@ -90,6 +90,8 @@ __device__ __forceinline__ void cfma(float2& acc, float2 a, float2 b) {
 // while the kernel before it in the stream still runs.  pdl_wait() returns once
 // that kernel has finished and its writes are visible; every thread of such a
 // kernel calls it before it reads anything a kernel writes, or writes anything.
+// The operands of such a kernel are written while it exists: no __ldg, no
+// ld.global.nc and no const __restrict__ on them (a stale L1 line would do).
 // pdl_trigger() lets the next launch_pdl kernel start (it still waits).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -169,3 +169,24 @@ def test_backend_ops(backend, O):
     assert rel_err(backend.gather("u", idx), T.reshape(-1, order="F")[idx]) < TOL[backend.precision]
     backend.delete_tensor("u")
     assert backend.load_tensor_data("u") is None
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 5), (1, 1, 700), (3, 1, 64), (7, 5, 33), (1, 9, 2049), (2, 3, 5000), (65, 17, 100),
+                                   (300, 40, 7), (1024, 16, 128), (1000, 9, 260), (70, 40, 400), (333, 130, 50),
+                                   (700, 500, 20), (2000, 70, 20)])
+def test_complex128_small_results(pq, m, n, k):
+    """Complex128 pairs with small results: K shared by 1 to 32 lanes per
+    element on the generic kernel (single elements, ragged blocks, K past the
+    offset table), and 16-, 32- and 64-wide tiles with ragged edges on the
+    tiled one.  Every component is a sum of 2K products in FP64, within
+    (2K + 6) 2^-53 of the sum of absolute products in any order."""
+    rng = np.random.default_rng(m * n + k)
+    A = rng.standard_normal((m, k)) + 1j * rng.standard_normal((m, k))
+    B = rng.standard_normal((k, n)) + 1j * rng.standard_normal((k, n))
+    be = pq.GB300Backend(pq.PREC_C128)
+    be.save_tensor_data("a", A)
+    be.save_tensor_data("b", B)
+    be.contract_tensors("a", [-1, 1], "b", [1, -2], "c")
+    got = be.load_tensor_data("c").reshape(m, n)
+    be.close()
+    assert np.all(np.abs(got - A @ B) <= 2 * (2 * k + 6) * 2.0 ** -53 * (np.abs(A) @ np.abs(B)))

@@ -25,38 +25,204 @@ using namespace pq;
 
 namespace {
 
-constexpr int TB = 16;  // tile of the small SIMT GEMMs
+constexpr int TB = 16;  // tile of the bf16 inference layers
 
-// C[M x N] = op(A) @ op(B) (+ bias[N]) with optional ReLU, FP32.
-//   op(A) = A [M x K] (ta = 0) or A^T with A [K x M] (ta = 1)
-//   op(B) = B [K x N] (tb = 0) or B^T with B [N x K] (tb = 1)
-// beta = 1 accumulates into C.
-__global__ void k_sgemm(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C,
-                        const float* __restrict__ bias, int M, int N, int K, int ta, int tb, int relu, float beta) {
-  __shared__ float As[TB][TB + 1];
-  __shared__ float Bs[TB][TB + 1];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int row = blockIdx.y * TB + ty, col = blockIdx.x * TB + tx;
-  float acc = 0.f;
-  for (int k0 = 0; k0 < K; k0 += TB) {
-    int ka = k0 + tx, kb = k0 + ty;
-    float a = 0.f, b = 0.f;
-    if (row < M && ka < K) a = ta ? A[(size_t)ka * M + row] : A[(size_t)row * K + ka];
-    if (col < N && kb < K) b = tb ? B[(size_t)col * K + kb] : B[(size_t)kb * N + col];
-    As[ty][tx] = a;
-    Bs[ty][tx] = b;
-    __syncthreads();
+// FP32 layer products on 32 x 32 tiles, 256 threads, four results each, K in
+// steps of 128 through shared memory (all of a step's loads in flight at once: 10
+// -> 7 us per layer against steps of 32).  A training batch (1024 rows, 128 wide) is
+// latency-bound, so the tile is the largest that still gives a block to most
+// SMs (128 blocks), and the weight gradients, whose K is the batch, are split
+// into chunks of rows (`part`) that k_reduce_parts adds up in order: with K
+// walked by 64 blocks they took 61 us per layer, and the bias sums, one thread
+// per column over all rows, as long.  Forward and backward of a batch: 19
+// launches, 520 us -> 8 launches, 51 us.
+constexpr int GT = 32, GTP = GT + 1, GK = 128;
+
+struct Tile32 {
+  float a[GK][GTP];  // a[k][m]
+  float b[GK][GTP];  // b[k][n]
+};
+// acc += a^T b over the staged K steps, for rows ty, ty + 16 and columns tx, tx + 16.
+__device__ __forceinline__ void tile_fma(const Tile32& t, int kn, int tx, int ty, float (&acc)[2][2]) {
+#pragma unroll 8
+  for (int k = 0; k < kn; ++k) {
+    const float a0 = t.a[k][ty], a1 = t.a[k][ty + 16], b0 = t.b[k][tx], b1 = t.b[k][tx + 16];
+    acc[0][0] = fmaf(a0, b0, acc[0][0]);
+    acc[0][1] = fmaf(a0, b1, acc[0][1]);
+    acc[1][0] = fmaf(a1, b0, acc[1][0]);
+    acc[1][1] = fmaf(a1, b1, acc[1][1]);
+  }
+}
+
+// BACK = false: Y [n x N] = relu(X [n x K] W [K x N] + bias).
+// BACK = true:  Y [n x N] = (X [n x K] W^T, W [N x K]), zero where H [n x N] <= 0
+// (the gradient through the ReLU of activations H).
+template <bool BACK>
+__global__ void __launch_bounds__(256)
+    k_layer(const float* __restrict__ X, const float* __restrict__ W, const float* __restrict__ bias,
+            const float* __restrict__ H, float* __restrict__ Y, int n, int N, int K) {
+  __shared__ Tile32 t;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
+  const int m0 = blockIdx.x * GT, n0 = blockIdx.y * GT;
+  float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+  for (int k0 = 0; k0 < K; k0 += GK) {
+    // element e of a step: X and W^T rows along K, W rows along N
+    float ra[GT * GK / 256], rb[GT * GK / 256];
 #pragma unroll
-    for (int k = 0; k < TB; ++k) acc = fmaf(As[ty][k], Bs[k][tx], acc);
+    for (int i = 0; i < GT * GK / 256; ++i) {
+      const int k = lx + 32 * (i & 3), r = ly + 8 * (i >> 2);  // 4 runs of 32 k, rows 8 apart
+      ra[i] = m0 + r < n && k0 + k < K ? X[(size_t)(m0 + r) * K + k0 + k] : 0.f;
+      if (BACK)
+        rb[i] = n0 + r < N && k0 + k < K ? W[(size_t)(n0 + r) * K + k0 + k] : 0.f;
+      else
+        rb[i] = n0 + lx < N && k0 + ly + 8 * i < K ? W[(size_t)(k0 + ly + 8 * i) * N + n0 + lx] : 0.f;
+    }
+    if (k0) __syncthreads();  // the previous step has been read
+#pragma unroll
+    for (int i = 0; i < GT * GK / 256; ++i) {
+      const int k = lx + 32 * (i & 3), r = ly + 8 * (i >> 2);
+      t.a[k][r] = ra[i];
+      if (BACK)
+        t.b[k][r] = rb[i];
+      else
+        t.b[ly + 8 * i][lx] = rb[i];
+    }
+    __syncthreads();
+    tile_fma(t, min(GK, K - k0), tx, ty, acc);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int row = m0 + ty + 16 * i, col = n0 + tx + 16 * j;
+      if (row >= n || col >= N) continue;
+      const size_t o = (size_t)row * N + col;
+      if (BACK)
+        Y[o] = H[o] <= 0.f ? 0.f : acc[i][j];
+      else {
+        const float v = acc[i][j] + bias[col];
+        Y[o] = v > 0.f ? v : 0.f;
+      }
+    }
+}
+
+// The output layer (one value per row, a warp each): y = h . w + b.  With
+// targets, also the gradient of the mean squared error, dy = 2 (y - t) / n, its
+// product with w through the ReLU of h, and the block's sum of squared errors.
+__global__ void __launch_bounds__(256)
+    k_head(const float* __restrict__ H, const float* __restrict__ w, const float* __restrict__ b, int n, int K,
+           float* __restrict__ y, const float* __restrict__ t, float* __restrict__ dy, float* __restrict__ dh,
+           float* __restrict__ loss_part) {
+  __shared__ float sq[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row = blockIdx.x * 8 + warp;
+  float e = 0.f;
+  if (row < n) {
+    const float* h = H + (size_t)row * K;
+    float acc = 0.f;
+    for (int k = lane; k < K; k += 32) acc = fmaf(h[k], w[k], acc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    acc += b[0];
+    if (lane == 0) y[row] = acc;
+    if (t) {
+      e = acc - t[row];
+      const float g = 2.f * e / (float)n;
+      if (lane == 0) dy[row] = g;
+      if (dh)
+        for (int k = lane; k < K; k += 32) dh[(size_t)row * K + k] = h[k] <= 0.f ? 0.f : g * w[k];
+    }
+  }
+  if (!t) return;
+  if (lane == 0) sq[warp] = e * e;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float s = 0.f;
+    for (int i = 0; i < 8; ++i) s += sq[i];
+    loss_part[blockIdx.x] = s;
+  }
+}
+
+// Weight and bias gradients of up to kDwLayers layers in one launch:
+// part[c][woff ..] = X^T dY and part[c][boff ..] = column sums of dY over chunk c
+// of `rows` rows (blockIdx.y), tiles of all layers along blockIdx.x.
+constexpr int kDwLayers = 8;
+struct DwTable {
+  int layers;
+  int first[kDwLayers + 1];  // tiles before each layer
+  int M[kDwLayers], N[kDwLayers];
+  int64_t woff[kDwLayers], boff[kDwLayers];
+  const float* x[kDwLayers];
+  const float* dy[kDwLayers];
+};
+__global__ void __launch_bounds__(256)
+    k_dw(const __grid_constant__ DwTable d, int n, int rows, int64_t n_params, float* __restrict__ part) {
+  __shared__ Tile32 t;
+  int l = 0;
+  while (l + 1 < d.layers && d.first[l + 1] <= (int)blockIdx.x) ++l;
+  const int M = d.M[l], N = d.N[l], nt = (N + GT - 1) / GT, id = (int)blockIdx.x - d.first[l];
+  const int m0 = id / nt * GT, n0 = id % nt * GT;
+  const float *X = d.x[l], *D = d.dy[l];
+  const int r0 = blockIdx.y * rows, r1 = min(n, r0 + rows);
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
+  float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+  float col = 0.f;  // threads 0 .. 31 of the first row of tiles: a column's sum
+  for (int k0 = r0; k0 < r1; k0 += GK) {
+    float ra[GT * GK / 256], rb[GT * GK / 256];
+#pragma unroll
+    for (int i = 0; i < GT * GK / 256; ++i) {
+      const int r = ly + 8 * i;
+      const bool in = k0 + r < r1;
+      ra[i] = in && m0 + lx < M ? X[(size_t)(k0 + r) * M + m0 + lx] : 0.f;
+      rb[i] = in && n0 + lx < N ? D[(size_t)(k0 + r) * N + n0 + lx] : 0.f;
+    }
+    if (k0 != r0) __syncthreads();  // the previous step has been read
+#pragma unroll
+    for (int i = 0; i < GT * GK / 256; ++i) {
+      t.a[ly + 8 * i][lx] = ra[i];
+      t.b[ly + 8 * i][lx] = rb[i];
+    }
+    __syncthreads();
+    const int kn = min(GK, r1 - k0);
+    tile_fma(t, kn, tx, ty, acc);
+    if (m0 == 0 && threadIdx.x < GT)
+      for (int k = 0; k < kn; ++k) col += t.b[k][threadIdx.x];
+  }
+  float* P = part + blockIdx.y * n_params;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int r = m0 + ty + 16 * i, c = n0 + tx + 16 * j;
+      if (r < M && c < N) P[d.woff[l] + (int64_t)r * N + c] = acc[i][j];
+    }
+  if (m0 == 0 && threadIdx.x < GT && n0 + (int)threadIdx.x < N) P[d.boff[l] + n0 + threadIdx.x] = col;
+}
+
+// g[i] = sum of the chunks' parts in order; the last block adds up the loss.
+__global__ void __launch_bounds__(256)
+    k_reduce_parts(const float* __restrict__ part, int chunks, int64_t n_params, float* __restrict__ g,
+                   const float* __restrict__ loss_part, int n_loss, int n, float* __restrict__ loss) {
+  if (blockIdx.x + 1 < gridDim.x) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_params) return;
+    float s = 0.f;
+    for (int c = 0; c < chunks; ++c) s += part[c * n_params + i];
+    g[i] = s;
+    return;
+  }
+  __shared__ float sm[256];
+  float s = 0.f;
+  for (int i = threadIdx.x; i < n_loss; i += 256) s += loss_part[i];
+  sm[threadIdx.x] = s;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if ((int)threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
     __syncthreads();
   }
-  if (row < M && col < N) {
-    size_t o = (size_t)row * N + col;
-    if (bias) acc += bias[col];
-    if (beta != 0.f) acc += beta * C[o];
-    if (relu) acc = acc > 0.f ? acc : 0.f;
-    C[o] = acc;
-  }
+  if (threadIdx.x == 0) *loss = sm[0] / (float)n;
 }
 
 // Inference layer in bf16: weights and inputs rounded to bf16, FP32 accumulate.
@@ -101,35 +267,6 @@ __global__ void k_to_bf16(const float* __restrict__ x, __nv_bfloat16* __restrict
   if (i < n) y[i] = __float2bfloat16(x[i]);
 }
 
-// dY = 2 (y - t) / n for the MSE loss; also accumulates the loss sum.
-__global__ void k_mse_grad(const float* __restrict__ y, const float* __restrict__ t, float* __restrict__ dy, int n,
-                           float* loss) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  float l = 0.f;
-  if (i < n) {
-    float d = y[i] - t[i];
-    dy[i] = 2.f * d / (float)n;
-    l = d * d;
-  }
-  for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, l / (float)n);
-}
-
-// dZ *= (H > 0) (ReLU backward, H is the post-activation)
-__global__ void k_relu_back(float* __restrict__ dz, const float* __restrict__ h, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && h[i] <= 0.f) dz[i] = 0.f;
-}
-
-// db[j] = sum_b dZ[b, j]
-__global__ void k_colsum(const float* __restrict__ dz, float* __restrict__ db, int M, int N) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= N) return;
-  float s = 0.f;
-  for (int b = 0; b < M; ++b) s += dz[(size_t)b * N + j];
-  db[j] = s;
-}
-
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
                        int64_t n, float lr, float b1, float b2, float eps, float c1, float c2) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -140,12 +277,6 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float
   m[i] = mi;
   v[i] = vi;
   p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-}
-
-void sgemm(const float* A, const float* B, float* C, const float* bias, int M, int N, int K, int ta, int tb, int relu,
-           float beta, cudaStream_t s) {
-  dim3 blk(TB, TB), grd((N + TB - 1) / TB, (M + TB - 1) / TB);
-  k_sgemm<<<grd, blk, 0, s>>>(A, B, C, bias, M, N, K, ta, tb, relu, beta);
 }
 
 }  // namespace
@@ -167,11 +298,18 @@ struct pq_mlp {
   std::vector<float*> dact;
   float* d_t = nullptr;
   float* d_loss = nullptr;
+  float* d_part = nullptr;       // weight-gradient chunks (chunks(cap) x n_params)
+  float* d_loss_part = nullptr;  // squared errors per k_head block
   __nv_bfloat16* d_wbf = nullptr;
   __nv_bfloat16* d_xb[2] = {nullptr, nullptr};
 };
 
 namespace {
+
+// The batch in chunks of rows for the weight gradients: 128 rows each, and at
+// most 64 chunks.
+int chunk_rows(int n) { return std::max(128, ((n + 63) / 64 + GT - 1) / GT * GT); }
+int chunk_count(int n) { return (n + chunk_rows(n) - 1) / chunk_rows(n); }
 
 void free_ws(pq_mlp* m) {
   for (auto p : m->act) cudaFree(p);
@@ -179,9 +317,11 @@ void free_ws(pq_mlp* m) {
   m->act.clear();
   m->dact.clear();
   cudaFree(m->d_t);
+  cudaFree(m->d_part);
+  cudaFree(m->d_loss_part);
   cudaFree(m->d_xb[0]);
   cudaFree(m->d_xb[1]);
-  m->d_t = nullptr;
+  m->d_t = m->d_part = m->d_loss_part = nullptr;
   m->d_xb[0] = m->d_xb[1] = nullptr;
   m->cap = 0;
 }
@@ -200,6 +340,10 @@ int ensure_ws(pq_mlp* m, int n) {
   }
   int wmax = std::max(m->n_in, m->hidden);
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_t, sizeof(float) * (size_t)n);
+  // (a smaller batch has no more chunks than this one)
+  if (e == cudaSuccess)
+    e = cudaMalloc((void**)&m->d_part, sizeof(float) * (size_t)m->n_params * (size_t)std::min(64, (n + 127) / 128));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_loss_part, sizeof(float) * (size_t)((n + 7) / 8));
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_xb[0], sizeof(__nv_bfloat16) * (size_t)n * wmax);
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_xb[1], sizeof(__nv_bfloat16) * (size_t)n * wmax);
   if (e != cudaSuccess) {
@@ -210,32 +354,51 @@ int ensure_ws(pq_mlp* m, int n) {
   return PQ_OK;
 }
 
-// Forward pass (FP32) over n rows already in act[0].
-void forward(pq_mlp* m, int n) {
+// Forward pass (FP32) over n rows already in act[0]; with targets (d_t), the
+// output layer's kernel also starts the backward pass.
+void forward(pq_mlp* m, int n, bool train) {
   const int L = (int)m->din.size();
-  for (int l = 0; l < L; ++l)
-    sgemm(m->act[l], m->d_p + m->woff[l], m->act[l + 1], m->d_p + m->boff[l], n, m->dout[l], m->din[l], 0, 0,
-          l + 1 < L ? 1 : 0, 0.f, m->ctx->stream);
+  cudaStream_t s = m->ctx->stream;
+  for (int l = 0; l + 1 < L; ++l) {
+    dim3 grid((n + GT - 1) / GT, (m->dout[l] + GT - 1) / GT);
+    k_layer<false><<<grid, 256, 0, s>>>(m->act[l], m->d_p + m->woff[l], m->d_p + m->boff[l], nullptr, m->act[l + 1], n,
+                                        m->dout[l], m->din[l]);
+  }
+  k_head<<<(n + 7) / 8, 256, 0, s>>>(m->act[L - 1], m->d_p + m->woff[L - 1], m->d_p + m->boff[L - 1], n, m->din[L - 1],
+                                     m->act[L], train ? m->d_t : nullptr, m->dact[L], L > 1 ? m->dact[L - 1] : nullptr,
+                                     m->d_loss_part);
 }
 
-// Backward pass: gradients of the mean squared error into d_g; returns with
-// the loss in d_loss (device).
+// Backward pass after forward(train): gradients of the mean squared error into
+// d_g; returns with the loss in d_loss (device).
 void backward(pq_mlp* m, int n) {
   const int L = (int)m->din.size();
   cudaStream_t s = m->ctx->stream;
-  cudaMemsetAsync(m->d_loss, 0, sizeof(float), s);
-  k_mse_grad<<<(n + 255) / 256, 256, 0, s>>>(m->act[L], m->d_t, m->dact[L], n, m->d_loss);
-  for (int l = L - 1; l >= 0; --l) {
-    // dW_l = act[l]^T dact[l+1];  db_l = colsum(dact[l+1])
-    sgemm(m->act[l], m->dact[l + 1], m->d_g + m->woff[l], nullptr, m->din[l], m->dout[l], n, 1, 0, 0, 0.f, s);
-    k_colsum<<<(m->dout[l] + 127) / 128, 128, 0, s>>>(m->dact[l + 1], m->d_g + m->boff[l], n, m->dout[l]);
-    if (l > 0) {
-      // dact[l] = dact[l+1] W_l^T, masked by ReLU of act[l]
-      sgemm(m->dact[l + 1], m->d_p + m->woff[l], m->dact[l], nullptr, n, m->din[l], m->dout[l], 0, 1, 0, 0.f, s);
-      int64_t sz = (int64_t)n * m->din[l];
-      k_relu_back<<<(unsigned)((sz + 255) / 256), 256, 0, s>>>(m->dact[l], m->act[l], sz);
-    }
+  // dact[l] = dact[l+1] W_l^T, masked by ReLU of act[l] (k_head wrote dact[L-1])
+  for (int l = L - 2; l > 0; --l) {
+    dim3 grid((n + GT - 1) / GT, (m->din[l] + GT - 1) / GT);
+    k_layer<true><<<grid, 256, 0, s>>>(m->dact[l + 1], m->d_p + m->woff[l], nullptr, m->act[l], m->dact[l], n,
+                                       m->din[l], m->dout[l]);
   }
+  const int chunks = chunk_count(n);
+  for (int l0 = 0; l0 < L; l0 += kDwLayers) {
+    DwTable d;
+    d.layers = std::min(kDwLayers, L - l0);
+    d.first[0] = 0;
+    for (int i = 0; i < d.layers; ++i) {
+      const int l = l0 + i;
+      d.M[i] = m->din[l];
+      d.N[i] = m->dout[l];
+      d.woff[i] = m->woff[l];
+      d.boff[i] = m->boff[l];
+      d.x[i] = m->act[l];
+      d.dy[i] = m->dact[l + 1];
+      d.first[i + 1] = d.first[i] + ((d.M[i] + GT - 1) / GT) * ((d.N[i] + GT - 1) / GT);
+    }
+    k_dw<<<dim3(d.first[d.layers], chunks), 256, 0, s>>>(d, n, chunk_rows(n), m->n_params, m->d_part);
+  }
+  k_reduce_parts<<<(unsigned)((m->n_params + 255) / 256) + 1, 256, 0, s>>>(m->d_part, chunks, m->n_params, m->d_g,
+                                                                         m->d_loss_part, (n + 7) / 8, n, m->d_loss);
 }
 
 }  // namespace
@@ -339,7 +502,7 @@ int pq_mlp_gradients(pq_mlp* m, const float* X, const float* y, int64_t n, float
   cudaStream_t s = m->ctx->stream;
   cudaMemcpyAsync(m->act[0], X, sizeof(float) * n * m->n_in, cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(m->d_t, y, sizeof(float) * n, cudaMemcpyHostToDevice, s);
-  forward(m, (int)n);
+  forward(m, (int)n, true);
   backward(m, (int)n);
   cudaMemcpyAsync(grad, m->d_g, sizeof(float) * m->n_params, cudaMemcpyDeviceToHost, s);
   float l = 0;
@@ -390,7 +553,7 @@ int pq_mlp_train(pq_mlp* m, const float* X, const float* y, int64_t n, int epoch
     if (e != cudaSuccess) break;
     for (int64_t i0 = 0; i0 + b <= n; i0 += b) {
       k_gather_rows<<<(b + 127) / 128, 128, 0, s>>>(dX, dY, dperm + i0, b, m->n_in, m->act[0], m->d_t);
-      forward(m, b);
+      forward(m, b, true);
       backward(m, b);
       ++m->step;
       float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
@@ -418,7 +581,7 @@ int pq_mlp_predict(pq_mlp* m, const float* X, int64_t n, float* out, int bf16) {
   const int L = (int)m->din.size();
   cudaMemcpyAsync(m->act[0], X, sizeof(float) * n * m->n_in, cudaMemcpyHostToDevice, s);
   if (!bf16) {
-    forward(m, (int)n);
+    forward(m, (int)n, false);
   } else {
     k_to_bf16<<<(unsigned)((m->n_params + 255) / 256), 256, 0, s>>>(m->d_p, m->d_wbf, m->n_params);
     k_to_bf16<<<(unsigned)((n * m->n_in + 255) / 256), 256, 0, s>>>(m->act[0], m->d_xb[0], n * m->n_in);

@@ -191,3 +191,25 @@ def test_learned_plan_gains_over_flop_plan(pq, O):
         v = np.asarray(r).reshape(-1, order="F")
         assert np.max(np.abs(v - sv)) <= 1e-6 * np.max(np.abs(sv))
     be.close()
+
+
+@pytest.mark.parametrize("n,hidden,layers", [(1, 1, 1), (33, 7, 2), (127, 64, 1), (129, 32, 3), (1024, 128, 3),
+                                             (1000, 130, 4), (8193, 33, 9)])
+def test_mlp_gradients_shapes(pq, be, n, hidden, layers):
+    """Tile edges in every dimension, one to 64 row chunks, more layers than one
+    weight-gradient launch takes, and the loss; FP32 against FP64.  The longest
+    chain of roundings is 160 rows of a chunk, 64 chunks and 130-wide products
+    through 9 layers and back, under 2600 steps of 2^-24 = 1.6e-4 of sums of
+    absolute values of order the largest gradient."""
+    import mlp_oracle as MO
+    from pqgb300.costmodel import CostModel
+
+    m = CostModel(be, hidden=hidden, layers=layers, seed=n)
+    rng = np.random.default_rng(n)
+    X = rng.standard_normal((n, 5)).astype(np.float32)
+    y = rng.standard_normal(n).astype(np.float32)
+    g, loss = m.gradients(X, y)
+    lo, go = MO.loss_and_grad(m.params.astype(np.float64), X, y, 5, hidden, layers)
+    assert abs(loss - lo) <= 1e-5 * max(1.0, abs(lo))
+    assert np.max(np.abs(g - go)) <= 1.6e-4 * max(1.0, np.max(np.abs(go)))
+    m.close()

@@ -36,6 +36,11 @@ namespace pq {
 namespace {
 
 constexpr int kSkThreads = 128;
+// FP64 rows are bound by the multiply-adds (2 per clock and SM), so what counts
+// is that every SM gets the same number of rows: 2^16 rows in blocks of 128 are 3
+// or 4 per SM, in blocks of 64 they are 6 or 7 (2^18 amplitudes, 4 qubits: 72 ->
+// 41 us, 2^20: 135 -> 128), and that K is not padded (2^20, 3 qubits: 135 -> 62).
+constexpr int kSkThreads64 = 64;
 
 struct SkinnyDesc {
   int64_t R, Z;
@@ -227,7 +232,7 @@ __global__ void __launch_bounds__(kSkThreads)
 
 // Every other mix of element types (complex128 results in FP64).
 template <typename TX, typename TC, int KMAX>
-__global__ void __launch_bounds__(kSkThreads)
+__global__ void __launch_bounds__(kSkThreads64)
     k_skinny(const TX* __restrict__ X, const void* __restrict__ W, TC* __restrict__ C,
              const __grid_constant__ SkinnyDesc d) {
   using R = typename std::conditional<std::is_same<TC, double2>::value, double, float>::type;
@@ -236,14 +241,14 @@ __global__ void __launch_bounds__(kSkThreads)
   extern __shared__ __align__(16) unsigned char w_raw[];
   R2* w = reinterpret_cast<R2*>(w_raw);
   const int nw = (d.N + 3) / 4 * 4;
-  const int64_t step = (int64_t)gridDim.x * kSkThreads;
+  const int64_t step = (int64_t)gridDim.x * kSkThreads64;
   for (int64_t z = blockIdx.y; z < d.Z; z += gridDim.y) {
     int64_t zx, zw, zc;
     batch_offsets(d, z, zx, zw, zc);
     if (z != blockIdx.y) __syncthreads();  // the previous W has been read
-    for (int t = threadIdx.x; t < KMAX * nw; t += kSkThreads) w[t] = w_value<R>(d, W, zw, t / nw, t % nw);
+    for (int t = threadIdx.x; t < KMAX * nw; t += kSkThreads64) w[t] = w_value<R>(d, W, zw, t / nw, t % nw);
     __syncthreads();
-    for (int64_t r = (int64_t)blockIdx.x * kSkThreads + threadIdx.x; r < d.R; r += step) {
+    for (int64_t r = (int64_t)blockIdx.x * kSkThreads64 + threadIdx.x; r < d.R; r += step) {
       int64_t xo, co;
       row_offsets(d, r, xo, co);
       xo += zx;
@@ -258,8 +263,10 @@ __global__ void __launch_bounds__(kSkThreads)
         for (int n = 0; n < 4; ++n) acc[n] = czero(R());
 #pragma unroll
         for (int k = 0; k < KMAX; ++k) {
+          if (k < d.K) {  // (uniform: no FP64 time for padding)
 #pragma unroll
-          for (int n = 0; n < 4; ++n) cfma(acc[n], a[k], w[k * nw + n0 + n]);
+            for (int n = 0; n < 4; ++n) cfma(acc[n], a[k], w[k * nw + n0 + n]);
+          }
         }
 #pragma unroll
         for (int n = 0; n < 4; ++n)
@@ -272,19 +279,19 @@ __global__ void __launch_bounds__(kSkThreads)
 // Row blocks by batch index; persistent-style over the blocks that fit an SM at
 // the kernels' register counts (complex64: 64 registers at K <= 16, 46 or fewer
 // below; FP64: 96).
-dim3 sk_grid(const SkinnyDesc& d, int per_sm) {
+dim3 sk_grid(const SkinnyDesc& d, int per_sm, int threads = kSkThreads) {
   const int64_t y = std::min<int64_t>(d.Z, 65535);
   const int64_t x = std::max<int64_t>(1, 152 * per_sm / y);
-  return dim3((unsigned)std::min<int64_t>((d.R + kSkThreads - 1) / kSkThreads, x), (unsigned)y);
+  return dim3((unsigned)std::min<int64_t>((d.R + threads - 1) / threads, x), (unsigned)y);
 }
 
 template <typename TX, typename TC>
 cudaError_t launch_mixed(const void* X, const void* W, void* C, const SkinnyDesc& d, cudaStream_t s) {
   const size_t col = (size_t)((d.N + 3) / 4 * 4) * (std::is_same<TC, double2>::value ? 16 : 8);
   if (d.K <= 4)
-    k_skinny<TX, TC, 4><<<sk_grid(d, 10), kSkThreads, 4 * col, s>>>((const TX*)X, W, (TC*)C, d);
+    k_skinny<TX, TC, 4><<<sk_grid(d, 18, kSkThreads64), kSkThreads64, 4 * col, s>>>((const TX*)X, W, (TC*)C, d);
   else
-    k_skinny<TX, TC, 16><<<sk_grid(d, 5), kSkThreads, 16 * col, s>>>((const TX*)X, W, (TC*)C, d);
+    k_skinny<TX, TC, 16><<<sk_grid(d, 9, kSkThreads64), kSkThreads64, 16 * col, s>>>((const TX*)X, W, (TC*)C, d);
   return cudaGetLastError();
 }
 

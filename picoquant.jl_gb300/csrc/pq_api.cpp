@@ -92,12 +92,11 @@ static void convert_host(const void* src, int sdt, void* dst, int ddt, int64_t n
 }
 
 int check_status(Ctx* ctx) {
-  int h = 0;
-  cudaError_t e = cudaMemcpyAsync(&h, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  cudaError_t e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "stream synchronize");
+  const int h = *static_cast<volatile int*>(ctx->h_status);
   if (h != 0) {
-    cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);
+    *static_cast<volatile int*>(ctx->h_status) = 0;  // (nothing is in flight)
     return fail(ctx, PQ_ERR_DEVICE, "a kernel reported device status " + std::to_string(h));
   }
   return PQ_OK;
@@ -143,9 +142,11 @@ int pq_ctx_create(int device, int precision, pq_ctx** out) {
   }
   uint64_t thr = UINT64_MAX;
   cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &thr);
-  e = cudaMalloc((void**)&ctx->d_status, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(ctx->d_status, 0, sizeof(int));
+  e = cudaHostAlloc((void**)&ctx->h_status, sizeof(int), cudaHostAllocMapped);
+  if (e == cudaSuccess) *ctx->h_status = 0;
+  if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&ctx->d_status, ctx->h_status, 0);
   if (e != cudaSuccess) {
+    if (ctx->h_status) cudaFreeHost(ctx->h_status);
     cudaMemPoolDestroy(ctx->pool);
     cudaStreamDestroy(ctx->stream);
     delete c;
@@ -165,7 +166,7 @@ int pq_ctx_destroy(pq_ctx* c) {
   cudaStreamSynchronize(ctx->stream);
   if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
   if (ctx->stage_done) cudaEventDestroy(ctx->stage_done);
-  cudaFree(ctx->d_status);
+  cudaFreeHost(ctx->h_status);
   cudaMemPoolDestroy(ctx->pool);
   cudaStreamDestroy(ctx->stream);
   delete c;

@@ -122,7 +122,11 @@ struct Ctx {
   size_t elem = 16;   // bytes per stored element
   cudaStream_t stream = nullptr;
   cudaMemPool_t pool = nullptr;
-  int* d_status = nullptr;          // device status word (0 = ok)
+  // Status word (0 = ok) in mapped pinned host memory: kernels write it through
+  // d_status when a wait expires, the host reads h_status after a synchronise
+  // (a copy of it per synchronising call took 8 us).
+  int* h_status = nullptr;
+  int* d_status = nullptr;
   std::unordered_map<int64_t, Tensor> tensors;
   std::string last_error;
   int64_t mem_cap = 0;

@@ -62,7 +62,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 // Records an expired wait in the context's status word (read by the host at
 // the next synchronising call, where it becomes PQ_ERR_DEVICE).
 __device__ __forceinline__ void report_timeout(int* status) {
-  if (status) atomicExch(status, kStatusTcTimeout);
+  if (status) atomicExch_system(status, kStatusTcTimeout);
 }
 // 1D bulk copy global -> shared (16-byte aligned addresses, size a multiple
 // of 16), completing as transaction bytes on `bar`.

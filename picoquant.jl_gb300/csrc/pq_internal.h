@@ -206,10 +206,23 @@ cudaError_t launch_scatter(const void* src, const CopyJob* d_jobs, int n, cudaSt
 // Batched leaf gather for slicing: out[x + xs*b] = in[x_off(x) + slice_off(s0+b)]
 // for b < nb, where x runs over `d` (csa = input strides of the kept modes)
 // and the slice offset is the mixed-radix digits of (s0+b) over the sliced
-// dims times their strides in `in`.  Entries with s0+b >= s_end are zero.
-cudaError_t launch_slice_gather(int dt, const void* in, void* out, const GenericDesc& d,
-                                int nsl, const int64_t* sl_dim, const int64_t* sl_stride,
-                                int64_t s0, int64_t nb, int64_t s_end, cudaStream_t stream);
+// dims times their strides in `in`.  Entries with s0+b >= s_end are zero.  Up
+// to kSliceGroup leaves per launch, leaf m on blocks [blk[m], blk[m+1]) with the
+// descriptor jobs[job0 + m] (device table).
+struct SliceJob {
+  GenericDesc d;
+  int nsl, dt;
+  int64_t dim[kMaxModes], stride[kMaxModes];
+};
+constexpr int kSliceGroup = 64;
+struct SliceGroup {
+  int n, job0;
+  int blk[kSliceGroup + 1];
+  const void* in[kSliceGroup];
+  void* out[kSliceGroup];
+};
+cudaError_t launch_slice_gather(const SliceGroup& g, const SliceJob* d_jobs, int64_t s0, int64_t nb, int64_t s_end,
+                                cudaStream_t stream);
 // Neumaier FP64 sum over the batch axis: acc[e] += sum_b X[e + n*b].
 // FP64 squared 2-norm of n complex elements into *out (device); `part`
 // holds 2 * norm2_blocks(n) doubles of scratch.

@@ -320,54 +320,57 @@ cudaError_t launch_scatter(const void* src, const CopyJob* d_jobs, int n, cudaSt
   return cudaGetLastError();
 }
 
-struct SliceTab {
-  int n;
-  int64_t dim[kMaxModes];
-  int64_t stride[kMaxModes];
-};
-
 template <typename T>
-__global__ void __launch_bounds__(kGenThreads)
-    k_slice_gather(const T* in, T* out, const __grid_constant__ GenericDesc d,
-                   const __grid_constant__ SliceTab st, int64_t s0, int64_t nb, int64_t s_end) {
-  const int64_t total = d.csize * nb;
-  const int64_t step = (int64_t)gridDim.x * blockDim.x;
-  pdl_wait();
-  pdl_trigger();
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += step) {
-    int64_t b = e / d.csize;
-    int64_t x = e - b * d.csize;
+__device__ __forceinline__ void slice_copy(const T* in, T* out, const SliceJob& j, int64_t first, int64_t step,
+                                           int64_t s0, int64_t nb, int64_t s_end) {
+  const int64_t total = j.d.csize * nb;
+  for (int64_t e = first; e < total; e += step) {
+    int64_t b = e / j.d.csize;
+    int64_t x = e - b * j.d.csize;
     int64_t s = s0 + b, so = 0;
     if (s >= s_end) {
       out[e] = T{0, 0};
       continue;
     }
-    for (int i = 0; i < st.n; ++i) {
-      int64_t q = s / st.dim[i];
-      so += (s - q * st.dim[i]) * st.stride[i];
+    for (int i = 0; i < j.nsl; ++i) {
+      int64_t q = s / j.dim[i];
+      so += (s - q * j.dim[i]) * j.stride[i];
       s = q;
     }
     int64_t oa, ob;
-    decode2<false>(x, d, oa, ob);
+    decode2<false>(x, j.d, oa, ob);
     out[e] = in[so + oa];
   }
 }
 
-cudaError_t launch_slice_gather(int dt, const void* in, void* out, const GenericDesc& d, int nsl,
-                                const int64_t* sl_dim, const int64_t* sl_stride, int64_t s0, int64_t nb,
-                                int64_t s_end, cudaStream_t stream) {
-  SliceTab st;
-  st.n = nsl;
-  for (int i = 0; i < nsl && i < kMaxModes; ++i) {
-    st.dim[i] = sl_dim[i];
-    st.stride[i] = sl_stride[i];
-  }
-  const int grid = grid_for(d.csize * nb, kGenThreads);
-  if (dt == PQ_C128)
-    return launch_pdl(k_slice_gather<double2>, dim3(grid), dim3(kGenThreads), 0, stream, (const double2*)in,
-                      (double2*)out, d, st, s0, nb, s_end);
-  return launch_pdl(k_slice_gather<float2>, dim3(grid), dim3(kGenThreads), 0, stream, (const float2*)in, (float2*)out, d,
-                    st, s0, nb, s_end);
+// The sliced leaves of one batch in one launch (one launch each took 12 of the
+// 67 launches of a small sliced amplitude): a block finds its leaf in the prefix
+// table and copies that leaf's descriptor into shared memory while the launch
+// before still runs.
+__global__ void __launch_bounds__(kGenThreads)
+    k_slice_gather(const __grid_constant__ SliceGroup g, const SliceJob* __restrict__ jobs, int64_t s0, int64_t nb,
+                   int64_t s_end) {
+  __shared__ SliceJob job;
+  int m = 0;
+  while (m + 1 < g.n && g.blk[m + 1] <= (int)blockIdx.x) ++m;
+  const int* src = reinterpret_cast<const int*>(jobs + g.job0 + m);
+  for (int t = threadIdx.x; t < (int)(sizeof(SliceJob) / sizeof(int)); t += blockDim.x)
+    reinterpret_cast<int*>(&job)[t] = src[t];
+  __syncthreads();
+  pdl_wait();
+  pdl_trigger();
+  const int64_t step = (int64_t)(g.blk[m + 1] - g.blk[m]) * blockDim.x;
+  const int64_t first = (int64_t)(blockIdx.x - g.blk[m]) * blockDim.x + threadIdx.x;
+  if (job.dt == PQ_C128)
+    slice_copy(static_cast<const double2*>(g.in[m]), static_cast<double2*>(g.out[m]), job, first, step, s0, nb, s_end);
+  else
+    slice_copy(static_cast<const float2*>(g.in[m]), static_cast<float2*>(g.out[m]), job, first, step, s0, nb, s_end);
+}
+
+cudaError_t launch_slice_gather(const SliceGroup& g, const SliceJob* d_jobs, int64_t s0, int64_t nb, int64_t s_end,
+                                cudaStream_t stream) {
+  if (g.n <= 0 || g.blk[g.n] <= 0) return cudaSuccess;
+  return launch_pdl(k_slice_gather, dim3((unsigned)g.blk[g.n]), dim3(kGenThreads), 0, stream, g, d_jobs, s0, nb, s_end);
 }
 
 // Neumaier compensated accumulation of one value into (s, c).

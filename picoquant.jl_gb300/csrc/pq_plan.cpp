@@ -294,9 +294,9 @@ struct pq_plan {
   Compiled scp;
   std::vector<int> sl_leaf_of;             // SSA leaf -> index into sl_leafbuf (or -1)
   std::vector<size_t> sl_leaf_off;         // offsets of gathered leaves in arena (after scp arena)
-  std::vector<GenericDesc> sl_leaf_desc;
-  std::vector<std::vector<int64_t>> sl_leaf_sdim, sl_leaf_sstride;
-  std::vector<int> sl_leaf_dt;             // storage type of each gathered leaf
+  std::vector<SliceJob> sl_jobs;           // descriptors of the gathered leaves
+  void* d_sljobs = nullptr;                // the same on the device
+  size_t d_sljobs_bytes = 0;
   size_t sl_total_bytes = 0;
   double* d_acc = nullptr;  // 2*n complex sum + 2*n compensation
   int64_t out_elems = 0;
@@ -608,19 +608,20 @@ int launch_all(pq_plan* p, const Compiled& cp, const std::vector<const void*>& l
   return PQ_OK;
 }
 
-// Copy a compiled plan's grouped-step descriptors to the device (once per
-// compile, outside any stream capture).
-int upload_groups(pq_plan* p, const Compiled& c, void** buf, size_t* bytes) {
+// Copy a table of descriptors (grouped steps, gathered leaves) to the device
+// (once per compile, outside any stream capture).
+template <typename T>
+int upload_table(pq_plan* p, const std::vector<T>& v, void** buf, size_t* bytes) {
   Ctx* ctx = p->ctx;
   if (*buf) dev_free(ctx, *buf, *bytes);
   *buf = nullptr;
   *bytes = 0;
-  if (c.gdesc.empty()) return PQ_OK;
-  const size_t b = c.gdesc.size() * sizeof(GenericDesc);
+  if (v.empty()) return PQ_OK;
+  const size_t b = v.size() * sizeof(T);
   int st = dev_alloc(ctx, b, buf);
   if (st) return st;
   *bytes = b;
-  cudaError_t e = cudaMemcpyAsync(*buf, c.gdesc.data(), b, cudaMemcpyHostToDevice, ctx->stream);
+  cudaError_t e = cudaMemcpyAsync(*buf, v.data(), b, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "plan descriptor upload");
   return PQ_OK;
@@ -699,7 +700,7 @@ int pq_plan_create(pq_ctx* c, int n_leaves, const int32_t* leaf_ranks, const int
     delete p;
     return fail(ctx, PQ_ERR_INVALID, "plan_create: " + err);
   }
-  const int st = upload_groups(p, p->cp, &p->d_gdesc, &p->d_gdesc_bytes);
+  const int st = upload_table(p, p->cp.gdesc, &p->d_gdesc, &p->d_gdesc_bytes);
   if (st) {
     delete p;
     return st;
@@ -718,6 +719,7 @@ int pq_plan_destroy(pq_plan* p) {
   if (p->d_acc) dev_free(ctx, p->d_acc, (size_t)p->out_elems * 32);
   if (p->d_gdesc) dev_free(ctx, p->d_gdesc, p->d_gdesc_bytes);
   if (p->d_sgdesc) dev_free(ctx, p->d_sgdesc, p->d_sgdesc_bytes);
+  if (p->d_sljobs) dev_free(ctx, p->d_sljobs, p->d_sljobs_bytes);
   delete p;
   return PQ_OK;
 }
@@ -870,10 +872,7 @@ int prepare_sliced(pq_plan* p, const int64_t* leaf_ids, int n_sliced, const int3
     std::vector<char> bl(p->nleaves, 0);
     p->sl_leaf_of.assign(p->nleaves, -1);
     p->sl_leaf_off.clear();
-    p->sl_leaf_desc.clear();
-    p->sl_leaf_sdim.clear();
-    p->sl_leaf_sstride.clear();
-    p->sl_leaf_dt.clear();
+    p->sl_jobs.clear();
     for (int i = 0; i < p->nleaves; ++i) {
       const auto& lab = p->leaf_labels[i];
       bool hit = false;
@@ -890,11 +889,13 @@ int prepare_sliced(pq_plan* p, const int64_t* leaf_ids, int n_sliced, const int3
         strides[j] = acc;
         acc *= p->leaf_dims[i][j];
       }
-      GenericDesc g;
-      std::memset(&g, 0, sizeof(g));
+      SliceJob job;
+      std::memset(&job, 0, sizeof(job));
+      GenericDesc& g = job.d;
       int64_t ksz = 1;
       for (size_t j = 0; j < lab.size(); ++j) {
         if (std::find(S.begin(), S.end(), lab[j]) != S.end()) continue;
+        if (g.nc == kMaxModes) return fail(ctx, PQ_ERR_UNSUPPORTED, "run_sliced: a sliced leaf has too many modes");
         ll[i].push_back(lab[j]);
         g.cdim[g.nc] = p->leaf_dims[i][j];
         g.csa[g.nc] = strides[j];
@@ -905,17 +906,15 @@ int prepare_sliced(pq_plan* p, const int64_t* leaf_ids, int n_sliced, const int3
       g.csize = ksz;
       g.ksize = 1;
       ll[i].push_back(beta);
-      std::vector<int64_t> sd, ss;
-      for (int l : S) {
-        sd.push_back(p->label_dims[l]);
-        auto it = std::find(lab.begin(), lab.end(), l);
-        ss.push_back(it == lab.end() ? 0 : strides[it - lab.begin()]);
+      job.nsl = (int)S.size();
+      job.dt = p->cp.dt[i];
+      for (int q = 0; q < job.nsl; ++q) {
+        job.dim[q] = p->label_dims[S[q]];
+        auto it = std::find(lab.begin(), lab.end(), S[q]);
+        job.stride[q] = it == lab.end() ? 0 : strides[it - lab.begin()];
       }
-      p->sl_leaf_of[i] = (int)p->sl_leaf_desc.size();
-      p->sl_leaf_desc.push_back(g);
-      p->sl_leaf_sdim.push_back(sd);
-      p->sl_leaf_sstride.push_back(ss);
-      p->sl_leaf_dt.push_back(p->cp.dt[i]);
+      p->sl_leaf_of[i] = (int)p->sl_jobs.size();
+      p->sl_jobs.push_back(job);
     }
     std::vector<int> outl = p->out_labels;
     outl.push_back(beta);
@@ -933,13 +932,14 @@ int prepare_sliced(pq_plan* p, const int64_t* leaf_ids, int n_sliced, const int3
     std::string err;
     if (!compile(ctx, ll, ldims, p->steps_in, outl, order, &bl, p->scp, err, &p->cp.dt))
       return fail(ctx, PQ_ERR_INVALID, "run_sliced: " + err);
-    const int su = upload_groups(p, p->scp, &p->d_sgdesc, &p->d_sgdesc_bytes);
+    int su = upload_table(p, p->scp.gdesc, &p->d_sgdesc, &p->d_sgdesc_bytes);
+    if (!su) su = upload_table(p, p->sl_jobs, &p->d_sljobs, &p->d_sljobs_bytes);
     if (su) return su;
     // gathered leaf buffers after the arena
     size_t off = align_up(p->scp.arena_bytes, 256);
-    for (size_t j = 0; j < p->sl_leaf_desc.size(); ++j) {
+    for (const SliceJob& j : p->sl_jobs) {
       p->sl_leaf_off.push_back(off);
-      off += align_up((size_t)p->sl_leaf_desc[j].csize * batch * elem_bytes(p->sl_leaf_dt[j]), 256);
+      off += align_up((size_t)j.d.csize * batch * elem_bytes(j.dt), 256);
     }
     p->sl_total_bytes = off;
     p->sl_labels = S;
@@ -955,16 +955,33 @@ int prepare_sliced(pq_plan* p, const int64_t* leaf_ids, int n_sliced, const int3
 
 cudaError_t gather_batch(pq_plan* p, const std::vector<const void*>& ptrs, int64_t s0, int64_t nb) {
   Ctx* ctx = p->ctx;
-  for (int i = 0; i < p->nleaves; ++i) {
-    int j = p->sl_leaf_of[i];
-    if (j < 0) continue;
-    cudaError_t e = launch_slice_gather(p->sl_leaf_dt[j], ptrs[i], (char*)p->arena + p->sl_leaf_off[j],
-                                        p->sl_leaf_desc[j], (int)p->sl_labels.size(), p->sl_leaf_sdim[j].data(),
-                                        p->sl_leaf_sstride[j].data(), s0, p->sl_batch, s0 + nb, ctx->stream);
+  SliceGroup g;
+  g.n = 0;
+  g.job0 = 0;
+  int blocks = 0;
+  auto flush = [&]() {
+    if (!g.n) return cudaSuccess;
+    g.blk[g.n] = blocks;
+    cudaError_t e = launch_slice_gather(g, (const SliceJob*)p->d_sljobs, s0, p->sl_batch, s0 + nb, ctx->stream);
     ctx->launches++;
-    if (e != cudaSuccess) return e;
+    g.job0 += g.n;
+    g.n = 0;
+    blocks = 0;
+    return e;
+  };
+  for (int i = 0; i < p->nleaves; ++i) {  // (jobs are in leaf order)
+    const int j = p->sl_leaf_of[i];
+    if (j < 0) continue;
+    g.blk[g.n] = blocks;
+    g.in[g.n] = ptrs[i];
+    g.out[g.n] = (char*)p->arena + p->sl_leaf_off[j];
+    blocks += (int)std::min<int64_t>((p->sl_jobs[j].d.csize * p->sl_batch + 255) / 256, 152);
+    if (++g.n == kSliceGroup) {
+      cudaError_t e = flush();
+      if (e != cudaSuccess) return e;
+    }
   }
-  return cudaSuccess;
+  return flush();
 }
 
 }  // namespace

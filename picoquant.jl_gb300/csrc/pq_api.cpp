@@ -102,6 +102,15 @@ int check_status(Ctx* ctx) {
   return PQ_OK;
 }
 
+int download(Ctx* ctx, void* dst, const void* src, size_t bytes, const char* what) {
+  const bool staged = bytes <= kDownBytes;
+  cudaError_t e = cudaMemcpyAsync(staged ? ctx->h_down : dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, what);
+  const int st = check_status(ctx);
+  if (!st && staged) std::memcpy(dst, ctx->h_down, bytes);
+  return st;
+}
+
 }  // namespace pq
 
 using namespace pq;
@@ -142,8 +151,11 @@ int pq_ctx_create(int device, int precision, pq_ctx** out) {
   }
   uint64_t thr = UINT64_MAX;
   cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &thr);
-  e = cudaHostAlloc((void**)&ctx->h_status, sizeof(int), cudaHostAllocMapped);
-  if (e == cudaSuccess) *ctx->h_status = 0;
+  e = cudaHostAlloc((void**)&ctx->h_status, 256 + kDownBytes, cudaHostAllocMapped);
+  if (e == cudaSuccess) {
+    *ctx->h_status = 0;
+    ctx->h_down = reinterpret_cast<unsigned char*>(ctx->h_status) + 256;
+  }
   if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&ctx->d_status, ctx->h_status, 0);
   if (e != cudaSuccess) {
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
@@ -337,16 +349,9 @@ int pq_load_tensor_data(pq_ctx* c, int64_t id, void* dst, int64_t n_elems, int d
   const Tensor& t = it->second;
   if (!dst || n_elems < t.size) return fail(ctx, PQ_ERR_INVALID, "load_tensor_data: destination too small");
   if (dtype != PQ_C64 && dtype != PQ_C128) return fail(ctx, PQ_ERR_INVALID, "load_tensor_data: bad dtype");
-  cudaError_t e;
-  if (t.dtype == dtype) {
-    e = cudaMemcpyAsync(dst, t.ptr, t.bytes, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "load_tensor_data download");
-    return check_status(ctx);
-  }
+  if (t.dtype == dtype) return download(ctx, dst, t.ptr, t.bytes, "load_tensor_data download");
   std::vector<unsigned char> tmp(t.bytes);
-  e = cudaMemcpyAsync(tmp.data(), t.ptr, t.bytes, cudaMemcpyDeviceToHost, ctx->stream);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "load_tensor_data download");
-  int st = check_status(ctx);
+  int st = download(ctx, tmp.data(), t.ptr, t.bytes, "load_tensor_data download");
   if (st) return st;
   convert_host(tmp.data(), t.dtype, dst, dtype, t.size);
   return PQ_OK;
@@ -722,11 +727,10 @@ int pq_gather_elements(pq_ctx* c, int64_t id, const int64_t* idx, int64_t n, voi
   if (e == cudaSuccess) e = launch_gather(T.dtype, T.ptr, (const int64_t*)d_idx, n, d_out, ctx->stream);
   ctx->launches += 1;
   std::vector<unsigned char> tmp((size_t)n * eb);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(tmp.data(), d_out, tmp.size(), cudaMemcpyDeviceToHost, ctx->stream);
+  st = e == cudaSuccess ? download(ctx, tmp.data(), d_out, tmp.size(), "gather_elements")
+                        : cuda_fail(ctx, e, "gather_elements");
   dev_free(ctx, d_idx, (size_t)n * 8);
   dev_free(ctx, d_out, (size_t)n * eb);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "gather_elements");
-  st = check_status(ctx);
   if (st) return st;
   convert_host(tmp.data(), T.dtype, out, dtype, n);
   return PQ_OK;

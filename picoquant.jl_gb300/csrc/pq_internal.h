@@ -140,6 +140,10 @@ struct Ctx {
   void* d_stage = nullptr;
   size_t d_stage_cap = 0;
   cudaEvent_t stage_done = nullptr;
+  // small downloads pass through this pinned buffer (kDownBytes behind the
+  // status word): a copy into pageable memory is staged and waited for inside
+  // the driver
+  void* h_down = nullptr;
   // Mixed-precision contexts store tensors of at most this many elements as
   // complex128 (gates, per-qubit tensors: cheap, and their rounding would
   // dominate the error) and larger ones as complex64.
@@ -159,6 +163,10 @@ inline int storage_dtype(const Ctx* ctx, int64_t n) {
 // Status helpers: set the context error and return the code.
 int fail(Ctx* ctx, int code, const std::string& msg);
 int cuda_fail(Ctx* ctx, cudaError_t e, const char* what);
+
+// Copy device memory to the host and wait for the stream (status checked).
+constexpr size_t kDownBytes = 1 << 18;
+int download(Ctx* ctx, void* dst, const void* src, size_t bytes, const char* what);
 
 // Stream-ordered device allocation accounted against the context cap.
 int dev_alloc(Ctx* ctx, size_t bytes, void** p);

@@ -288,7 +288,7 @@ struct pq_mlp {
   std::vector<int64_t> woff, boff;       // offsets in the flat parameter buffer
   int64_t n_params = 0;
   float* d_p = nullptr;
-  float* d_g = nullptr;
+  float* d_g = nullptr;  // gradients, then the loss (read together)
   float* d_m = nullptr;
   float* d_v = nullptr;
   int64_t step = 0;
@@ -436,10 +436,10 @@ int pq_mlp_create(pq_ctx* c, int n_in, int hidden, int hidden_layers, uint64_t s
     for (int64_t i = 0; i < (int64_t)m->din[l] * m->dout[l]; ++i) h[m->woff[l] + i] = U(rng);
   }
   cudaError_t e = cudaMalloc((void**)&m->d_p, sizeof(float) * m->n_params);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_g, sizeof(float) * m->n_params);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_g, sizeof(float) * (m->n_params + 1));
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_m, sizeof(float) * m->n_params);
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_v, sizeof(float) * m->n_params);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_loss, sizeof(float));
+  if (e == cudaSuccess) m->d_loss = m->d_g + m->n_params;
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_wbf, sizeof(__nv_bfloat16) * m->n_params);
   if (e == cudaSuccess) e = cudaMemcpy(m->d_p, h.data(), sizeof(float) * m->n_params, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(m->d_m, 0, sizeof(float) * m->n_params);
@@ -449,7 +449,6 @@ int pq_mlp_create(pq_ctx* c, int n_in, int hidden, int hidden_layers, uint64_t s
     cudaFree(m->d_g);
     cudaFree(m->d_m);
     cudaFree(m->d_v);
-    cudaFree(m->d_loss);
     cudaFree(m->d_wbf);
     delete m;
     return cuda_fail(ctx, e, "mlp create");
@@ -466,7 +465,6 @@ int pq_mlp_destroy(pq_mlp* m) {
   cudaFree(m->d_g);
   cudaFree(m->d_m);
   cudaFree(m->d_v);
-  cudaFree(m->d_loss);
   cudaFree(m->d_wbf);
   delete m;
   return PQ_OK;
@@ -504,14 +502,14 @@ int pq_mlp_gradients(pq_mlp* m, const float* X, const float* y, int64_t n, float
   cudaMemcpyAsync(m->d_t, y, sizeof(float) * n, cudaMemcpyHostToDevice, s);
   forward(m, (int)n, true);
   backward(m, (int)n);
-  cudaMemcpyAsync(grad, m->d_g, sizeof(float) * m->n_params, cudaMemcpyDeviceToHost, s);
-  float l = 0;
-  cudaMemcpyAsync(&l, m->d_loss, sizeof(float), cudaMemcpyDeviceToHost, s);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(m->ctx, e, "mlp gradients");
-  st = check_status(m->ctx);
-  if (loss) *loss = l;
-  return st;
+  std::vector<float> h((size_t)m->n_params + 1);
+  st = download(m->ctx, h.data(), m->d_g, sizeof(float) * h.size(), "mlp gradients");
+  if (st) return st;
+  std::memcpy(grad, h.data(), sizeof(float) * m->n_params);
+  if (loss) *loss = h[(size_t)m->n_params];
+  return PQ_OK;
 }
 
 int pq_mlp_train(pq_mlp* m, const float* X, const float* y, int64_t n, int epochs, int batch, float lr,
@@ -595,10 +593,9 @@ int pq_mlp_predict(pq_mlp* m, const float* X, int64_t n, float* out, int bf16) {
       cur = 1 - cur;
     }
   }
-  cudaMemcpyAsync(out, m->act[L], sizeof(float) * n, cudaMemcpyDeviceToHost, s);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(m->ctx, e, "mlp predict");
-  return check_status(m->ctx);
+  return download(m->ctx, out, m->act[L], sizeof(float) * n, "mlp predict");
 }
 
 }  // extern "C"

@@ -1130,9 +1130,7 @@ int pq_sliced_result(pq_plan* p, double* out, int64_t n) {
   Ctx* ctx = p->ctx;
   if (!p->d_acc || n < p->out_elems) return fail(ctx, PQ_ERR_INVALID, "sliced_result: no result or buffer too small");
   std::vector<double> h((size_t)p->out_elems * 4);
-  cudaError_t e = cudaMemcpyAsync(h.data(), p->d_acc, h.size() * 8, cudaMemcpyDeviceToHost, ctx->stream);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "sliced_result copy");
-  int st = check_status(ctx);
+  int st = download(ctx, h.data(), p->d_acc, h.size() * 8, "sliced_result copy");
   if (st) return st;
   for (int64_t i = 0; i < 2 * p->out_elems; ++i) out[i] = h[i] + h[2 * p->out_elems + i];
   return PQ_OK;

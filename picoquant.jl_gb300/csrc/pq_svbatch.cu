@@ -540,11 +540,8 @@ int pq_svbatch_execute(pq_svbatch* b, double* amps_out) {
   if (e != cudaSuccess) return cuda_fail(ctx, e, "svbatch_execute: graph launch");
   ctx->launches += b->kernel_launches;
   std::vector<double2> h((size_t)b->total_amps);
-  if (b->total_amps) {
-    e = cudaMemcpyAsync(h.data(), b->d_amps, h.size() * sizeof(double2), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "svbatch_execute: read amplitudes");
-  }
-  int st = check_status(ctx);
+  int st = b->total_amps ? download(ctx, h.data(), b->d_amps, h.size() * sizeof(double2), "svbatch_execute: read amplitudes")
+                         : check_status(ctx);
   if (st) return st;
   for (size_t a = 0; a < h.size(); ++a) {
     amps_out[2 * a] = h[(size_t)b->perm[a]].x;

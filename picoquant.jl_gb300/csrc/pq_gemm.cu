@@ -8,9 +8,8 @@
 // Tile shapes (256 threads, each owning R x S results):
 //   square  BM=64,  BN=64,  R=4,  S=4   general pairs (complex128 results also
 //                                        32 x 32 and 16 x 16)
-//   tall    BM=256, BN=16,  R=16, S=1   narrow N (e.g. a big boundary absorbing
-//                                        a qubit with few open bonds)
-//   wide    BM=16,  BN=256, R=1,  S=16  narrow M
+// Complex64 results with a narrow side (a big boundary absorbing a qubit with
+// few open bonds) go row by row (launch_tall).
 // The next K tile's gathered global loads are issued into registers before
 // the current tile is consumed from shared memory (double buffering).
 #include "pq_types.cuh"
@@ -222,13 +221,7 @@ static cudaError_t gemm_launch(const void* A, const void* B, void* C, const Gemm
 }
 
 template <typename TA, typename TB, typename TC>
-static cudaError_t gemm_shape(int shape, const void* A, const void* B, void* C, const GemmDesc& d, cudaStream_t s) {
-  // the narrow tiles need 32 KiB of complex64 staging; complex128 results
-  // (FP64 accumulation, twice the tile bytes) use square tiles
-  if constexpr (std::is_same<TC, float2>::value) {
-    if (shape == GEMM_TALL) return gemm_launch<TA, TB, TC, 256, 16, 16, 1>(A, B, C, d, s);
-    if (shape == GEMM_WIDE) return gemm_launch<TA, TB, TC, 16, 256, 1, 16>(A, B, C, d, s);
-  }
+static cudaError_t gemm_shape(const void* A, const void* B, void* C, const GemmDesc& d, cudaStream_t s) {
   // Complex128 results: FP64 multiply-adds (2 per clock and SM) bound every
   // tile, so the tile is the one with the least work on the busiest SM, tiles
   // there times tile area, the larger at a tie.  M = 1024, N = 16, K = 128: 16
@@ -246,10 +239,10 @@ static cudaError_t gemm_shape(int shape, const void* A, const void* B, void* C, 
 }
 
 template <typename TA, typename TB>
-static cudaError_t gemm_launch_c(int tc, int shape, const void* A, const void* B, void* C, const GemmDesc& d,
+static cudaError_t gemm_launch_c(int tc, const void* A, const void* B, void* C, const GemmDesc& d,
                                  cudaStream_t s) {
-  if (tc == PQ_C128) return gemm_shape<TA, TB, double2>(shape, A, B, C, d, s);
-  return gemm_shape<TA, TB, float2>(shape, A, B, C, d, s);
+  if (tc == PQ_C128) return gemm_shape<TA, TB, double2>(A, B, C, d, s);
+  return gemm_shape<TA, TB, float2>(A, B, C, d, s);
 }
 
 int gemm_tile_shape(const GemmDesc& d) {
@@ -261,11 +254,11 @@ int gemm_tile_shape(const GemmDesc& d) {
 cudaError_t launch_gemm(int ta, int tb, int tc, const void* A, const void* B, void* C, const GemmDesc& d,
                         cudaStream_t stream) {
   if (d.M * d.N * d.Z == 0) return cudaSuccess;
-  const int shape = gemm_tile_shape(d);
-  if (ta == PQ_C128 && tb == PQ_C128) return gemm_launch_c<double2, double2>(tc, shape, A, B, C, d, stream);
-  if (ta == PQ_C128) return gemm_launch_c<double2, float2>(tc, shape, A, B, C, d, stream);
-  if (tb == PQ_C128) return gemm_launch_c<float2, double2>(tc, shape, A, B, C, d, stream);
-  return gemm_launch_c<float2, float2>(tc, shape, A, B, C, d, stream);
+  if (tc == PQ_C64 && gemm_tile_shape(d) != GEMM_SQUARE) return launch_tall(ta, tb, A, B, C, d, stream);
+  if (ta == PQ_C128 && tb == PQ_C128) return gemm_launch_c<double2, double2>(tc, A, B, C, d, stream);
+  if (ta == PQ_C128) return gemm_launch_c<double2, float2>(tc, A, B, C, d, stream);
+  if (tb == PQ_C128) return gemm_launch_c<float2, double2>(tc, A, B, C, d, stream);
+  return gemm_launch_c<float2, float2>(tc, A, B, C, d, stream);
 }
 
 }  // namespace pq

@@ -197,6 +197,8 @@ cudaError_t launch_generic_group(const GenericGroup& g, const GenericDesc* d_des
 bool skinny_eligible(int precision, const GemmDesc& d);
 cudaError_t launch_skinny(int ta, int tb, int tc, const void* A, const void* B, void* C,
                           const GemmDesc& d, cudaStream_t stream);
+// Complex64 results with one narrow side (gemm_tile_shape), any K (pq_skinny.cu).
+cudaError_t launch_tall(int ta, int tb, const void* A, const void* B, void* C, const GemmDesc& d, cudaStream_t stream);
 // out[c] = in[base + sum_i idx_i * stride_i] over `d` (uses csa as input
 // strides, C storage column-major), converting tin -> tout.
 cudaError_t launch_permute(int tin, int tout, const void* in, int64_t base, void* out,

@@ -55,6 +55,16 @@ struct SkinnyDesc {
 };
 static_assert(sizeof(SkinnyDesc) + 64 <= 32764, "kernel parameters");
 
+// Offset of x over n mixed-radix modes.
+__host__ __device__ inline int64_t offset_of(int64_t x, int n, const int64_t* dim, const int64_t* s) {
+  int64_t o = 0;
+  for (int i = 0; i < n; ++i) {
+    o += x % dim[i] * s[i];
+    x /= dim[i];
+  }
+  return o;
+}
+
 // Offsets of batch index z in X, W and C.
 __device__ __forceinline__ void batch_offsets(const SkinnyDesc& d, int64_t z, int64_t& zx, int64_t& zw, int64_t& zc) {
   zx = zw = zc = 0;
@@ -276,6 +286,109 @@ __global__ void __launch_bounds__(kSkThreads64)
   }
 }
 
+// Narrow pairs with a longer K (complex64 results): one thread per row again, up
+// to 8 columns of W per block (blockIdx.y; with 16 the compensated sums leave
+// three blocks per SM: 2^16 rows, N = 16, K = 128 in 82 us against 60), K in
+// steps of 128 through shared memory.  Each 16 terms are summed in FP32 and
+// folded into a compensated sum per column, as the tiled GEMM does, so the error
+// does not grow with K.  The tile of 256 x 16 it replaces had half the SMs idle
+// and one K step of 16 in flight per block: 2^15 rows, N = 8, K = 128: 84 -> 33 us.
+constexpr int kTallK = 128;
+struct TallDesc {
+  GemmDesc g;  // rows m in X (sa) and C (sc), columns n in W (sb) and C
+  int w64;
+};
+template <typename TX, int NQ, int KV>
+__global__ void __launch_bounds__(kSkThreads)
+    k_tall(const TX* __restrict__ X, const void* __restrict__ W, float2* __restrict__ C,
+           const __grid_constant__ TallDesc d) {
+  constexpr int NP = 2 * NQ;
+  __shared__ __align__(16) float w[kTallK * NP * 4];
+  __shared__ int64_t kx[kTallK], kw[kTallK];
+  __shared__ int64_t nw[4 * NQ], cn[4 * NQ];
+  const GemmDesc& g = d.g;
+  const int n0 = blockIdx.y * 4 * NQ, N = (int)min((int64_t)4 * NQ, g.N - n0);
+  const int64_t r = (int64_t)blockIdx.x * kSkThreads + threadIdx.x;
+  const bool in = r < g.M;
+  if (threadIdx.x < 4 * NQ) {
+    const bool col = (int)threadIdx.x < N;
+    nw[threadIdx.x] = col ? offset_of(n0 + threadIdx.x, g.nn, g.ndim, g.nsb) : 0;
+    cn[threadIdx.x] = col ? offset_of(n0 + threadIdx.x, g.nn, g.ndim, g.nsc) : 0;
+  }
+  const int64_t xr = in ? offset_of(r, g.nm, g.mdim, g.msa) : 0, cr = in ? offset_of(r, g.nm, g.mdim, g.msc) : 0;
+  for (int64_t z = blockIdx.z; z < g.Z; z += gridDim.z) {
+    const TX* x = X + xr + offset_of(z, g.nz, g.zdim, g.zsa);
+    const int64_t zw = offset_of(z, g.nz, g.zdim, g.zsb);
+    KahanC acc[4 * NQ];
+#pragma unroll
+    for (int n = 0; n < 4 * NQ; ++n) kahan_init(acc[n]);
+    for (int64_t k0 = 0; k0 < g.K; k0 += kTallK) {
+      const int kn = (int)min((int64_t)kTallK, g.K - k0), kp = (kn + 15) / 16 * 16;
+      __syncthreads();  // the previous step has been read
+      for (int k = threadIdx.x; k < kn; k += kSkThreads) {
+        kx[k] = offset_of(k0 + k, g.nk, g.kdim, g.ksa);
+        kw[k] = offset_of(k0 + k, g.nk, g.kdim, g.ksb);
+      }
+      __syncthreads();
+      for (int t = threadIdx.x; t < kp * 4 * NQ; t += kSkThreads) {
+        const int k = t / (4 * NQ), n = t % (4 * NQ);
+        float2 v = make_float2(0.f, 0.f);
+        if (k < kn && n < N) {
+          const int64_t o = zw + kw[k] + nw[n];
+          v = d.w64 ? cvt<float>(static_cast<const double2*>(W)[o]) : static_cast<const float2*>(W)[o];
+        }
+        w_store(w, NP, k, n, v);
+      }
+      __syncthreads();
+      if (!in) continue;
+      for (int kc = 0; kc < kn; kc += 16) {
+        TX a[16];
+#pragma unroll
+        for (int k = 0; k < 16; k += KV) {
+          if (kc + k < kn) {
+            load_run<KV>(x + kx[kc + k], &a[k]);
+          } else {
+#pragma unroll
+            for (int u = 0; u < KV; ++u) a[k + u].x = a[k + u].y = 0;
+          }
+        }
+        F2 ax[16], ay[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          ax[k] = f2_dup((float)a[k].x);
+          ay[k] = f2_dup((float)a[k].y);
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+          float2 o[4];
+          four_columns<16>(ax, ay, w + kc * NP * 4, NP, 4 * q, o);
+#pragma unroll
+          for (int n = 0; n < 4; ++n) kahan_add(acc[4 * q + n], o[n]);
+        }
+      }
+    }
+    if (in) {
+      float2* c = C + cr + offset_of(z, g.nz, g.zdim, g.zsc);
+#pragma unroll
+      for (int n = 0; n < 4 * NQ; ++n)
+        if (n < N) c[cn[n]] = kahan_value(acc[n]);
+    }
+  }
+}
+
+template <typename TX, int KV>
+cudaError_t launch_tall_kv(const void* X, const void* W, void* C, const TallDesc& d, cudaStream_t s) {
+  const int nq = d.g.N <= 4 ? 1 : 2;
+  const int64_t gx = (d.g.M + kSkThreads - 1) / kSkThreads, gy = (d.g.N + 4 * nq - 1) / (4 * nq);
+  if (gx > 2147483647LL || gy > 65535) return cudaErrorInvalidConfiguration;
+  const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)std::min<int64_t>(d.g.Z, 65535));
+  if (nq == 1)
+    k_tall<TX, 1, KV><<<grid, kSkThreads, 0, s>>>((const TX*)X, W, (float2*)C, d);
+  else
+    k_tall<TX, 2, KV><<<grid, kSkThreads, 0, s>>>((const TX*)X, W, (float2*)C, d);
+  return cudaGetLastError();
+}
+
 // Row blocks by batch index; persistent-style over the blocks that fit an SM at
 // the kernels' register counts (complex64: 64 registers at K <= 16, 46 or fewer
 // below; FP64: 96).
@@ -316,16 +429,6 @@ int log2_exact(int64_t v) {
   int l = 0;
   while ((int64_t(1) << l) < v) ++l;
   return (int64_t(1) << l) == v ? l : -1;
-}
-
-// Offset of x over n mixed-radix modes.
-int64_t offset_of(int64_t x, int n, const int64_t* dim, const int64_t* s) {
-  int64_t o = 0;
-  for (int i = 0; i < n; ++i) {
-    o += x % dim[i] * s[i];
-    x /= dim[i];
-  }
-  return o;
 }
 
 }  // namespace
@@ -406,6 +509,44 @@ cudaError_t launch_skinny(int ta, int tb, int tc, const void* A, const void* B, 
   if (d.K <= 4) return launch_k<4>(kv, X, W, C, d, stream);
   if (d.K <= 8) return launch_k<8>(kv, X, W, C, d, stream);
   return launch_k<16>(kv, X, W, C, d, stream);
+}
+
+cudaError_t launch_tall(int ta, int tb, const void* A, const void* B, void* C, const GemmDesc& g, cudaStream_t stream) {
+  TallDesc d;
+  d.g = g;
+  const bool a_big = g.M >= g.N;
+  if (!a_big) {
+    std::swap(d.g.M, d.g.N);
+    std::swap(d.g.nm, d.g.nn);
+    for (int i = 0; i < kMaxModes; ++i) {
+      d.g.mdim[i] = g.ndim[i];
+      d.g.msa[i] = g.nsb[i];
+      d.g.msc[i] = g.nsc[i];
+      d.g.ndim[i] = g.mdim[i];
+      d.g.nsb[i] = g.msa[i];
+      d.g.nsc[i] = g.msc[i];
+      std::swap(d.g.ksa[i], d.g.ksb[i]);
+      std::swap(d.g.zsa[i], d.g.zsb[i]);
+    }
+    std::swap(A, B);
+    std::swap(ta, tb);
+  }
+  d.w64 = tb == PQ_C128;
+  if (d.g.M * d.g.N * d.g.Z == 0) return cudaSuccess;
+  if (ta == PQ_C128) return launch_tall_kv<double2, 1>(A, B, C, d, stream);
+  // aligned runs along K, as for the skinny pairs
+  int kv = d.g.nk > 0 && d.g.ksa[0] == 1 ? 4 : 1;
+  auto limit = [&](int64_t v) {
+    while (kv > 1 && v % kv) kv /= 2;
+  };
+  if (kv > 1) limit(d.g.kdim[0]);
+  while (kv > 1 && (uintptr_t)A % (8 * kv)) kv /= 2;
+  for (int i = 1; i < d.g.nk; ++i) limit(d.g.ksa[i]);
+  for (int i = 0; i < d.g.nm; ++i) limit(d.g.msa[i]);
+  for (int i = 0; i < d.g.nz; ++i) limit(d.g.zsa[i]);
+  if (kv == 4) return launch_tall_kv<float2, 4>(A, B, C, d, stream);
+  if (kv == 2) return launch_tall_kv<float2, 2>(A, B, C, d, stream);
+  return launch_tall_kv<float2, 1>(A, B, C, d, stream);
 }
 
 }  // namespace pq

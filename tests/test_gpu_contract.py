@@ -190,3 +190,57 @@ def test_complex128_small_results(pq, m, n, k):
     got = be.load_tensor_data("c").reshape(m, n)
     be.close()
     assert np.all(np.abs(got - A @ B) <= 2 * (2 * k + 6) * 2.0 ** -53 * (np.abs(A) @ np.abs(B)))
+
+
+@pytest.mark.parametrize("m,n,k,z", [(4100, 9, 33, 1), (20000, 16, 130, 1), (8, 5000, 64, 1), (31, 3000, 257, 1),
+                                     (300, 20, 1000, 1), (1000, 12, 100, 3), (70000, 8, 18, 1), (129, 24, 4000, 2)])
+@pytest.mark.parametrize("order", ["mk", "km", "k4", "k2"])
+def test_complex64_narrow_long_k(pq, m, n, k, z, order):
+    """Complex64 pairs with one narrow side and K past 16: K steps of 128 with a
+    ragged last one, 1 to 31 columns in blocks of 4 or 8, either side
+    narrow, batches; the long operand contiguous along its rows, along K, or
+    in K runs of 4 or 2 (wide loads).  Sixteen terms at a time in FP32 (18
+    roundings of the real and imaginary sums), folded with compensation (3
+    more): within 21 2^-24 of the sum of absolute products per component."""
+    rng = np.random.default_rng(m + n + k)
+
+    def crand(*s):
+        return (rng.standard_normal(s) + 1j * rng.standard_normal(s)).astype(np.complex64)
+
+    big, small = max(m, n), min(m, n)
+    r = {"mk": 0, "km": 0, "k4": 4, "k2": 2}[order]
+    if r and k % r:
+        pytest.skip("K is not a multiple of the run")
+    X, W = crand(big, k, z), crand(k, small, z)
+    if order == "mk":
+        T, ix, iw = X, [-1, 1, 2], [1, -2, 2]
+    elif order == "km":
+        T, ix, iw = X.transpose(1, 0, 2), [1, -1, 2], [1, -2, 2]
+    else:
+        T, ix, iw = X.reshape(big, k // r, r, z).transpose(2, 0, 1, 3), [3, -1, 1, 2], [1, 3, -2, 2]
+    be = pq.GB300Backend(pq.PREC_C64, small_elems=0)
+    Wt = W if not r else W.reshape(k // r, r, small, z)
+    import ctypes as C
+
+    from pqgb300 import _lib as L
+
+    ids = {-1: 0, -2: 1, 1: 2, 2: 3, 3: 4}
+    ops = [(T, ix), (Wt, iw)] if m >= n else [(Wt, iw), (T, ix)]
+    for name, (t, _) in zip("ab", ops):
+        be.save_tensor_data(name, t)
+    h = C.c_void_p()
+    dims = [big, small, k // r if r else k, z, r or 1]
+    out = [0, 1, 3]
+    L.check(be.lib.pq_plan_create(be.ctx, 2, L.arr(C.c_int32, [t.ndim for t, _ in ops]),
+                                  L.arr(C.c_int32, [ids[x] for _, l in ops for x in l]), 5, L.arr(C.c_int64, dims), 1,
+                                  L.arr(C.c_int32, [0, 1]), 3, L.arr(C.c_int32, out), C.byref(h)), be.ctx, "plan_create")
+    f = (C.c_double * 8)()
+    L.check(be.lib.pq_plan_step_features(h, f), be.ctx, "features")
+    assert int(f[6]) == 1  # the GEMM class
+    L.check(be.lib.pq_plan_execute(h, L.arr(C.c_int64, [be.id_of("a"), be.id_of("b")]), be.id_of("r")), be.ctx, "run")
+    got = be.load_tensor_data("r")
+    be.lib.pq_plan_destroy(h)
+    be.close()
+    ref = np.einsum("mkz,knz->mnz", X.astype(np.complex128), W.astype(np.complex128), optimize=True)
+    bound = 2 * 21 * 2.0 ** -24 * np.einsum("mkz,knz->mnz", np.abs(X), np.abs(W), optimize=True)
+    assert np.all(np.abs(got - ref) <= bound)

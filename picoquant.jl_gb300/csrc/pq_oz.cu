@@ -23,7 +23,7 @@
 // The split's error, at most 2^-31 K of the scales and near 2^-32 of the result
 // on random pairs, is far below the complex64 rounding (3.5e-8 of max |C|
 // either way), so 8 products give what five bf16 slices gave with 15: the pair
-// M = 2^18, N = K = 256 takes 1.0 ms instead of 1.47.
+// M = 2^18, N = K = 256 takes 0.92 ms instead of 1.47.
 //
 // Complex128 results keep five bf16 slices
 //   s0 = rint(x 2^7) 2^-7,  s_i = rint((x - s0 - .. - s_{i-1}) 2^{7(i+1)}) 2^{-7(i+1)}
@@ -83,8 +83,10 @@
 //                  16-byte core-matrix row;
 //     warps 10-17  epilogue, once per tile: Cr from TMEM lanes 0-63, Ci from
 //                  lanes 64-127; the levels are combined with an error-free
-//                  two-sum, scaled by 2^(ea+eb) and scattered through the
-//                  result index map.
+//                  two-sum (128-wide complex64 tiles park the sums, in shared
+//                  memory or the spare TMEM block, and release the
+//                  accumulators first), scaled by 2^(ea+eb) and scattered
+//                  through the result index map.
 // Every mbarrier wait is bounded; on expiry the kernel records an error in the
 // context's status word and runs to the end (TMEM is always released).
 #include <cuda_bf16.h>
@@ -136,12 +138,24 @@ constexpr int kHalfUp = 15;
 // fits the 24-bit significand while a + b + 1 + log2 K <= 24.
 __host__ __device__ constexpr int first_bits(int64_t k, int side) { return k <= (side == 0 ? 128 : 256) ? 8 : 7; }
 
-template <int TN, int S>
+// 128-wide tiles of three slices with complex64 results: the epilogue parks a
+// tile's sums in shared memory (and stores whole complex values from there),
+// and the fourth TMEM block lets the next tile's MMAs of levels 2 and up start
+// before the epilogue has read this one.  Against parking in the fourth block
+// the issuer's wait for the epilogue fell from 17 % of its time to 1 %: 24.3k ->
+// 21.6k cycles per 64 x 128 x 256 tile, with the ring cut from five stages to
+// three.
+template <typename TC, int TN, int S>
+__host__ __device__ constexpr bool oz_park() {
+  return TN == 128 && Sl<S>::n == 3 && sizeof(TC) == 8;
+}
+
+template <int TN, int S, bool PARK>
 struct OzCfg {
   static constexpr int kBTile = TN * TK;                                   // 16-bit values per B plane tile
   static constexpr uint32_t b_bytes = Sl<S>::planes * kBTile * 2;          // B planes of one K tile
   static constexpr uint32_t stage_bytes = Sl<S>::n * kStackBytes + b_bytes;
-  static constexpr int stages = Sl<S>::half ? (TN == 128 ? 5 : 6) : ((TN == 128 && S >= 4) ? 3 : 4);
+  static constexpr int stages = PARK ? 3 : (Sl<S>::half ? 6 : ((TN == 128 && S >= 4) ? 3 : 4));
   // 16-wide tiles: one MMA per A slice i against B slices 0 .. met(i)-1 side
   // by side (N = 16 met(i)), every slice pair in its own TMEM region
   static constexpr bool narrow = TN == 16;
@@ -467,16 +481,19 @@ __global__ void __launch_bounds__(256) k_oz_pack(const T* __restrict__ X, uint16
   }
 }
 
-template <int TN, int S>
+constexpr int kParkPitch = 129;  // floats per parked row: rows on different banks
+
+template <int TN, int S, bool PARK>
 struct alignas(1024) OzSmem {
-  unsigned char stage[OzCfg<TN, S>::stages][OzCfg<TN, S>::stage_bytes];  // A stacks, then B planes
+  unsigned char stage[OzCfg<TN, S, PARK>::stages][OzCfg<TN, S, PARK>::stage_bytes];  // A stacks, then B planes
   int64_t koff[kMaxK];                                                        // A's K offsets
-  uint64_t full[OzCfg<TN, S>::stages];
-  uint64_t empty[OzCfg<TN, S>::stages];
+  uint64_t full[OzCfg<TN, S, PARK>::stages];
+  uint64_t empty[OzCfg<TN, S, PARK>::stages];
   uint64_t accf[2];  // accumulator set b holds a finished tile
   uint64_t acce[2];  // the epilogue has read accumulator set b
   uint64_t drain;
   uint32_t tmem_base;
+  float park[PARK ? 2 * kRows * kParkPitch : 1];  // [Re, Im][row][column] sums of a tile
 };
 
 // a + b = s + e exactly (Knuth's two-sum).
@@ -540,6 +557,18 @@ __host__ __device__ constexpr int conv_values() {
 // Generic-proxy shared-memory writes made visible to the tensor core's reads.
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// True when `v` holds in every thread of the epilogue warps, all of which call
+// it (named barrier 1; shared-memory accesses before it are seen after it).
+__device__ __forceinline__ bool epilogue_all(bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n barrier.cta.red.and.pred p, 1, %2, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(r)
+      : "r"((uint32_t)v), "n"(32 * kEpiWarps)
+      : "memory");
+  return r != 0;
+}
+
 // The ring position `by` stages on (by <= kStages), with its phase.
 template <int kStages>
 __device__ __forceinline__ void next_stage(int& s, uint32_t& ph, int by = 1) {
@@ -556,13 +585,14 @@ __global__ void __launch_bounds__(kThreads, 1)
               const __grid_constant__ GemmDesc d, const int64_t* __restrict__ cm_tab,
               const int64_t* __restrict__ cn_tab, const int* __restrict__ ea, const int* __restrict__ eb,
               int64_t mtiles, int64_t ntiles, int64_t ktiles, int kvec, int* status) {
-  using CF = OzCfg<TN, S>;
+  constexpr bool kPark = oz_park<TC, TN, S>();
+  using CF = OzCfg<TN, S, kPark>;
   constexpr int kSlices = Sl<S>::n, kPlanes = Sl<S>::planes, kPairs = Sl<S>::pairs;
   constexpr int kStages = CF::stages;
   constexpr uint32_t kTmemCols = CF::tmem_cols;
   constexpr int kSets = CF::acc_sets;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  OzSmem<TN, S>& sm = *reinterpret_cast<OzSmem<TN, S>*>(smem_raw);
+  OzSmem<TN, S, kPark>& sm = *reinterpret_cast<OzSmem<TN, S, kPark>*>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t ntot = ntiles * mtiles * d.Z;
 
@@ -621,25 +651,92 @@ __global__ void __launch_bounds__(kThreads, 1)
     int s = 0;       // ring stage and its phase
     uint32_t ph = 0;
     int64_t t = 0;   // tiles of this CTA
-    for (int64_t tile = blockIdx.x; tile < ntot && ok; tile += gridDim.x, ++t) {
-      // the epilogue has read this accumulator set's previous tile
-      const int b = (int)(t % kSets);
-      if (!__all_sync(0xffffffffu, mbar_wait(&sm.acce[b], (uint32_t)(((t / kSets) & 1) ^ 1)))) {
-        ok = false;
-        break;
+    // The MMAs of the K tile in stage `st`, levels lo .. hi (2: the rest).  The
+    // MMAs of one A operand follow each other: the first fills the tensor
+    // core's A buffer from shared memory, the others use it (an M = N = 128 MMA
+    // reads 8 KB in its 64 cycles, all of the SM's shared-memory bandwidth; with
+    // A kept, kHalf reads 88 KB per K tile instead of 128 KB: 7 % of the wide
+    // pair's time).  `first` overwrites the levels; l2 is the column of level 2.
+    auto issue = [&](int st, int lo, int hi, bool first, uint32_t set, uint32_t l2) {
+      const uint32_t sa = smem_u32(sm.stage[st]) >> 4;
+      constexpr uint32_t BOFF = (kSlices * kStackBytes) >> 4;
+#pragma unroll
+      for (int i = 0; i < kSlices; ++i) {
+#pragma unroll
+        for (int part = 0; part < 2; ++part) {
+          // part 0: [Ar; Ai] . Br = [Ar.Br ; Ai.Br]; part 1: [Ai; -Ar]
+          // with A negated . Bi = [-Ai.Bi ; Ar.Bi]
+          const uint64_t x = desc_at(sa + ((i * kStackBytes + part * 8 * 128) >> 4), ALBO, SBO);
+          const int j0 = i >= lo ? 0 : lo - i;                              // first slice of B
+          const int j1 = hi < 2 && Sl<S>::met(i) > hi + 1 - i ? hi + 1 - i : Sl<S>::met(i);  // past the last
+#pragma unroll
+          for (int j = 0; j < Sl<S>::met(0); ++j) {
+            if (j < j0 || j >= j1) continue;
+            const int lv = i + j < 2 ? i + j : 2;
+            // the first MMA into each level overwrites it
+            const uint32_t acc = (first && i == 0 && part == 0 && j <= 2) ? 0u : 1u;
+            const uint32_t dl = tmem + (lv < 2 ? set + (uint32_t)(lv * TN) : l2);
+            const uint64_t y = desc_at(sa + BOFF + (((part * kSlices + j) * CF::kBTile * 2) >> 4), BLBO, SBO);
+            const uint32_t id = part ? idesc_neg : idesc;
+            if (j == j0)
+              mma_f16_a_fill(dl, x, y, id, acc);
+            else if (j + 1 < j1)
+              mma_f16_a_use(dl, x, y, id, acc);
+            else
+              mma_f16_a_lastuse(dl, x, y, id, acc);
+          }
+        }
       }
-      fence_after();
-      for (int kt = 0; kt < (int)ktiles; ++kt) {
+    };
+    for (int64_t tile = blockIdx.x; tile < ntot && ok; tile += gridDim.x, ++t) {
+      const int b = (int)(t % kSets);
+      int kt0 = 0;  // K tiles whose MMAs are all issued
+      if constexpr (kPark) {
+        // Level 2 alternates between TMEM blocks 2 and 3, so the first K tiles'
+        // level-2 MMAs (10 of 16) do not wait for the epilogue of the tile
+        // before; their level 0 and 1 MMAs follow once it has read its sums.
+        const uint32_t l2 = (uint32_t)((2 + (t & 1)) * TN);
+        const int pre = (int)ktiles < kStages ? (int)ktiles : kStages;
+        int s1 = s;
+        uint32_t ph1 = ph;
+        for (int kt = 0; kt < pre && ok; ++kt) {
+          if (!__all_sync(0xffffffffu, mbar_wait(&sm.full[s1], ph1))) ok = false;
+          fence_after();
+          if (ok && elect_one()) issue(s1, 2, 2, kt == 0, 0, l2);
+          __syncwarp();
+          next_stage<kStages>(s1, ph1);
+        }
+        if (!ok || !__all_sync(0xffffffffu, mbar_wait(&sm.acce[b], (uint32_t)((t & 1) ^ 1)))) {
+          ok = false;
+          break;
+        }
+        fence_after();
+        for (int kt = 0; kt < pre; ++kt) {
+          if (elect_one()) {
+            issue(s, 0, 1, kt == 0, 0, l2);
+            mma_commit(&sm.empty[s]);  // smem stage free once these MMAs finish
+          }
+          __syncwarp();
+          next_stage<kStages>(s, ph);
+        }
+        kt0 = pre;
+      } else {
+        // the epilogue has read this accumulator set's previous tile
+        if (!__all_sync(0xffffffffu, mbar_wait(&sm.acce[b], (uint32_t)(((t / kSets) & 1) ^ 1)))) {
+          ok = false;
+          break;
+        }
+        fence_after();
+      }
+      for (int kt = kt0; kt < (int)ktiles; ++kt) {
         if (!__all_sync(0xffffffffu, mbar_wait(&sm.full[s], ph))) {
           ok = false;
           break;
         }
         fence_after();
-        // shared-memory descriptors: the address field is in the low word, the
-        // rest is constant
-        const uint32_t sa = smem_u32(sm.stage[s]) >> 4;
-        constexpr uint32_t BOFF = (kSlices * kStackBytes) >> 4;
         if constexpr (CF::narrow) {
+          const uint32_t sa = smem_u32(sm.stage[s]) >> 4;
+          constexpr uint32_t BOFF = (kSlices * kStackBytes) >> 4;
           // B block per part: the slices x 2 row groups per K half
           constexpr uint32_t NLBO = kSlices * 2 * 128;
           if (elect_one()) {
@@ -659,37 +756,14 @@ __global__ void __launch_bounds__(kThreads, 1)
           next_stage<kStages>(s, ph);
           continue;
         }
-        // The MMAs of one A operand follow each other: the first fills the
-        // tensor core's A buffer from shared memory, the others use it (an
-        // M = N = 128 MMA reads 8 KB in its 64 cycles, all of the SM's
-        // shared-memory bandwidth; with A kept, kHalf reads 88 KB per K tile
-        // instead of 128 KB: 7 % of the wide pair's time).
         if (elect_one()) {
-#pragma unroll
-          for (int i = 0; i < kSlices; ++i) {
-#pragma unroll
-            for (int part = 0; part < 2; ++part) {
-              // part 0: [Ar; Ai] . Br = [Ar.Br ; Ai.Br]; part 1: [Ai; -Ar]
-              // with A negated . Bi = [-Ai.Bi ; Ar.Bi]
-              const uint64_t x = desc_at(sa + ((i * kStackBytes + part * 8 * 128) >> 4), ALBO, SBO);
-#pragma unroll
-              for (int j = 0; j < Sl<S>::met(i); ++j) {
-                // the first MMA into each level overwrites it
-                const uint32_t acc = (kt == 0 && i == 0 && part == 0 && j <= 2) ? 0u : 1u;
-                const uint32_t dl = tmem + (uint32_t)((b * 3 + (i + j < 2 ? i + j : 2)) * TN);
-                const uint64_t y = desc_at(sa + BOFF + (((part * kSlices + j) * CF::kBTile * 2) >> 4), BLBO, SBO);
-                const uint32_t id = part ? idesc_neg : idesc;
-                if (j == 0)
-                  mma_f16_a_fill(dl, x, y, id, acc);
-                else if (j + 1 < Sl<S>::met(i))
-                  mma_f16_a_use(dl, x, y, id, acc);
-                else
-                  mma_f16_a_lastuse(dl, x, y, id, acc);
-              }
-            }
-          }
+          if constexpr (kPark)
+            issue(s, 0, 2, false, 0, (uint32_t)((2 + (t & 1)) * TN));
+          else
+            issue(s, 0, 2, kt == 0, (uint32_t)(b * 3 * TN), (uint32_t)((b * 3 + 2) * TN));
           mma_commit(&sm.empty[s]);  // smem stage free once these MMAs finish
         }
+        __syncwarp();
         next_stage<kStages>(s, ph);
       }
       if (!ok) break;
@@ -855,9 +929,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     // One accumulator set and complex64 results: the combined levels are
     // parked in the unused fourth TMEM block so that the accumulators are
     // released before the scaling and the scattered stores.
-    constexpr bool kStash = kSets == 1 && std::is_same<TC, float2>::value && 4 * TN <= (int)kTmemCols &&
+    constexpr bool kStash = !kPark && kSets == 1 && std::is_same<TC, float2>::value && 4 * TN <= (int)kTmemCols &&
                             CW % 16 == 0;
-    constexpr int NU = (CW + 31) / 32;       // columns of the warp's range per lane
+    // Where a thread's stores lie: its TMEM row and columns, or with parked
+    // sums row half e & 1 and 32 columns from (e >> 1) 32 for epilogue warp e,
+    // real and imaginary part together.
+    const int e = warp - 2 - kConvWarps;
+    constexpr int SW = kPark ? 32 : CW;
+    const int srow = kPark ? (e & 1) * 32 + lane : r, scol = kPark ? (e >> 1) * 32 : h * CW;
+    constexpr int NU = (SW + 31) / 32;       // columns of the warp's range per lane
     // per-tile offsets and scales, loaded one tile ahead: the row's from
     // this lane, the warp's columns spread over the lanes
     struct Meta {
@@ -869,15 +949,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     };
     auto meta = [&](int64_t tile, Meta& M) {
       const int64_t nt = tile % ntiles, rr = tile / ntiles, mt = rr % mtiles, z = rr / mtiles;
-      const int64_t m = mt * kRows + r;
+      const int64_t m = mt * kRows + srow;
       M.mrow = m < d.M;
       M.base = M.mrow ? decode(z, d.nz, d.zdim, d.zsc) + cm_tab[m] : 0;
       M.exa = M.mrow ? ea[z * d.M + m] : kExpZero;
-      M.c0 = nt * TN + h * CW;
+      M.c0 = nt * TN + scol;
 #pragma unroll
       for (int u = 0; u < NU; ++u) {
         const int64_t col = M.c0 + lane + 32 * u;
-        const bool valid = lane + 32 * u < CW && col < d.N;
+        const bool valid = lane + 32 * u < SW && col < d.N;
         M.ebl[u] = valid ? eb[z * d.N + col] : kExpZero;
         M.cnl[u] = valid ? (long long)cn_tab[col] : 0;
       }
@@ -895,11 +975,53 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int b = (int)(t % kSets);
       bool got = mbar_wait(&sm.accf[b], (uint32_t)((t / kSets) & 1));
       got = __all_sync(0xffffffffu, got);  // the TMEM loads below are warp-collective
+      // (with parked sums, of all epilogue warps: they meet in the barriers
+      // below, and here the last tile's parked sums have been read)
+      if constexpr (kPark) got = epilogue_all(got);
       if (!got) {
         ok = false;
         break;
       }
       fence_after();
+      if constexpr (kPark) {
+        // Phase 1 (holds levels 0 and 1): the three levels of each element
+        // summed into one float in shared memory; then the accumulators are
+        // released.
+        float* P = sm.park + (part * kRows + r) * kParkPitch + h * CW;
+        const uint32_t l2 = (uint32_t)((2 + (t & 1)) * TN);
+#pragma unroll
+        for (int piece = 0; piece < CW / 16; ++piece) {
+          __syncwarp();
+          const uint32_t col = lane_base + (uint32_t)(h * CW + piece * 16);
+          float l0[16], l1[16], lr[16];
+          tmem_ld16(col, l0);
+          tmem_ld16(col + TN, l1);
+          tmem_ld16(col + l2, lr);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) P[piece * 16 + j] = level_sum(l0[j], l1[j], lr[j]);
+        }
+        fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.acce[b]);
+        epilogue_all(true);  // the sums of both parts are parked
+        // Phase 2 (overlaps the next tile's MMAs): scale by 2^(ea + eb), store
+        // whole complex values through the result index map.
+        const float* Re = sm.park + srow * kParkPitch + scol;
+        const float* Im = Re + kRows * kParkPitch;
+        float2* Cc = reinterpret_cast<float2*>(C);
+#pragma unroll 8
+        for (int cc = 0; cc < SW; ++cc) {
+          const int ebj = __shfl_sync(0xffffffffu, M.ebl[0], cc);
+          const long long cnj = __shfl_sync(0xffffffffu, M.cnl[0], cc);
+          if (mrow && c0 + cc < d.N) {
+            const int ex = exa + ebj - kDown;
+            const bool zero = exa == kExpZero || ex < -2 * 1100;
+            Cc[base + cnj] = zero ? make_float2(0.f, 0.f) : make_float2(scale_pow2(Re[cc], ex), scale_pow2(Im[cc], ex));
+          }
+        }
+        continue;
+      }
       if constexpr (kStash) {
         // Phase 1 (holds the accumulators): the three levels of each element
         // summed into one float, parked in the spare TMEM block (columns
@@ -1114,8 +1236,9 @@ template <typename TA, typename TC, int TN, int S>
 cudaError_t oz_gemm_launch(const void* A, const uint16_t* pb, void* C, const GemmDesc& d, const int64_t* cm,
                            const int64_t* cn, const int* ea, const int* eb, const OzLayout& L, int* status,
                            cudaStream_t s) {
-  static_assert(sizeof(OzSmem<TN, S>) + 1024 <= 232448, "shared memory layout exceeds 227 KiB");
-  const size_t smem = sizeof(OzSmem<TN, S>) + 1024;
+  constexpr bool park = oz_park<TC, TN, S>();
+  static_assert(sizeof(OzSmem<TN, S, park>) + 1024 <= 232448, "shared memory layout exceeds 227 KiB");
+  const size_t smem = sizeof(OzSmem<TN, S, park>) + 1024;
   static bool attr = false;
   if (!attr) {
     cudaError_t e =

@@ -503,3 +503,30 @@ def test_ozaki_half_split(pq, O, order, k, n):
             assert np.all(np.abs(got - ref) <= ozaki_bound(A, B, ref))
         else:
             assert np.max(np.abs(got - ref)) <= 2.0 ** -23 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("k", [16, 24, 48, 64, 136])
+@pytest.mark.parametrize("order", ["mk", "km"])
+def test_ozaki_wide_many_tiles_per_cta(pq, order, k):
+    """128-wide tiles, three or four per persistent CTA with a ragged last one,
+    from one K tile (fewer than the ring's three stages) to nine: the sums of a
+    tile parked while the next tile's level-2 MMAs run in the other TMEM
+    block.  Complex64, an all-zero row, columns past N (N = 200: a full and a
+    ragged column tile)."""
+    rng = np.random.default_rng(k)
+    m, n = 64 * 152 + 64 * 70 + 37, 200
+    A = rand(rng, (m, k)).astype(np.complex64)
+    A[1000] = 0
+    B = rand(rng, (k, n)).astype(np.complex64)
+    be = ozaki_backend(pq)
+    if order == "km":
+        got, nl = run(be, A.T, [1, -1], B, [1, -2])
+    else:
+        got, nl = run(be, A, [-1, 1], B, [1, -2])
+    be.close()
+    assert nl == OZ_LAUNCHES
+    A, B = A.astype(np.complex128), B.astype(np.complex128)
+    ref = A @ B
+    assert np.all(got[1000] == 0)
+    assert np.all(np.abs(got - ref) <= ozaki_bound(A, B, ref))
+    _restatement_match(got, A, B)

@@ -73,7 +73,7 @@
 //                  issue one MMA per A slice i against the B slices it meets
 //                  side by side, each slice pair into its own 16-column
 //                  region;
-//     warps 2-9    A converters: gather A's 64 x 16 complex values of the K
+//     8 or 12 warps A converters: gather A's 64 x 16 complex values of the K
 //                  tile through its index map straight from HBM (the group's
 //                  next K tile in flight while this one is sliced), slice
 //                  them and store the [Ar; Ai; -Ar] stacks into the ring (no
@@ -81,7 +81,7 @@
 //                  groups of four warps take alternate K tiles, each thread
 //                  8 consecutive k of one row, so every store is a whole
 //                  16-byte core-matrix row;
-//     warps 10-17  epilogue, once per tile: Cr from TMEM lanes 0-63, Ci from
+//     8 or 4 warps  epilogue, once per tile: Cr from TMEM lanes 0-63, Ci from
 //                  lanes 64-127; the levels are combined with an error-free
 //                  two-sum (128-wide complex64 tiles park the sums, in shared
 //                  memory or the spare TMEM block, and release the
@@ -106,8 +106,8 @@ namespace {
 using namespace tcg;
 
 constexpr int TK = 16;
-constexpr int kThreads = 576;                    // producer, MMA, 8 converter + 8 epilogue warps
-constexpr int kConvWarps = 8, kEpiWarps = 8;
+constexpr int kThreads = 576;                    // producer, MMA, 16 converter and epilogue warps
+constexpr int kWorkWarps = 16;                   // converter + epilogue warps
 constexpr int kRows = 64;                        // complex rows of A per tile
 constexpr int kStackBytes = 3 * kRows * TK * 2;  // one slice's [Ar; Ai; -Ar] stack (6 KiB)
 constexpr int kExpZero = -4096;                  // exponent of an all-zero row
@@ -130,6 +130,14 @@ struct Sl {
   // slices 0 .. met(i) - 1 of B meet slice i of A
   __host__ __device__ static constexpr int met(int i) { return half ? (i < 2 ? 3 : 2) : n - i; }
 };
+// Converter warps (the rest are epilogue warps): 12 for 16- and 32-wide tiles of
+// complex64 A in three slices, whose few MMAs wait for A's loads -- a third
+// group of converters keeps half as much again in flight (2^20 x 16 x 256: 0.9 ->
+// 0.7 ms; a second K tile per thread spilled) -- else 8.
+template <typename TA, int TN, int S>
+__host__ __device__ constexpr int conv_warps() {
+  return TN <= 32 && Sl<S>::half && sizeof(TA) == 8 ? 12 : 8;
+}
 // kHalf: scaled values are held times 2^kHalfUp, so that the lowest bits of
 // the third slice stay in fp16's range.
 constexpr int kHalfUp = 15;
@@ -167,8 +175,7 @@ struct OzCfg {
   static constexpr int acc_sets = TN <= 64 ? 2 : 1;
   static constexpr uint32_t tmem_cols =
       TN == 128 ? 512 : (TN == 64 ? 512 : (TN == 32 ? 256 : (2 * set_cols > 256 ? 512 : 256)));
-  static constexpr int cw = TN / 2;                                         // columns per epilogue warp
-  static_assert(acc_sets * set_cols <= (int)tmem_cols && cw % 8 == 0 && stage_bytes % 1024 == 0, "tile width");
+  static_assert(acc_sets * set_cols <= (int)tmem_cols && stage_bytes % 1024 == 0, "tile width");
 };
 
 // First TMEM column of A slice i's region in a narrow tile.
@@ -549,7 +556,6 @@ __device__ __forceinline__ void ldg256(const void* p, float* v) {
 
 // A values per converter thread and K tile: 8 for complex64 A (whole 16-byte
 // core-matrix rows), 4 for complex128 A.
-constexpr int kConvThreads = 32 * kConvWarps;
 template <typename TA>
 __host__ __device__ constexpr int conv_values() {
   return sizeof(TA) == 8 ? 8 : 4;
@@ -558,13 +564,13 @@ __host__ __device__ constexpr int conv_values() {
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // True when `v` holds in every thread of the epilogue warps, all of which call
-// it (named barrier 1; shared-memory accesses before it are seen after it).
+// it (named barrier 1, 8 warps; shared-memory accesses before it are seen after it).
 __device__ __forceinline__ bool epilogue_all(bool v) {
   uint32_t r;
   asm volatile(
       "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n barrier.cta.red.and.pred p, 1, %2, q;\n selp.u32 %0, 1, 0, p;\n}\n"
       : "=r"(r)
-      : "r"((uint32_t)v), "n"(32 * kEpiWarps)
+      : "r"((uint32_t)v), "n"(32 * 8)
       : "memory");
   return r != 0;
 }
@@ -591,6 +597,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   constexpr int kStages = CF::stages;
   constexpr uint32_t kTmemCols = CF::tmem_cols;
   constexpr int kSets = CF::acc_sets;
+  constexpr int kConvWarps = conv_warps<TA, TN, S>(), kEpiWarps = kWorkWarps - kConvWarps;
+  constexpr int kGroupThreads = kRows * TK / conv_values<TA>();  // converters of one K tile
+  static_assert(!kPark || kEpiWarps == 8, "epilogue_all counts 8 warps");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   OzSmem<TN, S, kPark>& sm = *reinterpret_cast<OzSmem<TN, S, kPark>*>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -599,7 +608,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       // producer's expect_tx + one arrival per warp of the converter group of the K tile
-      mbar_init(&sm.full[s], 1 + kConvWarps * 4 / conv_values<TA>());
+      mbar_init(&sm.full[s], 1 + kGroupThreads / 32);
       mbar_init(&sm.empty[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -774,12 +783,13 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (!mbar_wait(&sm.drain, 0)) ok = false;
   } else if (warp < 2 + kConvWarps) {
     // converters: with NV values per thread and K tile, the converter warps
-    // form NV / 4 groups that take alternate K tiles; thread ch of a group
+    // form groups of 64 16 / NV threads that take K tiles in turn; thread ch of a group
     // handles row r = ch % 64 and the NV consecutive K values from
     // kq = (ch / 64) NV of its K tiles.  Complex64 A: NV = 8, a whole 16-byte
     // core-matrix row per stack block, stored without bank conflicts;
     // complex128 A: NV = 4 (half rows; fewer registers), one group.
-    constexpr int NV = conv_values<TA>(), H = NV / 4, GT = kConvThreads / H;
+    constexpr int NV = conv_values<TA>(), GT = kGroupThreads, H = 32 * kConvWarps / GT;
+    static_assert(H <= kStages, "ring");
     const int c = threadIdx.x - 64;
     const int grp = c / GT, ch = c % GT;
     const int r = ch & (kRows - 1), kq = (ch >> 6) * NV;
@@ -852,7 +862,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       row_info(ptl);
       load(pkt, nxt);
     }
-    int s = grp;  // H <= 2 <= kStages
+    int s = grp;
     uint32_t ph = 0;
     for (int64_t gk = grp; gk < items && ok; gk += H) {
       const int e = en;
@@ -918,14 +928,14 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else {
     // epilogue: warp w reads TMEM lanes of quadrant w % 4 (0, 1: Cr of rows
     // 0..63; 2, 3: Ci), columns [h TN/2, (h+1) TN/2)
-    constexpr int CW = CF::cw;
+    constexpr int CW = TN / (kEpiWarps / 4);
     const int q = warp & 3, h = (warp - 2 - kConvWarps) >> 2;
     const int part = q >> 1;               // 0: real parts, 1: imaginary parts
     const int r = (q & 1) * 32 + lane;     // complex row within the tile
     const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
     using R = typename std::conditional<std::is_same<TC, double2>::value, double, float>::type;
     R* Cr = reinterpret_cast<R*>(C);
-    constexpr int PW = CW >= 16 ? 16 : 8;   // columns per TMEM load
+    constexpr int PW = CW >= 16 && !CF::narrow ? 16 : 8;   // columns per TMEM load
     // One accumulator set and complex64 results: the combined levels are
     // parked in the unused fourth TMEM block so that the accumulators are
     // released before the scaling and the scattered stores.

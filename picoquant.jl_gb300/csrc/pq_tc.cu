@@ -12,23 +12,35 @@
 //     NS = 3 (PQ_PREC_6XTF32): x0y0 + x0y1 + x1y0 + x0y2 + x2y0 + x1y1  (6)
 //
 // k_tc_pack gathers an operand through its index map (any mode order, batch
-// modes) into 2*NS planes {re terms, im terms} laid out tile by tile; a tile is
-// ROWS (128 for A, 48 for B) x 16 K values in the canonical no-swizzle
-// K-major UMMA layout: 8-row x 16-byte core matrices (128 contiguous bytes),
-// row-adjacent core matrices 128 bytes apart, K-adjacent ones ROWS*16 bytes
-// apart.  One bulk copy moves one plane tile.  Rows and K beyond the operand
-// are zero.
+// modes) into the terms of its real and imaginary parts, laid out tile by tile;
+// a tile is ROWS (128 for A, 64 for B) x 16 K values in the canonical
+// no-swizzle K-major UMMA layout: 8-row x 16-byte core matrices (128 contiguous
+// bytes), row-adjacent core matrices 128 bytes apart.  A has one plane per part
+// and term; B one plane per term, of 128 rows: the 64 of the real part, then the
+// 64 of the imaginary part, so that Ar.[Br Bi] is one MMA.  Rows and K beyond
+// the operand are zero.
 //
-// k_tc_gemm: one CTA per 128 x 48 output tile (x batch), 14 warps.
-//   warp 0   producer: cp.async.bulk of the 4*NS plane tiles of one 16-deep K
-//            tile into a shared-memory ring (mbarrier complete_tx);
-//   warp 1   allocates TMEM and issues tcgen05.mma (M=128, N=48, K=8); every
-//            16-deep K tile is one chunk, rotating over four sets of two
-//            48-column FP32 accumulators, committed to the epilogue per chunk;
-//   warps 2-13 epilogue: warp w reads TMEM lanes 32*(w%4).. and 16 of the 48
-//            columns, folds each chunk's (Cr, Ci) into Kahan sums, hands the
-//            accumulator set back, and finally scatters C through the result
-//            index map.
+// k_tc_gemm: one CTA per 128 x 64 output tile (x batch), 18 warps.
+//   warp 0   producer: two cp.async.bulk per 16-deep K tile (the A and the B
+//            planes, each contiguous) into a shared-memory ring (mbarrier
+//            complete_tx);
+//   warp 1   allocates TMEM and issues tcgen05.mma (M=128, K=8); every 16-deep
+//            K tile is one chunk, rotating over four sets of two 64-column FP32
+//            accumulators (all 512 TMEM columns), committed to the epilogue per
+//            chunk;
+//   warps 2-17 epilogue: warp w reads TMEM lanes 32*(w%4).. and 16 of the 64
+//            columns, folds each chunk's (Cr, Ci) into Kahan sums (two columns
+//            per f32x2 instruction), hands the accumulator set back, and finally
+//            scatters C through the result index map.
+// What bounds it: the MMAs (about 1500 SM cycles per K tile with two terms) and
+// the epilogue (1400) are close to each other, the bulk copies need 900 (each
+// measured with the others' work left out; 1600 together).  With both packs, the
+// index table and the launches, 8192 x 512 x 1024 (M x N x K) takes 235 us (300
+// with N = 64 MMAs and scalar sums) and 32768 x 128 x 128 takes 60 us; 128 x 48
+// tiles, which read A three times for N = 128 and pad it to 144, and packs of
+// one value per thread took 52 us for its GEMM and 27 (now 17) for A's pack alone.
+// The four launches of a pair are programmatic dependents of each other, so that
+// index decodes and barrier set-up run while the launch before them drains.
 // The tensor core rounds accumulations toward zero.  The small correction
 // products of a chunk go in first, the hi x hi products last, so each chunk
 // takes its few truncations at (partial) full magnitude; chunks are summed
@@ -51,11 +63,11 @@ namespace {
 
 using namespace tcg;
 
-constexpr int TM = 128, TN = 48, TK = 16;
-constexpr int kThreads = 448;                  // producer, MMA, 12 epilogue warps
-constexpr int kEpiWarps = 12;
+constexpr int TM = 128, TN = 64, TK = 16;
+constexpr int kThreads = 576;                  // producer, MMA, 16 epilogue warps
+constexpr int kEpiWarps = 16;
 constexpr int kSets = 4;                       // TMEM accumulator sets in rotation
-constexpr uint32_t kTmemCols = 512;            // 4 sets x 2 accumulators x 48 columns = 384 used
+constexpr uint32_t kTmemCols = 512;            // 4 sets x 2 accumulators x 64 columns
 // Expected relative shrinkage of a value truncated (rounded toward zero) to
 // FP32: half an ulp over a log-uniform mantissa, 2^-24 * ln 2 ...
 constexpr float kTruncUnit = 4.13145e-8f;
@@ -66,13 +78,13 @@ constexpr float kTruncUnit = 4.13145e-8f;
 // partial sums' mantissas are not log-uniform).
 constexpr float kTruncBias = 2.2f * kTruncUnit;
 constexpr int kATile = TM * TK;                // floats per A plane tile (8 KiB)
-constexpr int kBTile = TN * TK;                // floats per B plane tile (3 KiB)
+constexpr int kBTile = TN * TK;                // floats per B plane tile (4 KiB)
 
 template <int NS>
 struct Cfg {
   static constexpr int planes = 2 * NS;                                  // per operand
   static constexpr uint32_t stage_bytes = planes * (kATile + kBTile) * 4;
-  static constexpr int stages = NS == 2 ? 5 : 3;
+  static constexpr int stages = NS == 2 ? 4 : 3;
   static constexpr int products = NS == 2 ? 3 : 6;
 };
 
@@ -98,49 +110,111 @@ __device__ __forceinline__ void split(double x, float* t) {
 }
 
 // Pack operand X (side 0: A with m modes, side 1: B with n modes) into planes
-// laid out [z][row tile][k tile][plane][ROWS*16 floats].
+// laid out [z][row tile][k tile][plane][ROWS*16 floats].  A block packs `kper`
+// K tiles of one row tile, a thread four K values of one row at a time: one
+// 32-byte load where they are adjacent and aligned (four 8-byte ones where
+// not), one 16-byte store per plane.  The rows' offsets (a mixed-radix decode)
+// are found once per block, and before the kernel waits for the operand.
+constexpr int kPackMaxK = 8;  // K tiles per block at most
 template <typename T, int NS, int ROWS>
-__global__ void __launch_bounds__(256) k_tc_pack(const T* __restrict__ X, float* __restrict__ planes,
-                                                 const __grid_constant__ GemmDesc d, int side, int64_t rows,
-                                                 int64_t rtiles, int64_t ktiles) {
-  constexpr int TILE = ROWS * TK, GROUPS = ROWS / 8;
+__global__ void __launch_bounds__(256) k_tc_pack(const T* X, float* planes, const __grid_constant__ GemmDesc d,
+                                                 int side, int64_t rows, int64_t rtiles, int64_t ktiles, int kper) {
+  constexpr int TILE = ROWS * TK, QUADS = TILE / 4;
   __shared__ int64_t roff[ROWS];
-  __shared__ int64_t koff[TK];
-  const int64_t kt = blockIdx.x, rt = blockIdx.y, z = blockIdx.z;
+  __shared__ int64_t koff[kPackMaxK * TK];
+  const int64_t kt0 = blockIdx.x * (int64_t)kper, rt = blockIdx.y, z = blockIdx.z;
+  const int nkt = (int)(ktiles - kt0 < kper ? ktiles - kt0 : kper);
   const int nrm = side == 0 ? d.nm : d.nn;
   const int64_t* rdim = side == 0 ? d.mdim : d.ndim;
   const int64_t* rstr = side == 0 ? d.msa : d.nsb;
   const int64_t* kstr = side == 0 ? d.ksa : d.ksb;
   const int64_t* zstr = side == 0 ? d.zsa : d.zsb;
-  for (int t = threadIdx.x; t < ROWS + TK; t += blockDim.x) {
+  for (int t = threadIdx.x; t < ROWS + nkt * TK; t += blockDim.x) {
     if (t < ROWS) {
       int64_t r = rt * ROWS + t;
       roff[t] = r < rows ? decode(r, nrm, rdim, rstr) : -1;
     } else {
-      int64_t k = kt * TK + (t - ROWS);
+      int64_t k = kt0 * TK + (t - ROWS);
       koff[t - ROWS] = k < d.K ? decode(k, d.nk, d.kdim, kstr) : -1;
     }
   }
+  const T* Xz = X + decode(z, d.nz, d.zdim, zstr);
+  pdl_trigger();
+  pdl_wait();
   __syncthreads();
-  const int64_t zo = decode(z, d.nz, d.zdim, zstr);
-  float* tile = planes + (((z * rtiles + rt) * ktiles + kt) * (2 * NS)) * (int64_t)TILE;
-  for (int o = threadIdx.x; o < TILE; o += blockDim.x) {
-    // o = ((kc * GROUPS + g) * 32) + r8 * 4 + k4
-    const int core = o >> 5, within = o & 31;
-    const int kc = core / GROUPS, g = core - kc * GROUPS;
-    const int r = g * 8 + (within >> 2), k = kc * 4 + (within & 3);
-    float re[3] = {0.f, 0.f, 0.f}, im[3] = {0.f, 0.f, 0.f};
-    if (roff[r] >= 0 && koff[k] >= 0) {
-      T v = X[zo + roff[r] + koff[k]];
-      split<NS>(v.x, re);
-      split<NS>(v.y, im);
+  float* tiles = planes + (((z * rtiles + rt) * ktiles + kt0) * (2 * NS)) * (int64_t)TILE;
+#pragma unroll 2
+  for (int o = threadIdx.x; o < nkt * QUADS; o += blockDim.x) {
+    // quad w of tile t: core matrix (kc, row group) row by row = kc * ROWS + row
+    const int t = o / QUADS, w = o - t * QUADS, kc = w / ROWS, r = w - kc * ROWS;
+    const int64_t* ko = koff + t * TK + kc * 4;
+    const int64_t ro = roff[r], k0 = ko[0], k1 = ko[1], k2 = ko[2], k3 = ko[3];
+    T v[4] = {};
+    if (ro >= 0) {
+      const T* x = Xz + ro;
+      bool wide = false;
+      if constexpr (sizeof(T) == 8)
+        wide = k0 >= 0 && k1 == k0 + 1 && k2 == k0 + 2 && k3 == k0 + 3 && ((uintptr_t)(x + k0) & 31) == 0;
+      if (wide) {
+        if constexpr (sizeof(T) == 8)
+          asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                       : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[2].x), "=f"(v[2].y),
+                         "=f"(v[3].x), "=f"(v[3].y)
+                       : "l"(x + k0));
+      } else {
+        if (k0 >= 0) v[0] = x[k0];
+        if (k1 >= 0) v[1] = x[k1];
+        if (k2 >= 0) v[2] = x[k2];
+        if (k3 >= 0) v[3] = x[k3];
+      }
     }
+    float re[4][3], im[4][3];
 #pragma unroll
-    for (int t = 0; t < NS; ++t) {
-      tile[(0 * NS + t) * TILE + o] = re[t];
-      tile[(1 * NS + t) * TILE + o] = im[t];
+    for (int i = 0; i < 4; ++i) {
+      split<NS>(v[i].x, re[i]);
+      split<NS>(v[i].y, im[i]);
+    }
+    // A: a plane per part and term; B: the two parts of a term are one plane of
+    // 2*ROWS rows
+    constexpr bool kB = ROWS == TN;
+    float* tile = tiles + (int64_t)t * (2 * NS * TILE) + (kB ? kc * (8 * ROWS) + r * 4 : w * 4);
+#pragma unroll
+    for (int p = 0; p < NS; ++p) {
+      *(float4*)(tile + (kB ? 2 * p * TILE : p * TILE)) = make_float4(re[0][p], re[1][p], re[2][p], re[3][p]);
+      *(float4*)(tile + (kB ? 2 * p * TILE + 4 * ROWS : (NS + p) * TILE)) =
+          make_float4(im[0][p], im[1][p], im[2][p], im[3][p]);
     }
   }
+}
+
+// Kahan-compensated sums of two values at a time (sum and compensation as FP32
+// pairs; the steps of kahan_add1 on both halves, one instruction each).
+struct Kahan2 {
+  F2 s, c;
+};
+__device__ __forceinline__ F2 f2_pack(float x, float y) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {
+  F2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ void kahan2_add(Kahan2& k, F2 x) {
+  const F2 y = f2_sub(x, k.c), t = f2_add(k.s, y);
+  k.c = f2_sub(f2_sub(t, k.s), y);
+  k.s = t;
+}
+__device__ __forceinline__ float2 kahan2_value(const Kahan2& k) {
+  const float2 s = f2_get(k.s), c = f2_get(k.c);
+  return make_float2(s.x - c.x, s.y - c.y);
 }
 
 template <int NS>
@@ -160,9 +234,8 @@ struct alignas(1024) TcSmem {
 // the epilogue of one tile overlaps the MMAs of the next.
 template <typename TC, int NS>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_tc_gemm(const float* __restrict__ pa, const float* __restrict__ pb, TC* __restrict__ C,
-              const __grid_constant__ GemmDesc d, const int64_t* __restrict__ cm_tab,
-              const int64_t* __restrict__ cn_tab, int64_t mtiles, int64_t ntiles, int64_t ktiles, int* status) {
+    k_tc_gemm(const float* pa, const float* pb, TC* C, const __grid_constant__ GemmDesc d, const int64_t* cm_tab,
+              const int64_t* cn_tab, int64_t mtiles, int64_t ntiles, int64_t ktiles, int* status) {
   using CF = Cfg<NS>;
   constexpr int S = CF::stages, P = CF::planes;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -190,6 +263,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   fence_after();
   const uint32_t tmem = sm.tmem_base;
   bool ok = true;
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -206,14 +280,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             break;
           }
           mbar_expect_tx(&sm.full[s], CF::stage_bytes);
-          const float* a = atile + kt * (P * kATile);
-          const float* b = btile + kt * (P * kBTile);
           float* dst = sm.stage[s];
-#pragma unroll
-          for (int p = 0; p < P; ++p) {
-            bulk_g2s(dst + p * kATile, a + p * kATile, kATile * 4, &sm.full[s]);
-            bulk_g2s(dst + P * kATile + p * kBTile, b + p * kBTile, kBTile * 4, &sm.full[s]);
-          }
+          bulk_g2s(dst, atile + kt * (P * kATile), P * kATile * 4, &sm.full[s]);
+          bulk_g2s(dst + P * kATile, btile + kt * (P * kBTile), P * kBTile * 4, &sm.full[s]);
         }
       }
       // the copies of the last stages are in flight until their full barrier
@@ -223,11 +292,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 1) {
     // The whole warp runs the loop and waits, one elected thread issues a K
-    // tile's MMAs and commits, so that descriptors stay uniform.  An N = 48 MMA
-    // takes 24 cycles of the tensor core and reads 5.5 KB of operands (43 cycles
-    // of shared memory).
-    constexpr uint32_t idesc = idesc_tf32(TM, TN), idesc_neg = idesc_tf32(TM, TN, true);
-    constexpr uint32_t ALBO = (TM / 8) * 128, BLBO = (TN / 8) * 128, SBO = 128;
+    // tile's MMAs and commits, so that descriptors stay uniform.  Ar.[Br Bi] goes
+    // as one N = 128 MMA: 1500 cycles per K tile with two terms, 1650 as N = 64.
+    constexpr uint32_t idesc2 = idesc_tf32(TM, 2 * TN), idesc = idesc_tf32(TM, TN),
+                       idesc_neg = idesc_tf32(TM, TN, true);
+    constexpr uint32_t ALBO = (TM / 8) * 128, BLBO = (2 * TN / 8) * 128, SBO = 128;
     int s = 0, b = 0;  // ring stage and accumulator set, with their phases
     uint32_t ph = 0, use = 0;
     for (int64_t tile = blockIdx.x; tile < ntot && ok; tile += gridDim.x) {
@@ -256,10 +325,9 @@ __global__ void __launch_bounds__(kThreads, 1)
               const uint32_t oa = (uint32_t)j * 2 * ALBO, ob = (uint32_t)j * 2 * BLBO;
               const uint64_t ar = desc_at(sa + (((0 * NS + ti) * kATile * 4 + oa) >> 4), ALBO, SBO);
               const uint64_t ai = desc_at(sa + (((1 * NS + ti) * kATile * 4 + oa) >> 4), ALBO, SBO);
-              const uint64_t br = desc_at(sb + (((0 * NS + tj) * kBTile * 4 + ob) >> 4), BLBO, SBO);
-              const uint64_t bi = desc_at(sb + (((1 * NS + tj) * kBTile * 4 + ob) >> 4), BLBO, SBO);
-              mma_tf32(dr, ar, br, idesc, acc);     // + Ar.Br
-              mma_tf32(di, ar, bi, idesc, acc);     // + Ar.Bi
+              const uint64_t br = desc_at(sb + ((tj * 2 * kBTile * 4 + ob) >> 4), BLBO, SBO);
+              const uint64_t bi = desc_at(sb + ((tj * 2 * kBTile * 4 + ob + TN * 16) >> 4), BLBO, SBO);
+              mma_tf32(dr, ar, br, idesc2, acc);    // + Ar.[Br Bi]
               mma_tf32(dr, ai, bi, idesc_neg, 1u);  // - Ai.Bi
               mma_tf32(di, ai, br, idesc, 1u);      // + Ai.Br
             }
@@ -283,51 +351,86 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else {
     // epilogue: warp w reads TMEM lanes of quadrant w % 4, columns [16h, 16h+16)
     constexpr int CW = TN / (kEpiWarps / 4);  // columns per epilogue warp
-    static_assert(CW == 16, "one 16-column load per accumulator");
     const int q = warp & 3, h = (warp - 2) >> 2;
     const int row = q * 32 + lane;
     const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
-    int64_t g = 0;
+    int b = 0;
+    uint32_t use = 0;
     for (int64_t tile = blockIdx.x; tile < ntot && ok; tile += gridDim.x) {
       const int64_t nt = tile % ntiles, r = tile / ntiles, mt = r % mtiles, z = r / mtiles;
-      KahanC acc[CW];
+      const int64_t m = mt * TM + row, n0 = nt * TN + h * CW;
+      const int ncol = (int)(d.N - n0 < CW ? d.N - n0 : CW);  // columns of this warp inside C (may be <= 0)
+      // result offsets, loaded ahead of the sums: this lane's row (-1: outside C)
+      // and the column n0 + lane
+      const int64_t base = m < d.M ? decode(z, d.nz, d.zdim, d.zsc) + cm_tab[m] : -1;
+      const int64_t coff = lane < ncol ? cn_tab[n0 + lane] : 0;
+      Kahan2 ar[CW / 2], ai[CW / 2];  // sums of the real and imaginary parts, two columns each
 #pragma unroll
-      for (int j = 0; j < CW; ++j) kahan_init(acc[j]);
-      for (int64_t kt = 0; kt < ktiles; ++kt, ++g) {
-        const int b = (int)(g % kSets);
-        const uint32_t use = (uint32_t)((g / kSets) & 1);
-        bool got = mbar_wait(&sm.accf[b], use);
-        got = __all_sync(0xffffffffu, got);  // the TMEM loads below are warp-collective
-        if (!got) {
+      for (int j = 0; j < CW / 2; ++j) ar[j] = ai[j] = Kahan2{0, 0};
+      for (int kt = (int)ktiles; kt > 0; --kt) {
+        // the TMEM loads below are warp-collective
+        if (!__all_sync(0xffffffffu, mbar_wait(&sm.accf[b], use))) {
           ok = false;
           break;
         }
         fence_after();
         const uint32_t col = (uint32_t)(b * 2 * TN + h * CW);
-        float vr[16], vi[16];
-        tmem_ld16(lane_base + col, vr);
-        tmem_ld16(lane_base + col + TN, vi);
-        tmem_wait_ld();
-        fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.acce[b]);  // values are in registers: hand the set back
+        // eight columns at a time: 64 registers of sums and 16 of values fit the
+        // 112 that 18 warps leave a thread
 #pragma unroll
-        for (int j = 0; j < CW; ++j) kahan_add(acc[j], make_float2(vr[j], vi[j]));
+        for (int c = 0; c < CW; c += 8) {
+          float vr[8], vi[8];
+          tmem_ld8(lane_base + col + c, vr);
+          tmem_ld8(lane_base + col + c + TN, vi);
+          tmem_wait_ld();
+          if (c + 8 == CW) {  // values are in registers: hand the set back
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.acce[b]);
+          }
+#pragma unroll
+          for (int j = 0; j < 8; j += 2) {
+            kahan2_add(ar[(c + j) / 2], f2_pack(vr[j], vr[j + 1]));
+            kahan2_add(ai[(c + j) / 2], f2_pack(vi[j], vi[j + 1]));
+          }
+        }
+        if (++b == kSets) {
+          b = 0;
+          use ^= 1u;
+        }
       }
       if (!ok) break;
-      const int64_t m = mt * TM + row;
-      if (m < d.M) {
-        const int64_t base = decode(z, d.nz, d.zdim, d.zsc) + cm_tab[m];
-        const int64_t n0 = nt * TN + h * CW;
+      // lane j holds the result offset of column n0 + j: adjacent columns leave as
+      // 32-byte stores where they are adjacent (and aligned) in C too
+      const int64_t cn_prev = __shfl_up_sync(0xffffffffu, coff, 1);
+      const uint32_t step = __ballot_sync(0xffffffffu, lane < ncol && coff == cn_prev + 1);
 #pragma unroll
-        for (int j = 0; j < CW; ++j) {
-          if (n0 + j >= d.N) break;
+      for (int c = 0; c < CW; c += 4) {
+        float2 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) {
           // the truncations of every chunk shrink it by kTruncBias relative
           // on average; the sum is linear in the chunks, so the expectation
           // is added back once here
-          const float2 v = kahan_value(acc[j]);
-          C[base + cn_tab[n0 + j]] = store_as<TC>(make_float2(fmaf(kTruncBias, v.x, v.x), fmaf(kTruncBias, v.y, v.y)));
+          const float2 re = kahan2_value(ar[(c + j) / 2]), im = kahan2_value(ai[(c + j) / 2]);
+          v[j] = make_float2(fmaf(kTruncBias, re.x, re.x), fmaf(kTruncBias, im.x, im.x));
+          v[j + 1] = make_float2(fmaf(kTruncBias, re.y, re.y), fmaf(kTruncBias, im.y, im.y));
         }
+        int64_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = base + __shfl_sync(0xffffffffu, coff, c + j);
+        if (base < 0) continue;
+        if constexpr (sizeof(TC) == 8) {
+          if (((step >> (c + 1)) & 7u) == 7u && ((uintptr_t)(C + o[0]) & 31) == 0) {
+            asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(C + o[0]), "f"(v[0].x), "f"(v[0].y),
+                         "f"(v[1].x), "f"(v[1].y), "f"(v[2].x), "f"(v[2].y), "f"(v[3].x), "f"(v[3].y)
+                         : "memory");
+            continue;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (c + j < ncol) C[o[j]] = store_as<TC>(v[j]);
       }
     }
   }
@@ -342,19 +445,23 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 int splits_of(int precision) { return precision == PQ_PREC_6XTF32 ? 3 : 2; }
 
-template <typename T, int NS>
-void pack_both(const void* A, int ta, const void* B, int tb, float* pa, float* pb, const GemmDesc& d, int64_t mt,
-               int64_t nt, int64_t kt, cudaStream_t s) {
-  dim3 ga((unsigned)kt, (unsigned)mt, (unsigned)d.Z), gb((unsigned)kt, (unsigned)nt, (unsigned)d.Z);
-  (void)sizeof(T);
-  if (ta == PQ_C128)
-    k_tc_pack<double2, NS, TM><<<ga, 256, 0, s>>>((const double2*)A, pa, d, 0, d.M, mt, kt);
-  else
-    k_tc_pack<float2, NS, TM><<<ga, 256, 0, s>>>((const float2*)A, pa, d, 0, d.M, mt, kt);
-  if (tb == PQ_C128)
-    k_tc_pack<double2, NS, TN><<<gb, 256, 0, s>>>((const double2*)B, pb, d, 1, d.N, nt, kt);
-  else
-    k_tc_pack<float2, NS, TN><<<gb, 256, 0, s>>>((const float2*)B, pb, d, 1, d.N, nt, kt);
+template <typename T, int NS, int ROWS>
+cudaError_t pack(const void* X, float* planes, const GemmDesc& d, int side, int64_t rows, int64_t rtiles, int64_t kt,
+                 cudaStream_t s) {
+  // as many K tiles per block as leave the SMs four blocks each
+  const int64_t kper = std::max<int64_t>(1, std::min<int64_t>(kPackMaxK, kt * rtiles * d.Z / (4 * sm_count())));
+  const dim3 grid((unsigned)ceil_div(kt, kper), (unsigned)rtiles, (unsigned)d.Z);
+  return launch_pdl(k_tc_pack<T, NS, ROWS>, grid, dim3(256), 0, s, (const T*)X, planes, d, side, rows, rtiles, kt,
+                    (int)kper);
+}
+template <int NS>
+cudaError_t pack_both(const void* A, int ta, const void* B, int tb, float* pa, float* pb, const GemmDesc& d,
+                      int64_t mt, int64_t nt, int64_t kt, cudaStream_t s) {
+  cudaError_t e = ta == PQ_C128 ? pack<double2, NS, TM>(A, pa, d, 0, d.M, mt, kt, s)
+                                : pack<float2, NS, TM>(A, pa, d, 0, d.M, mt, kt, s);
+  if (e != cudaSuccess) return e;
+  return tb == PQ_C128 ? pack<double2, NS, TN>(B, pb, d, 1, d.N, nt, kt, s)
+                       : pack<float2, NS, TN>(B, pb, d, 1, d.N, nt, kt, s);
 }
 
 template <typename TC, int NS>
@@ -372,8 +479,8 @@ cudaError_t gemm_launch(const float* pa, const float* pb, void* C, const GemmDes
   }
   const int64_t tiles = mt * nt * d.Z;
   const unsigned grid = (unsigned)std::min<int64_t>(tiles, sm_count());
-  k_tc_gemm<TC, NS><<<grid, kThreads, smem, s>>>(pa, pb, (TC*)C, d, cm, cn, mt, nt, kt, status);
-  return cudaGetLastError();
+  return launch_pdl(k_tc_gemm<TC, NS>, dim3(grid), dim3(kThreads), smem, s, pa, pb, (TC*)C, d, cm, cn, mt, nt, kt,
+                    status);
 }
 
 }  // namespace
@@ -429,16 +536,14 @@ cudaError_t launch_tc(int precision, int ta, int tb, int tc, const void* A, cons
   int64_t* cm = (int64_t*)(pb + d.Z * nt * kt * (int64_t)(2 * NS * kBTile));
   int64_t* cn = cm + d.M;
   const int64_t idx_blocks = std::min<int64_t>(ceil_div(d.M + d.N, 256), 152 * 8);
-  k_result_index<<<(unsigned)idx_blocks, 256, 0, stream>>>(d, cm, cn);
-  cudaError_t e;
+  cudaError_t e = launch_pdl(k_result_index<0>, dim3((unsigned)idx_blocks), dim3(256), 0, stream, d, cm, cn);
+  if (e != cudaSuccess) return e;
   if (NS == 2) {
-    pack_both<float, 2>(A, ta, B, tb, pa, pb, d, mt, nt, kt, stream);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = pack_both<2>(A, ta, B, tb, pa, pb, d, mt, nt, kt, stream)) != cudaSuccess) return e;
     return tc == PQ_C128 ? gemm_launch<double2, 2>(pa, pb, C, d, cm, cn, mt, nt, kt, status, stream)
                          : gemm_launch<float2, 2>(pa, pb, C, d, cm, cn, mt, nt, kt, status, stream);
   }
-  pack_both<float, 3>(A, ta, B, tb, pa, pb, d, mt, nt, kt, stream);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if ((e = pack_both<3>(A, ta, B, tb, pa, pb, d, mt, nt, kt, stream)) != cudaSuccess) return e;
   return tc == PQ_C128 ? gemm_launch<double2, 3>(pa, pb, C, d, cm, cn, mt, nt, kt, status, stream)
                        : gemm_launch<float2, 3>(pa, pb, C, d, cm, cn, mt, nt, kt, status, stream);
 }

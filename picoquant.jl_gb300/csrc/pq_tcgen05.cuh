@@ -9,6 +9,7 @@
 #include <cstdint>
 
 #include "pq_internal.h"
+#include "pq_types.cuh"
 
 namespace pq {
 namespace tcg {
@@ -200,11 +201,14 @@ __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::aft
 template <int Unused = 0>
 __global__ void __launch_bounds__(256) k_result_index(const __grid_constant__ GemmDesc d, int64_t* __restrict__ cm,
                                                       int64_t* __restrict__ cn) {
+  pdl_trigger();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < d.M + d.N; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t o = i < d.M ? decode(i, d.nm, d.mdim, d.msc) : decode(i - d.M, d.nn, d.ndim, d.nsc);
+    pdl_wait();  // the tables may still be read by the launch before
     if (i < d.M)
-      cm[i] = decode(i, d.nm, d.mdim, d.msc);
+      cm[i] = o;
     else
-      cn[i - d.M] = decode(i - d.M, d.nn, d.ndim, d.nsc);
+      cn[i - d.M] = o;
   }
 }
 

@@ -530,3 +530,35 @@ def test_ozaki_wide_many_tiles_per_cta(pq, order, k):
     assert np.all(got[1000] == 0)
     assert np.all(np.abs(got - ref) <= ozaki_bound(A, B, ref))
     _restatement_match(got, A, B)
+
+
+@pytest.mark.parametrize("prec", [2, 4], ids=["3xtf32", "6xtf32"])
+@pytest.mark.parametrize("m,n,k,a_order,c_order", [
+    (64, 64, 272, "mk", "mn"),       # one tile, half its rows padding
+    (1281, 65, 17, "mk", "mn"),      # one row, column and K value past a tile; rows not 32-byte aligned
+    (300, 127, 33, "mk", "nm"),      # transposed result: scattered stores
+    (2500, 128, 68, "km", "mn"),     # A contiguous along M; K tiles grouped in a pack block
+    (20000, 129, 36, "mk", "mn"),    # several output tiles per CTA, odd result rows
+    (128, 4100, 132, "km", "nm"),    # B the wide side
+])
+def test_tf32_tile_edges(pq, prec, m, n, k, a_order, c_order):
+    """The TF32 kernels at the edges of their 128 x 64 tiles and 16-deep K tiles
+    and on both sides of the wide loads and stores (aligned adjacent values, or
+    not).  TF32 terms of an operand are exact to 2^-22 and a chunk of 16 takes a
+    few truncations of 2^-23, so that an element is within 2^-20 of
+    |row of A| |column of B|."""
+    rng = np.random.default_rng(m + n + k)
+    A = rand(rng, (m, k)).astype(np.complex64)
+    B = rand(rng, (k, n)).astype(np.complex64)
+    be = pq.GB300Backend(prec, small_elems=0)
+    got, nl = run(be, A if a_order == "mk" else A.T, [-1, 1] if a_order == "mk" else [1, -1], B,
+                  [1, -2])
+    if c_order == "nm":
+        # the same product with the operands' roles exchanged: C is stored n by m
+        got, nl = run(be, B, [1, -1], A if a_order == "mk" else A.T, [-2, 1] if a_order == "mk" else [1, -2])
+        got = got.T
+    be.close()
+    assert nl == TC_LAUNCHES
+    A, B = A.astype(np.complex128), B.astype(np.complex128)
+    bound = np.outer(np.sqrt(np.sum(np.abs(A) ** 2, axis=1)), np.sqrt(np.sum(np.abs(B) ** 2, axis=0)))
+    assert np.all(np.abs(got - A @ B) <= 2.0 ** -20 * bound)

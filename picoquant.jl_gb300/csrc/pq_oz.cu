@@ -290,15 +290,25 @@ __global__ void __launch_bounds__(256) k_oz_exp(const T* __restrict__ X, const _
   }
 }
 
-// Row scale exponents of A when A is contiguous along K (its first K mode
-// has stride 1 and extent >= 2) but not along M: KL consecutive lanes read
-// consecutive k of one row (KL = the first K mode's extent, a power of two,
-// at most 32), combine their maxima with shuffles, and the RS = 32 / KL row
-// groups of a warp take consecutive rows -- when A's first M mode follows its
-// first K mode in memory, every load of a warp is one contiguous 256-byte
-// run.  A warp takes four such steps at a time, twice; one block of 8 warps
-// per 64 RS rows and batch index z.
-template <typename T>
+// Four complex64 values (32 bytes, 32-byte aligned) of a read-only operand.
+__device__ __forceinline__ void ldg256(const void* p, float* v) {
+  asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+      : "l"(p));
+}
+
+// Row scale exponents of A when A is contiguous along K (its first K mode has
+// stride 1 and extent >= 2) but not along M: KL consecutive lanes read the
+// values of one row, V adjacent ones each (V = 4: runs of complex64, one 32-byte
+// load where aligned), combine their maxima with shuffles, and the RS = 32 / KL
+// row groups of a warp take consecutive rows.  V * KL is at most the extent of
+// A's leading contiguous run of K (all K modes that continue it in A, in
+// whatever order B has them), so that a load of a warp covers whole runs.  A
+// warp takes four rows per lane group, a block 8 warps; one z per blockIdx.y.
+// Bound by reading A once: 2^20 rows of 256 complex64 in runs of 16 take
+// 323 us, 6.6 TB/s (537 us when only K modes merged with B's counted as a run:
+// two values per row and load).
+template <typename T, int V>
 __global__ void __launch_bounds__(256) k_oz_exp_k(const T* __restrict__ X, const __grid_constant__ GemmDesc d,
                                                   int64_t rows, int KL, int* __restrict__ e_out) {
   using R = typename Real<T>::R;
@@ -310,35 +320,44 @@ __global__ void __launch_bounds__(256) k_oz_exp_k(const T* __restrict__ X, const
   const int RS = 32 / KL;
   const int sub = lane / KL, kl = lane % KL;
   const int64_t zo = decode(z, d.nz, d.zdim, d.zsa);
-  const int64_t r0 = (int64_t)blockIdx.x * 64 * RS + warp * 8 * RS;
-#pragma unroll 1
-  for (int rr = 0; rr < 8 * RS; rr += 4 * RS) {
-    const T* xr[4];
-    bool v[4];
-    R mx[4];
+  const int64_t r0 = ((int64_t)blockIdx.x * 8 + warp) * 4 * RS + sub;
+  const T* xr[4];
+  bool v[4];
+  R mx[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int64_t row = r0 + i * RS;
+    v[i] = row < rows;
+    xr[i] = X + zo + (v[i] ? decode(row, d.nm, d.mdim, d.msa) : 0);
+    mx[i] = 0;
+  }
+#pragma unroll 2
+  for (int k = V * kl; k < d.K; k += V * KL) {
+    const int64_t o = koff[k];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int64_t row = r0 + rr + i * RS + sub;
-      v[i] = row < rows;
-      xr[i] = X + zo + (v[i] ? decode(row, d.nm, d.mdim, d.msa) : 0);
-      mx[i] = 0;
-    }
-#pragma unroll 2
-    for (int k = kl; k < d.K; k += KL) {
-      const int64_t o = koff[k];
+      if (!v[i]) continue;
+      const T* x = xr[i] + o;
+      if constexpr (V == 4) {
+        if (((uintptr_t)x & 31) == 0) {
+          float f[8];
+          ldg256(x, f);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (v[i]) {
-          const T x = xr[i][o];
-          mx[i] = fmax(mx[i], absmax((R)x.x, (R)x.y));
+          for (int q = 0; q < 8; q += 2) mx[i] = fmaxf(mx[i], absmax(f[q], f[q + 1]));
+          continue;
         }
       }
-    }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      for (int s = KL / 2; s > 0; s >>= 1) mx[i] = fmax(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], s));
-      if (kl == 0 && v[i]) e_out[z * rows + r0 + rr + i * RS + sub] = exp_of(mx[i]);
+      for (int q = 0; q < V; ++q) {
+        const T y = x[q];
+        mx[i] = fmax(mx[i], absmax((R)y.x, (R)y.y));
+      }
     }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    for (int s = KL / 2; s > 0; s >>= 1) mx[i] = fmax(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], s));
+    if (kl == 0 && v[i]) e_out[z * rows + r0 + i * RS] = exp_of(mx[i]);
   }
 }
 
@@ -346,12 +365,19 @@ __global__ void __launch_bounds__(256) k_oz_exp_k(const T* __restrict__ X, const
 // (and its first M mode does not), else the row-per-thread kernel.
 template <typename T>
 void row_exponents(const T* A, const GemmDesc& d, int* ea, cudaStream_t s) {
-  int KL = 1;
-  if (d.nk > 0 && d.ksa[0] == 1 && !(d.nm > 0 && d.msa[0] == 1))
-    while (KL < 32 && 2 * KL <= d.kdim[0]) KL *= 2;
-  if (KL >= 2) {
-    const int64_t rows_per_block = 64 * (32 / KL);
-    k_oz_exp_k<T><<<dim3((unsigned)ceil_div(d.M, rows_per_block), (unsigned)d.Z), 256, 0, s>>>(A, d, d.M, KL, ea);
+  if (d.nk > 0 && d.ksa[0] == 1 && d.kdim[0] >= 2 && !(d.nm > 0 && d.msa[0] == 1)) {
+    int64_t run = d.kdim[0];  // K values adjacent in A
+    for (int i = 1; i < d.nk && d.ksa[i] == run; ++i) run *= d.kdim[i];
+    const bool four = sizeof(T) == 8 && run % 4 == 0;  // K is a multiple of the run
+    int KL = 1;
+    while (KL < 32 && 2 * KL * (four ? 4 : 1) <= run) KL *= 2;
+    const dim3 grid((unsigned)ceil_div(d.M, 8 * 4 * (32 / KL)), (unsigned)d.Z);
+    if constexpr (sizeof(T) == 8)
+      if (four) {
+        k_oz_exp_k<T, 4><<<grid, 256, 0, s>>>(A, d, d.M, KL, ea);
+        return;
+      }
+    k_oz_exp_k<T, 1><<<grid, 256, 0, s>>>(A, d, d.M, KL, ea);
   } else {
     k_oz_exp<T, 128><<<dim3((unsigned)ceil_div(d.M, 128), (unsigned)d.Z), 256, 0, s>>>(A, d, 0, d.M, ea);
   }
@@ -545,13 +571,6 @@ __device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
 }
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-
-// Four complex64 values (32 bytes, 32-byte aligned) of a read-only operand.
-__device__ __forceinline__ void ldg256(const void* p, float* v) {
-  asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-      : "l"(p));
 }
 
 // A values per converter thread and K tile: 8 for complex64 A (whole 16-byte

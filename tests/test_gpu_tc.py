@@ -562,3 +562,25 @@ def test_tf32_tile_edges(pq, prec, m, n, k, a_order, c_order):
     A, B = A.astype(np.complex128), B.astype(np.complex128)
     bound = np.outer(np.sqrt(np.sum(np.abs(A) ** 2, axis=1)), np.sqrt(np.sum(np.abs(B) ** 2, axis=0)))
     assert np.all(np.abs(got - A @ B) <= 2.0 ** -20 * bound)
+
+
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+@pytest.mark.parametrize("k1,k2,k3", [(2, 2, 32), (2, 8, 16), (2, 3, 24), (4, 3, 8), (3, 2, 8), (2, 32, 4), (8, 64, 1)])
+def test_ozaki_row_scales_over_split_k_runs(pq, dtype, k1, k2, k3):
+    """Row exponents of an operand whose leading run along K is several modes
+    that its partner stores apart (runs of 4 to 512, some no multiple of four
+    or of the lanes), with rows of wildly different magnitude; error_bound is
+    the scheme's own bound on each element."""
+    rng = np.random.default_rng(k1 * 1000 + k2 * 10 + k3)
+    m1, m2, n = 5, 301, 96
+    A = rand(rng, (k1, k2, m1, k3, m2)) * np.exp2(rng.integers(-50, 50, size=(1, 1, m1, 1, m2)))
+    B = rand(rng, (k2, n, k1, k3))
+    A, B = A.astype(dtype), B.astype(dtype)
+    be = ozaki_backend(pq, small=0 if dtype is np.complex64 else 1 << 30)
+    got, nl = run(be, A, [1, 2, -1, 3, -2], B, [2, -3, 1, 3])
+    be.close()
+    assert nl == OZ_LAUNCHES
+    A2 = A.astype(np.complex128).transpose(2, 4, 0, 1, 3).reshape(m1 * m2, -1)
+    B2 = B.astype(np.complex128).transpose(2, 0, 3, 1).reshape(-1, n)
+    ref = A2 @ B2
+    assert np.all(np.abs(got.reshape(m1 * m2, n) - ref) <= ozaki_bound(A2, B2, ref))

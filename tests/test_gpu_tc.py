@@ -584,3 +584,30 @@ def test_ozaki_row_scales_over_split_k_runs(pq, dtype, k1, k2, k3):
     B2 = B.astype(np.complex128).transpose(2, 0, 3, 1).reshape(-1, n)
     ref = A2 @ B2
     assert np.all(np.abs(got.reshape(m1 * m2, n) - ref) <= ozaki_bound(A2, B2, ref))
+
+
+@pytest.mark.parametrize("m,n,k,spread", [
+    (2048, 128, 16, 0),     # every warp's columns whole and in range
+    (2500, 200, 16, 10),    # a ragged last column range, rows past the end
+    (1100, 256, 40, 62),    # products of the scales leave the normal floats: both loops in one tile
+])
+def test_ozaki_wide_store_loops(pq, m, n, k, spread):
+    """128-wide tiles store a warp's columns without branches where all scales
+    are normal floats, one by one elsewhere (ragged N, zero rows and columns,
+    results below 2^-126); within the scheme's bound either way.  Results
+    below the smallest normal float round to multiples of 2^-149."""
+    rng = np.random.default_rng(m + n + k)
+    A = rand(rng, (m, k)) * np.exp2(rng.integers(-spread, 1, size=(m, 1)))
+    B = rand(rng, (k, n)) * np.exp2(rng.integers(-spread, 1, size=(1, n)))
+    A[m // 2] = 0
+    B[:, n - 3] = 0
+    A[: m // 3] *= 2.0 ** -min(spread, 60)
+    A, B = A.astype(np.complex64), B.astype(np.complex64)
+    be = ozaki_backend(pq)
+    got, nl = run(be, A, [-1, 1], B, [1, -2])
+    be.close()
+    assert nl == OZ_LAUNCHES
+    A, B = A.astype(np.complex128), B.astype(np.complex128)
+    ref = A @ B
+    assert np.all(got[m // 2] == 0) and np.all(got[:, n - 3] == 0)
+    assert np.all(np.abs(got - ref) <= ozaki_bound(A, B, ref) + 2.0 ** -148)

@@ -299,12 +299,13 @@ __device__ __forceinline__ void ldg256(const void* p, float* v) {
 
 // Row scale exponents of A when A is contiguous along K (its first K mode has
 // stride 1 and extent >= 2) but not along M: KL consecutive lanes read the
-// values of one row, V adjacent ones each (V = 4: runs of complex64, one 32-byte
-// load where aligned), combine their maxima with shuffles, and the RS = 32 / KL
-// row groups of a warp take consecutive rows.  V * KL is at most the extent of
-// A's leading contiguous run of K (all K modes that continue it in A, in
+// values of one row, V adjacent ones each (V = 4: complex64 that k_vector
+// allows, one 32-byte load), combine their maxima with shuffles, and the
+// RS = 32 / KL row groups of a warp take consecutive rows.  V * KL is at most A's
+// leading contiguous run of K (all K modes that continue it in A, in
 // whatever order B has them), so that a load of a warp covers whole runs.  A
-// warp takes four rows per lane group, a block 8 warps; one z per blockIdx.y.
+// warp takes four rows per lane group (no branch between their loads, so that
+// eight are in flight per lane), a block 8 warps; one z per blockIdx.y.
 // Bound by reading A once: 2^20 rows of 256 complex64 in runs of 16 take
 // 323 us, 6.6 TB/s (537 us when only K modes merged with B's counted as a run:
 // two values per row and load).
@@ -322,43 +323,62 @@ __global__ void __launch_bounds__(256) k_oz_exp_k(const T* __restrict__ X, const
   const int64_t zo = decode(z, d.nz, d.zdim, d.zsa);
   const int64_t r0 = ((int64_t)blockIdx.x * 8 + warp) * 4 * RS + sub;
   const T* xr[4];
-  bool v[4];
   R mx[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int64_t row = r0 + i * RS;
-    v[i] = row < rows;
-    xr[i] = X + zo + (v[i] ? decode(row, d.nm, d.mdim, d.msa) : 0);
+    // rows past the end read the last row (and store nothing)
+    const int64_t row = r0 + i * RS < rows ? r0 + i * RS : rows - 1;
+    xr[i] = X + zo + decode(row, d.nm, d.mdim, d.msa);
     mx[i] = 0;
   }
 #pragma unroll 2
   for (int k = V * kl; k < d.K; k += V * KL) {
     const int64_t o = koff[k];
+    if constexpr (V == 4) {
+      float f[4][8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (!v[i]) continue;
-      const T* x = xr[i] + o;
-      if constexpr (V == 4) {
-        if (((uintptr_t)x & 31) == 0) {
-          float f[8];
-          ldg256(x, f);
+      for (int i = 0; i < 4; ++i) ldg256(xr[i] + o, f[i]);
 #pragma unroll
-          for (int q = 0; q < 8; q += 2) mx[i] = fmaxf(mx[i], absmax(f[q], f[q + 1]));
-          continue;
-        }
-      }
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int q = 0; q < V; ++q) {
-        const T y = x[q];
-        mx[i] = fmax(mx[i], absmax((R)y.x, (R)y.y));
-      }
+        for (int q = 0; q < 8; q += 2) mx[i] = fmaxf(mx[i], absmax(f[i][q], f[i][q + 1]));
+    } else {
+      T y[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) y[i] = xr[i][o];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) mx[i] = fmax(mx[i], absmax((R)y[i].x, (R)y[i].y));
     }
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     for (int s = KL / 2; s > 0; s >>= 1) mx[i] = fmax(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], s));
-    if (kl == 0 && v[i]) e_out[z * rows + r0 + i * RS] = exp_of(mx[i]);
+    if (kl == 0 && r0 + i * RS < rows) e_out[z * rows + r0 + i * RS] = exp_of(mx[i]);
   }
+}
+
+// Whether the exponent pass and the converters may read complex64 A as aligned
+// 32-byte runs of four K values: the leading K modes that follow each other in A
+// (in whatever order B has them) make a run from stride 1 whose extent is a
+// multiple of 4 (so runs of 4 from a multiple of 4 never cross it), and every
+// other stride and the base keep the alignment.  Otherwise they read value by
+// value, which coalesces over rows when A's first M mode has stride 1; over rows
+// 128 bytes apart it costs the converters a wavefront of the L1 per row and
+// value, 88 % of its rate (2^20 x 256 x 256 with runs of 16, exponent pass
+// included: 3.35 ms value by value, 2.75 so).
+bool k_vector(const void* A, const GemmDesc& d) {
+  if (((uintptr_t)A & 31) || d.nk < 1 || d.ksa[0] != 1) return false;
+  int64_t run = d.kdim[0];
+  int lead = 1;
+  for (; run % 4 && lead < d.nk && d.ksa[lead] == run; ++lead) run *= d.kdim[lead];
+  if (run % 4) return false;
+  for (int i = lead; i < d.nk; ++i)
+    if (d.ksa[i] % 4) return false;
+  for (int i = 0; i < d.nm; ++i)
+    if (d.msa[i] % 4) return false;
+  for (int i = 0; i < d.nz; ++i)
+    if (d.zsa[i] % 4) return false;
+  return true;
 }
 
 // A's row exponents: the K-major kernel when A's first K mode has stride 1
@@ -368,7 +388,7 @@ void row_exponents(const T* A, const GemmDesc& d, int* ea, cudaStream_t s) {
   if (d.nk > 0 && d.ksa[0] == 1 && d.kdim[0] >= 2 && !(d.nm > 0 && d.msa[0] == 1)) {
     int64_t run = d.kdim[0];  // K values adjacent in A
     for (int i = 1; i < d.nk && d.ksa[i] == run; ++i) run *= d.kdim[i];
-    const bool four = sizeof(T) == 8 && run % 4 == 0;  // K is a multiple of the run
+    const bool four = sizeof(T) == 8 && k_vector(A, d);
     int KL = 1;
     while (KL < 32 && 2 * KL * (four ? 4 : 1) <= run) KL *= 2;
     const dim3 grid((unsigned)ceil_div(d.M, 8 * 4 * (32 / KL)), (unsigned)d.Z);
@@ -1279,29 +1299,6 @@ void prep_b_tn(const void* X, int tn, uint16_t* planes, int* e, const GemmDesc& 
   else if (tn == 64) prep_b<T, 64, S>(X, planes, e, d, rtiles, kt, s);
   else if (tn == 32) prep_b<T, 32, S>(X, planes, e, d, rtiles, kt, s);
   else prep_b<T, 16, S>(X, planes, e, d, rtiles, kt, s);
-}
-
-// Whether the converters may read complex64 A as aligned 32-byte runs of four
-// K values: the leading K modes that follow each other in A (in whatever order
-// B has them) make a run from stride 1 whose extent is a multiple of 4 (so runs
-// of 4 from a multiple of 4 never cross it), and every other stride and the base
-// keep the alignment.  Otherwise they read value by value, which coalesces over
-// rows when A's first M mode has stride 1; over rows 128 bytes apart it costs a
-// wavefront of the L1 per row and value, 88 % of its rate (2^20 x 256 x 256 with
-// runs of 16, exponent pass included: 3.35 ms value by value, 2.75 so).
-bool k_vector(const void* A, const GemmDesc& d) {
-  if (((uintptr_t)A & 31) || d.nk < 1 || d.ksa[0] != 1) return false;
-  int64_t run = d.kdim[0];
-  int lead = 1;
-  for (; run % 4 && lead < d.nk && d.ksa[lead] == run; ++lead) run *= d.kdim[lead];
-  if (run % 4) return false;
-  for (int i = lead; i < d.nk; ++i)
-    if (d.ksa[i] % 4) return false;
-  for (int i = 0; i < d.nm; ++i)
-    if (d.msa[i] % 4) return false;
-  for (int i = 0; i < d.nz; ++i)
-    if (d.zsa[i] % 4) return false;
-  return true;
 }
 
 template <typename TA, typename TC, int TN, int S>

@@ -165,7 +165,7 @@ int fail(Ctx* ctx, int code, const std::string& msg);
 int cuda_fail(Ctx* ctx, cudaError_t e, const char* what);
 
 // Copy device memory to the host and wait for the stream (status checked).
-constexpr size_t kDownBytes = 1 << 18;
+constexpr size_t kDownBytes = 1 << 16;
 int download(Ctx* ctx, void* dst, const void* src, size_t bytes, const char* what);
 
 // Stream-ordered device allocation accounted against the context cap.

@@ -1036,6 +1036,7 @@ def report(args, pq, w, be, plan, rows, cols, depth, value, t_total, times, laun
     roof = None
     cpu = None
     ms_step = 1e3 * t_total / args.steps
+    roof_prec = "ozaki-c64" if prec_name == "ozaki" and args.storage == "c64" else prec_name
     sp = C.c_void_p()
     be.lib.pq_ctx_stream(be.ctx, C.byref(sp))
     ext = torch.cuda.ExternalStream(sp.value)
@@ -1043,7 +1044,7 @@ def report(args, pq, w, be, plan, rows, cols, depth, value, t_total, times, laun
         sliced = w["sliced"]
         ms, batched, feats = plan.profile_sliced(sliced, batch=args.batch)
         roof, kinfo, overall = roofline_from_profile(ms, batched, feats, peaks, peaks_kind,
-                                                     2 ** len(sliced) // args.batch, prec_name, ms_step)
+                                                     2 ** len(sliced) // args.batch, roof_prec, ms_step)
         extra["kernel_classes"] = kinfo
         extra["roofline_all_steps"] = overall
         rec = plan_record(w)
@@ -1136,7 +1137,7 @@ def report(args, pq, w, be, plan, rows, cols, depth, value, t_total, times, laun
         ms = w["plan"].profile()
         feats = w["plan"].features()
         roof, kinfo, overall = roofline_from_profile(ms, np.zeros(len(ms), bool), feats, peaks, peaks_kind, 1,
-                                                     prec_name, ms_step)
+                                                     roof_prec, ms_step)
         extra["kernel_classes"] = kinfo
         extra["roofline_all_steps"] = overall
         # the fidelity check: the open-output result is the whole 2^20 state,
@@ -1150,7 +1151,7 @@ def report(args, pq, w, be, plan, rows, cols, depth, value, t_total, times, laun
         "metric": METRIC, "value": value, "unit": "amplitudes/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": {"c64": "c64", "3xtf32": "c64(3xtf32)", "6xtf32": "c64(6xtf32)",
-                                                           "ozaki": "c64(ozaki-bf16)", "3xbf16": "c64(3xbf16)",
+                                                           "ozaki": "c64(ozaki-fp16x3)", "3xbf16": "c64(3xbf16)",
                                                            "c128": "c128", "ozaki4": "c64(ozaki4-bf16)"}[prec_name]
         if args.storage == "c64" else f"c128({prec_name})",
         "data": "synthetic (seeded random circuits)", "config": workload_config(args, rows, cols, depth),
@@ -1163,8 +1164,10 @@ def report(args, pq, w, be, plan, rows, cols, depth, value, t_total, times, laun
 
 # Tensor-core operations per algorithmic flop of a complex multiply-add:
 # 3xTF32 issues 3 split products of each of 4 real products, 6xTF32 6; the
-# exact-accumulation scheme 15 slice pairs of 4 real products.
-TENSOR_OPS_PER_FLOP = {"3xtf32": 3.0, "6xtf32": 6.0, "ozaki": 15.0}
+# exact-accumulation scheme 15 slice pairs of 4 real products for complex128
+# results and 8 for complex64 results ("ozaki-c64": all the heavy pairs of
+# complex64 storage).
+TENSOR_OPS_PER_FLOP = {"3xtf32": 3.0, "6xtf32": 6.0, "ozaki": 15.0, "ozaki-c64": 8.0}
 # DRAM bytes of one exact-accumulation contraction step (row-exponent pass +
 # GEMM) over its algorithmic bytes (|A| + |B| + |C| once), from an ncu
 # capture of the dominant pair at a quarter height (M = 2^18, N = K = 256):
@@ -1245,7 +1248,7 @@ def roofline_from_profile(ms, batched, feats, peaks, peaks_kind, nchunks, prec_n
             r = TENSOR_OPS_PER_FLOP[prec_name]
             roof.update({"tensor_ops_per_algorithmic_flop": r, "tensor_work_tflops": roof["algorithmic_tflops"] * r,
                          "tensor_work_frac": roof["algorithmic_tflops"] * r * 1e12 / p_tc})
-        if prec_name == "ozaki":
+        if prec_name in ("ozaki", "ozaki-c64"):
             roof["traffic"] = d["bytes"] / d["launches_per_run"] * OZ_CLASS_TRAFFIC_RATIO
             roof["traffic_unit"] = "bytes per launch"
             roof["traffic_source"] = OZ_CLASS_TRAFFIC_SOURCE

@@ -53,9 +53,9 @@ extern "C" {
  * PQ_PREC_3XTF32 : as PQ_PREC_C64, but large GEMM-shaped contractions run on
  *                  the tcgen05 tensor cores: every real product split into
  *                  TF32 hi+lo parts (3 products: hh, hl, lh), FP32 TMEM
- *                  accumulation over 8-deep K chunks folded into
+ *                  accumulation over 16-deep K chunks folded into
  *                  Kahan-compensated FP32 sums.
- * PQ_PREC_3XBF16 : as PQ_PREC_OZAKI with three bf16 slices (6 slice-pair
+ * PQ_PREC_3XBF16 : the scheme of PQ_PREC_OZAKI with three bf16 slices (6 slice-pair
  *                  products, about 21 significant bits: pair error ~1e-6, not
  *                  enough for 1e-6 amplitude error); K > 512 runs as
  *                  PQ_PREC_3XTF32.
@@ -64,16 +64,18 @@ extern "C" {
  * PQ_PREC_OZAKI  : as PQ_PREC_C64, but large GEMM-shaped contractions with
  *                  K <= 512 run the Ozaki scheme on the tcgen05 tensor cores:
  *                  rows of A / columns of B scaled by powers of two, cut into
- *                  five 7-bit bf16 slices, the 15 slice products of level
- *                  <= 4 accumulated in FP32 TMEM where levels 0 and 1 are
- *                  exact; the result is rounded once.  Larger K runs as
+ *                  slices whose products' leading levels are accumulated
+ *                  exactly in FP32 TMEM; the result is rounded once.
+ *                  Complex64 results: three fp16 slices, 8 products,
+ *                  complex128 results: five 7-bit bf16 slices, the 15
+ *                  products of level <= 4.  Larger K runs as
  *                  PQ_PREC_6XTF32.
- * PQ_PREC_OZAKI4 : as PQ_PREC_OZAKI with four slices: the 10 slice products
+ * PQ_PREC_OZAKI4 : the scheme with four bf16 slices: the 10 slice products
  *                  of level <= 3 (residual below 2^-29 of the row / column
- *                  scale), two thirds of the tensor-core work.  With
- *                  complex64 storage its added error is about the size of the
- *                  storage rounding (amplitude errors about twice
- *                  PQ_PREC_OZAKI's); complex128 storage (pq_ctx_set_small_elems
+ *                  scale).  With complex64 storage its added error is about
+ *                  the size of the storage rounding (amplitude errors about
+ *                  twice PQ_PREC_OZAKI's), and it has more products than
+ *                  PQ_PREC_OZAKI has there; complex128 storage (pq_ctx_set_small_elems
  *                  with a large threshold) removes the storage rounding but
  *                  runs the memory-bound steps in FP64.                     */
 #define PQ_PREC_C128    0

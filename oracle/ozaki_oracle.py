@@ -16,7 +16,10 @@ applicability", Numer. Algorithms 59, 2012) as the library runs it:
 
 Level-0 and level-1 sums are exact in both places, so the device result
 equals ``ozaki_matmul`` up to the FP32 rounding of the small level-2-4 sum
-(about 2^-30 relative) before the final rounding.
+(about 2^-30 relative) before the final rounding.  For complex64 results the
+device cuts three fp16 slices instead (grids of 2^-8 and 2^-20 and an 11-bit
+rest; 8 slice pairs, leading levels exact as well): the same value to below
+2^-31 K of the scales before the same final rounding.
 """
 from __future__ import annotations
 

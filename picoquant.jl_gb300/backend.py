@@ -57,8 +57,8 @@ class GB300Backend:
     PREC_C64 (ComplexF32 storage and FP32 math for large tensors),
     PREC_3XTF32 / PREC_6XTF32 (as PREC_C64, with split-precision TF32
     tensor-core products for large pairs), PREC_OZAKI (as PREC_C64, with
-    exact-accumulation bf16-slice tensor-core products for large pairs),
-    PREC_3XBF16 (accepted, runs as PREC_C64).  In the complex64 modes tensors of at most
+    exact-accumulation sliced tensor-core products for large pairs),
+    PREC_OZAKI4 / PREC_3XBF16 (the same scheme with fewer slices).  In the complex64 modes tensors of at most
     ``small_elems`` elements (default 65536) stay complex128: gate tensors and
     small intermediates cost nothing in time, and rounding them would dominate
     the error of the final amplitudes.

@@ -263,13 +263,13 @@ __global__ void __launch_bounds__(256) k_oz_exp(const T* __restrict__ X, const _
   const int64_t* kstr = side == 0 ? d.ksa : d.ksb;
   const int64_t* zstr = side == 0 ? d.zsa : d.zsb;
   for (int t = threadIdx.x; t < ROWS; t += blockDim.x) emax[t] = kExpZero;
-  for (int t = threadIdx.x; t < d.K; t += blockDim.x) koff[t] = decode(t, d.nk, d.kdim, kstr);
+  for (int t = threadIdx.x; t < d.K; t += blockDim.x) koff[t] = decode32(t, d.nk, d.kdim, kstr);
   __syncthreads();
   using R = typename Real<T>::R;
   const int r = threadIdx.x % ROWS, k0 = threadIdx.x / ROWS;
   const int64_t row = rt * ROWS + r;
   if (row < rows) {
-    const T* xr = X + decode(z, d.nz, d.zdim, zstr) + decode(row, nrm, rdim, rstr);
+    const T* xr = X + decode32(z, d.nz, d.zdim, zstr) + decode32(row, nrm, rdim, rstr);
     R mx = 0;
     int64_t k = k0;
     for (; k + 3 * KS < d.K; k += 4 * KS) {
@@ -315,12 +315,12 @@ __global__ void __launch_bounds__(256) k_oz_exp_k(const T* __restrict__ X, const
   using R = typename Real<T>::R;
   __shared__ int64_t koff[kMaxK];
   const int64_t z = blockIdx.y;
-  for (int t = threadIdx.x; t < d.K; t += blockDim.x) koff[t] = decode(t, d.nk, d.kdim, d.ksa);
+  for (int t = threadIdx.x; t < d.K; t += blockDim.x) koff[t] = decode32(t, d.nk, d.kdim, d.ksa);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int RS = 32 / KL;
   const int sub = lane / KL, kl = lane % KL;
-  const int64_t zo = decode(z, d.nz, d.zdim, d.zsa);
+  const int64_t zo = decode32(z, d.nz, d.zdim, d.zsa);
   const int64_t r0 = ((int64_t)blockIdx.x * 8 + warp) * 4 * RS + sub;
   const T* xr[4];
   R mx[4];
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(256) k_oz_exp_k(const T* __restrict__ X, const
   for (int i = 0; i < 4; ++i) {
     // rows past the end read the last row (and store nothing)
     const int64_t row = r0 + i * RS < rows ? r0 + i * RS : rows - 1;
-    xr[i] = X + zo + decode(row, d.nm, d.mdim, d.msa);
+    xr[i] = X + zo + decode32(row, d.nm, d.mdim, d.msa);
     mx[i] = 0;
   }
 #pragma unroll 2

@@ -132,13 +132,13 @@ __global__ void __launch_bounds__(256) k_tc_pack(const T* X, float* planes, cons
   for (int t = threadIdx.x; t < ROWS + nkt * TK; t += blockDim.x) {
     if (t < ROWS) {
       int64_t r = rt * ROWS + t;
-      roff[t] = r < rows ? decode(r, nrm, rdim, rstr) : -1;
+      roff[t] = r < rows ? decode32(r, nrm, rdim, rstr) : -1;
     } else {
       int64_t k = kt0 * TK + (t - ROWS);
-      koff[t - ROWS] = k < d.K ? decode(k, d.nk, d.kdim, kstr) : -1;
+      koff[t - ROWS] = k < d.K ? decode32(k, d.nk, d.kdim, kstr) : -1;
     }
   }
-  const T* Xz = X + decode(z, d.nz, d.zdim, zstr);
+  const T* Xz = X + decode32(z, d.nz, d.zdim, zstr);
   pdl_trigger();
   pdl_wait();
   __syncthreads();

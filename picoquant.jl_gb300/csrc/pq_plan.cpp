@@ -846,6 +846,14 @@ int pq_plan_step_features(pq_plan* p, double* feats) {
 
 namespace {
 
+void drop_sliced_graph(pq_plan* p) {
+  if (p->sgexec) cudaGraphExecDestroy(p->sgexec);
+  p->sgexec = nullptr;
+  p->sg_key.clear();
+  p->sg_args.clear();
+  p->sg_seen = 0;
+}
+
 // Validate the slicing request, (re)compile the batched network and resolve
 // the leaf pointers of the original (ptrs) and batched (lp) networks.
 int prepare_sliced(pq_plan* p, const int64_t* leaf_ids, int n_sliced, const int32_t* sliced_labels, int batch,
@@ -865,6 +873,8 @@ int prepare_sliced(pq_plan* p, const int64_t* leaf_ids, int n_sliced, const int3
   if (st) return st;
   // (re)compile the batched network when the slicing or batch changes
   if (S != p->sl_labels || batch != p->sl_batch || p->scp.steps.empty()) {
+    // a captured sliced run reads the descriptor tables that are replaced below
+    drop_sliced_graph(p);
     const int beta = p->nlabels;  // the batch label
     std::vector<int64_t> ldims = p->label_dims;
     ldims.push_back(batch);
@@ -1024,11 +1034,9 @@ int pq_plan_run_sliced(pq_plan* p, const int64_t* leaf_ids, int n_sliced, const 
     return PQ_OK;
   }
   if (key != p->sg_key || args != p->sg_args) {
-    if (p->sgexec) cudaGraphExecDestroy(p->sgexec);
-    p->sgexec = nullptr;
+    drop_sliced_graph(p);
     p->sg_key = key;
     p->sg_args = args;
-    p->sg_seen = 0;
   }
   // the first call runs directly (it also sets kernel attributes, allocates
   // nothing later); the second identical call is captured and launched

@@ -171,6 +171,40 @@ def test_sliced_run_graph_replay(pq, O, prec):
     be.close()
 
 
+def _replace_pool_blocks(be):
+    """Fill freed device blocks of table size with other data."""
+    rng = np.random.default_rng(0)
+    be.save_tensors([(f"fill{i}", rng.standard_normal(1 << (5 + i % 10)) + 0j) for i in range(60)])
+    be.sync()
+
+
+@pytest.mark.parametrize("between", ["profile", "rejected"])
+def test_sliced_replay_after_another_slicing(pq, O, prec, between):
+    """A captured sliced run reads device tables that another slicing or batch
+    replaces, also when that call only profiles or is rejected after it was
+    prepared: the first run again must be compiled and captured anew."""
+    r, c, d = 3, 4, 8
+    bits = "110100101101"
+    be = pq.GB300Backend(prec)
+    net, g = single_amp_net(pq, be, r, c, d, 7, bits)
+    steps, _, _, _ = pq.planning.best_flop_plan(net, out_edges=[], candidates=("sweep",))
+    plan = pq.NetworkPlan(net, steps=steps, out_edges=[])
+    sliced = plan.choose_slices(max_sliced=4, log2_target=0)
+    amps = [plan.run_sliced(sliced, batch=4) for _ in range(3)]  # direct, captured, replayed
+    if between == "profile":
+        plan.profile_sliced(sliced, batch=2)
+    else:
+        with pytest.raises(pq.PQError):
+            plan.run_sliced(sliced[:2], batch=2, begin=0, end=1 << 20)
+    _replace_pool_blocks(be)
+    amps += [plan.run_sliced(sliced, batch=4) for _ in range(3)]
+    assert all(a == amps[0] for a in amps)
+    ref = O.statevector(r * c, g)[O.amplitude_index(bits)]
+    assert abs(amps[0] - ref) / 2.0 ** (-(r * c) / 2) < TOL[prec]
+    plan.close()
+    be.close()
+
+
 def test_config3_scaled_sliced(pq, O, prec):
     """Config 3 in miniature: 4x4 grid, depth 10, CZ split into bond-2
     virtual edges, 6 sliced bonds (64 identical-shape slices) summed in FP64."""

@@ -875,6 +875,10 @@ int prepare_sliced(pq_plan* p, const int64_t* leaf_ids, int n_sliced, const int3
   if (S != p->sl_labels || batch != p->sl_batch || p->scp.steps.empty()) {
     // a captured sliced run reads the descriptor tables that are replaced below
     drop_sliced_graph(p);
+    // nothing below is keyed as the former slicing any more: a failure on the
+    // way (mode count, compile, memory cap) leaves the next call to start over
+    p->sl_labels.clear();
+    p->sl_batch = 0;
     const int beta = p->nlabels;  // the batch label
     std::vector<int64_t> ldims = p->label_dims;
     ldims.push_back(batch);

@@ -205,6 +205,29 @@ def test_sliced_replay_after_another_slicing(pq, O, prec, between):
     be.close()
 
 
+def test_sliced_run_after_failed_recompile(pq, O, prec):
+    """A recompile for another batch that fails (memory cap) leaves no half of
+    the former slicing behind: the former run again gives its result."""
+    r, c, d = 3, 4, 8
+    bits = "110100101101"
+    be = pq.GB300Backend(prec)
+    net, g = single_amp_net(pq, be, r, c, d, 7, bits)
+    steps, _, _, _ = pq.planning.best_flop_plan(net, out_edges=[], candidates=("sweep",))
+    plan = pq.NetworkPlan(net, steps=steps, out_edges=[])
+    sliced = plan.choose_slices(max_sliced=4, log2_target=0)
+    amps = [plan.run_sliced(sliced, batch=4) for _ in range(3)]
+    be.set_mem_cap(1)
+    with pytest.raises(pq.PQError):
+        plan.run_sliced(sliced, batch=2)
+    be.set_mem_cap(0)
+    amps += [plan.run_sliced(sliced, batch=4) for _ in range(3)]
+    assert all(a == amps[0] for a in amps)
+    ref = O.statevector(r * c, g)[O.amplitude_index(bits)]
+    assert abs(amps[0] - ref) / 2.0 ** (-(r * c) / 2) < TOL[prec]
+    plan.close()
+    be.close()
+
+
 def test_config3_scaled_sliced(pq, O, prec):
     """Config 3 in miniature: 4x4 grid, depth 10, CZ split into bond-2
     virtual edges, 6 sliced bonds (64 identical-shape slices) summed in FP64."""

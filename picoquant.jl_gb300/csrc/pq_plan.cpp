@@ -517,6 +517,11 @@ void resolve(pq_plan* p, const Compiled& cp, const std::vector<const void*>& lea
 
 int ensure_buffers(pq_plan* p, size_t arena, size_t scratch) {
   Ctx* ctx = p->ctx;
+  // a captured plan holds both addresses (the sliced run's graph is keyed by them)
+  if ((arena > p->arena_cap || scratch > p->scratch_cap) && p->gexec) {
+    cudaGraphExecDestroy(p->gexec);
+    p->gexec = nullptr;
+  }
   if (arena > p->arena_cap) {
     if (p->arena) dev_free(ctx, p->arena, p->arena_cap);
     p->arena = nullptr;
@@ -524,10 +529,6 @@ int ensure_buffers(pq_plan* p, size_t arena, size_t scratch) {
     int st = dev_alloc(ctx, arena, &p->arena);
     if (st) return st;
     p->arena_cap = arena;
-    if (p->gexec) {
-      cudaGraphExecDestroy(p->gexec);
-      p->gexec = nullptr;
-    }
   }
   if (scratch > p->scratch_cap) {
     if (p->scratch) dev_free(ctx, p->scratch, p->scratch_cap);

@@ -228,6 +228,43 @@ def test_sliced_run_after_failed_recompile(pq, O, prec):
     be.close()
 
 
+def test_captured_plan_after_scratch_growth(pq):
+    """A captured plan replays its scratch addresses; a sliced run that needs
+    more scratch moves it, after which the plan runs without the graph (the
+    former block belongs to others).  M = 512, N = 64, K = 256 in one pair; as
+    eight slices in a batch the row exponents alone take eight times the
+    scratch."""
+    import ctypes as C
+    from pqgb300 import _lib as L
+
+    rng = np.random.default_rng(5)
+    m, k, n, z = 512, 32, 64, 8
+    A = (rng.standard_normal((m, k, z)) + 1j * rng.standard_normal((m, k, z))).astype(np.complex64)
+    B = (rng.standard_normal((k, n, z)) + 1j * rng.standard_normal((k, n, z))).astype(np.complex64)
+    be = pq.GB300Backend(pq.PREC_OZAKI, small_elems=0)
+    be.save_tensor_data("a", A)
+    be.save_tensor_data("b", B)
+    h = C.c_void_p()
+    L.check(be.lib.pq_plan_create(be.ctx, 2, L.arr(C.c_int32, [3, 3]), L.arr(C.c_int32, [0, 1, 3, 1, 2, 3]), 4,
+                                  L.arr(C.c_int64, [m, k, n, z]), 1, L.arr(C.c_int32, [0, 1]), 2,
+                                  L.arr(C.c_int32, [0, 2]), C.byref(h)), be.ctx, "plan_create")
+    ids = L.arr(C.c_int64, [be.id_of("a"), be.id_of("b")])
+    L.check(be.lib.pq_plan_execute(h, ids, be.id_of("r")), be.ctx, "execute")
+    L.check(be.lib.pq_plan_capture(h, ids, be.id_of("r")), be.ctx, "capture")
+    before = be.load_tensor_data("r")
+    L.check(be.lib.pq_plan_run_sliced(h, ids, 1, L.arr(C.c_int32, [3]), 0, z, z, 1), be.ctx, "run_sliced")
+    be.sync()
+    fill = rng.standard_normal(1 << 10) + 0j
+    be.save_tensors([(f"fill{i}", fill) for i in range(100)])
+    L.check(be.lib.pq_plan_execute(h, ids, be.id_of("r")), be.ctx, "execute")
+    assert np.array_equal(be.load_tensor_data("r"), before)
+    assert all(np.array_equal(be.load_tensor_data(f"fill{i}"), fill.astype(np.complex64)) for i in range(100))
+    ref = np.einsum("mkz,knz->mn", A.astype(np.complex128), B.astype(np.complex128))
+    assert rel(before, ref) < 1e-6
+    be.lib.pq_plan_destroy(h)
+    be.close()
+
+
 def test_config3_scaled_sliced(pq, O, prec):
     """Config 3 in miniature: 4x4 grid, depth 10, CZ split into bond-2
     virtual edges, 6 sliced bonds (64 identical-shape slices) summed in FP64."""

@@ -101,3 +101,52 @@ def error_bound(A, B, ref, n_slices=N_SLICES):
     K = A.shape[1]
     scale = np.exp2(np.minimum(ea, 4096)[:, None] + np.minimum(eb, 4096)[None, :])
     return 2.0 ** -23 * np.abs(ref) + (2.0 ** -(7 * n_slices - 3) * K + 2.0 ** -29) * scale
+
+
+def scaled(X):
+    """Rows of X times 2^-e, and e."""
+    e = row_exponents(X)
+    return X * np.exp2(np.where(e == ZERO_EXP, 0, -e).astype(np.float64))[:, None], e
+
+
+def truncate24(x):
+    """x rounded toward zero to FP32's 24 significant bits."""
+    m, e = np.frexp(x)
+    return np.ldexp(np.trunc(np.ldexp(m, 24)), e - 24)
+
+
+def accumulate(A, B, half=False, order=None):
+    """A @ B as the tensor core adds it up, unrounded: 16-term sums of exact
+    products, each added to its level's accumulator and truncated, K tile by K
+    tile.  Five bf16 slices (the fp16 split, ``half``, is not restated), within
+    a K tile by level with the smallest of the rest first (``order`` "level"),
+    or by slice of A and of B from the last to the first ("slice")."""
+    assert not half
+    K = A.shape[1]
+    As, ea = scaled(A)
+    Bs, eb = scaled(B.T)
+    a = [slices(v) for v in (As.real, As.imag)]
+    b = [slices(v.T) for v in (Bs.real, Bs.imag)]
+    order = order or "level"
+    ps = [(i, j) for i in range(N_SLICES) for j in range(N_SLICES - i)][::-1]
+    if order == "level":
+        ps.sort(key=lambda p: (min(p[0] + p[1], 2), -(p[0] + p[1])))
+    groups = []  # (slice of A, its slices of B) in issue order
+    for i, j in ps:
+        if order == "slice" and groups and groups[-1][0] == i:
+            groups[-1][1].append(j)
+        else:
+            groups.append((i, [j]))
+    out = np.zeros((2, 3, A.shape[0], B.shape[1]))  # (re, im) x level
+    for k in range(0, K, 16):
+        t = slice(k, min(K, k + 16))
+        for i, js in groups:
+            for part in range(2):
+                for j in js:
+                    lv, bp = min(i + j, 2), b[part][j][t]
+                    x = (a[0][i], -a[1][i]) if part else (a[0][i], a[1][i])
+                    re, im = (x[1], x[0]) if part else (x[0], x[1])
+                    out[0, lv] = truncate24(out[0, lv] + re[:, t] @ bp)
+                    out[1, lv] = truncate24(out[1, lv] + im[:, t] @ bp)
+    scale = np.exp2((ea[:, None] + eb[None, :]).astype(np.float64))
+    return (out[0].sum(0) + 1j * out[1].sum(0)) * scale

@@ -186,8 +186,11 @@ __host__ __device__ constexpr int narrow_col(int i) {
   return c;
 }
 
-// slice pairs, level 0 first, then level 1, then the higher levels (the
-// inexact accumulator takes its small terms first).  Five slices:
+// Slice pairs, level 0 first, then level 1, then the rest with the smallest
+// first.  The order in which the bf16 splits issue them (the truncating rest
+// accumulator then takes the fewest additions at full size: by slice of A from
+// the first its rms error is 5 to 20 % larger, K = 512 to 32), and in which the
+// epilogue of 16-wide tiles adds the pairs' regions up.  Five slices:
 //   i: 0 0 1 0 1 2 3 4 0 1 2 3 0 1 2
 //   j: 0 1 0 4 3 2 1 0 3 2 1 0 2 1 0
 // four slices (levels 0 to 3, ten pairs):
@@ -706,15 +709,30 @@ __global__ void __launch_bounds__(kThreads, 1)
     int s = 0;       // ring stage and its phase
     uint32_t ph = 0;
     int64_t t = 0;   // tiles of this CTA
-    // The MMAs of the K tile in stage `st`, levels lo .. hi (2: the rest).  The
-    // MMAs of one A operand follow each other: the first fills the tensor
-    // core's A buffer from shared memory, the others use it (an M = N = 128 MMA
-    // reads 8 KB in its 64 cycles, all of the SM's shared-memory bandwidth; with
-    // A kept, kHalf reads 88 KB per K tile instead of 128 KB: 7 % of the wide
-    // pair's time).  `first` overwrites the levels; l2 is the column of level 2.
+    // The MMAs of the K tile in stage `st`, levels lo .. hi (2: the rest).
+    // kHalf: the MMAs of one A operand follow each other: the first fills the
+    // tensor core's A buffer from shared memory, the others use it (an M = N =
+    // 128 MMA reads 8 KB in its 64 cycles, all of the SM's shared-memory
+    // bandwidth; with A kept, kHalf reads 88 KB per K tile instead of 128 KB: 7 %
+    // of the wide pair's time).  bf16 slices: level by level (pair_i).  `first`
+    // overwrites the levels; l2 is the column of level 2.
     auto issue = [&](int st, int lo, int hi, bool first, uint32_t set, uint32_t l2) {
       const uint32_t sa = smem_u32(sm.stage[st]) >> 4;
       constexpr uint32_t BOFF = (kSlices * kStackBytes) >> 4;
+      if constexpr (!Sl<S>::half) {
+#pragma unroll
+        for (int q = 0; q < kPairs; ++q) {
+          const int i = pair_i<S>(q), j = pair_j<S>(q), lv = i + j < 2 ? i + j : 2;
+          if (lv < lo || lv > hi) continue;
+          const uint32_t dl = tmem + (lv < 2 ? set + (uint32_t)(lv * TN) : l2);
+#pragma unroll
+          for (int part = 0; part < 2; ++part)  // the first pair of each level overwrites it
+            mma_f16(dl, desc_at(sa + ((i * kStackBytes + part * 8 * 128) >> 4), ALBO, SBO),
+                    desc_at(sa + BOFF + (((part * kSlices + j) * CF::kBTile * 2) >> 4), BLBO, SBO),
+                    part ? idesc_neg : idesc, first && part == 0 && (q < 2 || q == 3) ? 0u : 1u);
+        }
+        return;
+      }
 #pragma unroll
       for (int i = 0; i < kSlices; ++i) {
 #pragma unroll

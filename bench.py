@@ -1151,7 +1151,7 @@ def report(args, pq, w, be, plan, rows, cols, depth, value, t_total, times, laun
         "metric": METRIC, "value": value, "unit": "amplitudes/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": {"c64": "c64", "3xtf32": "c64(3xtf32)", "6xtf32": "c64(6xtf32)",
-                                                           "ozaki": "c64(ozaki-fp16x3)", "3xbf16": "c64(3xbf16)",
+                                                           "ozaki": "c64(ozaki-fp16x4)", "3xbf16": "c64(3xbf16)",
                                                            "c128": "c128", "ozaki4": "c64(ozaki4-bf16)"}[prec_name]
         if args.storage == "c64" else f"c128({prec_name})",
         "data": "synthetic (seeded random circuits)", "config": workload_config(args, rows, cols, depth),
@@ -1165,9 +1165,9 @@ def report(args, pq, w, be, plan, rows, cols, depth, value, t_total, times, laun
 # Tensor-core operations per algorithmic flop of a complex multiply-add:
 # 3xTF32 issues 3 split products of each of 4 real products, 6xTF32 6; the
 # exact-accumulation scheme 15 slice pairs of 4 real products for complex128
-# results and 8 for complex64 results ("ozaki-c64": all the heavy pairs of
-# complex64 storage).
-TENSOR_OPS_PER_FLOP = {"3xtf32": 3.0, "6xtf32": 6.0, "ozaki": 15.0, "ozaki-c64": 8.0}
+# results and 11 for complex64 results with K <= 256 ("ozaki-c64": all the heavy
+# pairs of complex64 storage).
+TENSOR_OPS_PER_FLOP = {"3xtf32": 3.0, "6xtf32": 6.0, "ozaki": 15.0, "ozaki-c64": 11.0}
 # DRAM bytes of one exact-accumulation contraction step (row-exponent pass +
 # GEMM) over its algorithmic bytes (|A| + |B| + |C| once), from an ncu
 # capture of the dominant pair at a quarter height (M = 2^18, N = K = 256):

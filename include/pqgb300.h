@@ -66,9 +66,9 @@ extern "C" {
  *                  rows of A / columns of B scaled by powers of two, cut into
  *                  slices whose products' leading levels are accumulated
  *                  exactly in FP32 TMEM; the result is rounded once.
- *                  Complex64 results: three fp16 slices, 8 products,
- *                  complex128 results: five 7-bit bf16 slices, the 15
- *                  products of level <= 4.  Larger K runs as
+ *                  Five 7-bit bf16 slices, the 15 products of level <= 4, or
+ *                  for complex64 results with K <= 256 four fp16 slices, 11
+ *                  products, whose error is no larger.  Larger K runs as
  *                  PQ_PREC_6XTF32.
  * PQ_PREC_OZAKI4 : the scheme with four bf16 slices: the 10 slice products
  *                  of level <= 3 (residual below 2^-29 of the row / column

@@ -16,10 +16,15 @@ applicability", Numer. Algorithms 59, 2012) as the library runs it:
 
 Level-0 and level-1 sums are exact in both places, so the device result
 equals ``ozaki_matmul`` up to the FP32 rounding of the small level-2-4 sum
-(about 2^-30 relative) before the final rounding.  For complex64 results the
-device cuts three fp16 slices instead (grids of 2^-8 and 2^-20 and an 11-bit
-rest; 8 slice pairs, leading levels exact as well): the same value to below
-2^-31 K of the scales before the same final rounding.
+(about 2^-30 relative) before the final rounding.
+
+For complex64 results with K <= 256 the device cuts four fp16 slices instead
+(``half_slices``): s0 and s1 on fixed grids chosen so that levels 0 and 1 are
+exact again, s2 the remainder rounded to fp16's 11 bits and s3 the rest of
+that; 11 slice pairs (``HALF_PAIRS``).  Its residual and the pairs it drops are
+smaller than the five-slice scheme's, so ``error_bound`` holds for both.
+``accumulate`` restates the tensor core's sums of either split in the
+kernel's order (additions truncated to FP32's 24 bits).
 """
 from __future__ import annotations
 
@@ -103,10 +108,54 @@ def error_bound(A, B, ref, n_slices=N_SLICES):
     return 2.0 ** -23 * np.abs(ref) + (2.0 ** -(7 * n_slices - 3) * K + 2.0 ** -29) * scale
 
 
+# ---- four fp16 slices (complex64 results, K <= 256) --------------------------
+
+HALF_MAX_K = 256
+# slice 0 of A meets slices 0 .. 3 of B, slices 1 and 2 meet 0 .. 2, slice 3 meets 0
+HALF_MET = (4, 3, 3, 1)
+HALF_PAIRS = [(i, j) for i in range(4) for j in range(HALF_MET[i])]
+
+
+def half_bits(K, side):
+    """Bits of the first slice's grid and how many more the second's has, for
+    the rows of A (side 0) or the columns of B (side 1)."""
+    return (8 if K <= (128 if side == 0 else 256) else 7), (8 if K <= 128 else 7)
+
+
+def half_slices(x, K, side):
+    """The fp16 slices of x (|x| < 1); the device holds them times 2^15, which
+    is why a value below 2^-29 is a multiple of 2^-39."""
+    b0, more = half_bits(K, side)
+    r = np.array(x, dtype=np.float64)
+    out = []
+    for g in (2.0 ** b0, 2.0 ** (b0 + more)):
+        out.append(np.rint(r * g) / g)
+        r = r - out[-1]
+    for _ in range(2):
+        out.append(np.float64(np.float16(r * 2.0 ** 15)) * 2.0 ** -15)
+        r = r - out[-1]
+    return out
+
+
 def scaled(X):
     """Rows of X times 2^-e, and e."""
     e = row_exponents(X)
     return X * np.exp2(np.where(e == ZERO_EXP, 0, -e).astype(np.float64))[:, None], e
+
+
+def half_matmul(A, B):
+    """C = A @ B (K <= 256) from four fp16 slices, sums in FP64: (the FP64
+    value of the kept pairs, levels unscaled)."""
+    K = A.shape[1]
+    As, ea = scaled(A)
+    Bs, eb = scaled(B.T)
+    a = [half_slices(v, K, 0) for v in (As.real, As.imag)]
+    b = [half_slices(v.T, K, 1) for v in (Bs.real, Bs.imag)]
+    lv = [np.zeros((A.shape[0], B.shape[1]), dtype=np.complex128) for _ in range(3)]
+    for i, j in HALF_PAIRS:
+        lv[min(i + j, 2)] += (a[0][i] @ b[0][j] - a[1][i] @ b[1][j]) + 1j * (a[0][i] @ b[1][j] + a[1][i] @ b[0][j])
+    scale = np.exp2((ea[:, None] + eb[None, :]).astype(np.float64))
+    return (lv[0] + lv[1] + lv[2]) * scale, lv
 
 
 def truncate24(x):
@@ -115,20 +164,21 @@ def truncate24(x):
     return np.ldexp(np.trunc(np.ldexp(m, 24)), e - 24)
 
 
-def accumulate(A, B, half=False, order=None):
+def accumulate(A, B, half, order=None):
     """A @ B as the tensor core adds it up, unrounded: 16-term sums of exact
     products, each added to its level's accumulator and truncated, K tile by K
-    tile.  Five bf16 slices (the fp16 split, ``half``, is not restated), within
-    a K tile by level with the smallest of the rest first (``order`` "level"),
-    or by slice of A and of B from the last to the first ("slice")."""
-    assert not half
+    tile.  ``half``: four fp16 slices, within a K tile by slice of A and of B
+    from the last to the first; else five bf16 ones, within a K tile by level
+    with the smallest of the rest first (``order`` "level"), or "slice" as the
+    others."""
     K = A.shape[1]
     As, ea = scaled(A)
     Bs, eb = scaled(B.T)
-    a = [slices(v) for v in (As.real, As.imag)]
-    b = [slices(v.T) for v in (Bs.real, Bs.imag)]
-    order = order or "level"
-    ps = [(i, j) for i in range(N_SLICES) for j in range(N_SLICES - i)][::-1]
+    cut = (lambda v, side: half_slices(v, K, side)) if half else (lambda v, side: slices(v))
+    a = [cut(v, 0) for v in (As.real, As.imag)]
+    b = [cut(v.T, 1) for v in (Bs.real, Bs.imag)]
+    order = order or ("slice" if half else "level")
+    ps = (list(HALF_PAIRS) if half else [(i, j) for i in range(N_SLICES) for j in range(N_SLICES - i)])[::-1]
     if order == "level":
         ps.sort(key=lambda p: (min(p[0] + p[1], 2), -(p[0] + p[1])))
     groups = []  # (slice of A, its slices of B) in issue order

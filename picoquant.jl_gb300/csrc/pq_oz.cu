@@ -2,7 +2,7 @@
 // cores (sm_103a, PQ_PREC_OZAKI): the Ozaki scheme (Ozaki, Ogita, Oishi, Rump,
 // "Error-free transformations of matrix multiplication by using fast routines
 // of matrix multiplication and its applicability", Numer. Algorithms 59, 2012)
-// with bf16 slices and FP32 accumulation in TMEM.
+// with 16-bit slices and FP32 accumulation in TMEM.
 //
 // Scaling.  Every row m of A (over K, per batch index) gets the power of two
 // 2^ea[m] with every |Re|, |Im| of the row below it (frexp exponent of the row
@@ -11,21 +11,8 @@
 // and B's slice j are accumulated by level i + j into three FP32 accumulators
 // per real output (Cr, Ci): level 0, level 1 and the rest.
 //
-// Complex64 results of PQ_PREC_OZAKI (kHalf): three fp16 slices, s0 on a grid of
-// 2^-8 (or 2^-7, below), s1 on one 12 bits finer, s2 the rest with 11 bits, so
-// x - (s0 + s1 + s2) is below 2^-33 (2^-32); 8 of the 9 products (all but the
-// 2^-40-sized s2 t2).  Level 0 sums 2K products of multiples of 2^-16 of size at
-// most 1: with 8 bits in s0 and t0 it fits the 24-bit significand exactly for K
-// <= 128, with 7 and 8 for K <= 256, with 7 and 7 for K <= 512, so the tensor
-// core never drops a bit of it.  Level 1 is on a grid of 2^-28 .. 2^-26 and
-// about 2^-5 in size for rows without structure, exact as well; where it is
-// larger its truncation is below 2^-28 of the level-0 sums that come with it.
-// The split's error, at most 2^-31 K of the scales and near 2^-32 of the result
-// on random pairs, is far below the complex64 rounding (3.5e-8 of max |C|
-// either way), so 8 products give what five bf16 slices gave with 15: the pair
-// M = 2^18, N = K = 256 takes 0.90 ms instead of 1.47.
-//
-// Complex128 results keep five bf16 slices
+// Five bf16 slices (PQ_PREC_OZAKI: complex128 results, and complex64 ones with
+// K > 256)
 //   s0 = rint(x 2^7) 2^-7,  s_i = rint((x - s0 - .. - s_{i-1}) 2^{7(i+1)}) 2^{-7(i+1)}
 // (|s0| <= 1, |s_i| <= 2^{-7i-1}), each an integer of at most 8 bits times a
 // power of two, hence exact in bf16; x - (s0 + .. + s4) is below 2^-36, so a
@@ -36,11 +23,27 @@
 //   level 1   (0,1) (1,0)       multiples of 2^-21, |sum| <= 4K 2^-8
 //   levels 2-4 (the other 12)   |sum| <= 2^-14 relative
 // For K <= 512 the level-0 and level-1 sums are exact in FP32; only the small
-// levels 2-4 round (truncation, about 2^-30 relative after K).  The result is
+// levels 2-4 round (toward zero, K / 16 times per pair).  The result is
 // (L0 + L1 + L2) 2^(ea+eb) rounded once to the output type, so the error is
-// the output rounding plus the dropped pairs and slice residuals, at most
-// 2^-33 K 2^(ea+eb) per component.  (Four 7-bit slices, ten pairs, double the
-// amplitude error of deep circuits: their rows span many binades.)
+// the output rounding, the dropped pairs and slice residuals, at most 2^-33 K
+// 2^(ea+eb) per component, and the rest's roundings (rms 2^-34 of the scales
+// for K = 16, 2^-30 for 256, 2^-28 for 512 on random operands).  (Four 7-bit
+// slices, ten pairs, double the amplitude error of deep circuits: their rows
+// span many binades.)
+//
+// Four fp16 slices (kHalf, PQ_PREC_OZAKI with complex64 results and K <= 256): s0
+// on a grid of 2^-8 or 2^-7, s1 on one 8 or 7 bits finer (first_bits,
+// second_bits: as fine as leaves levels 0 and 1 exact in FP32 whatever the
+// operands are), s2 the remainder in fp16's 11 bits, s3 the rest of that, so
+// x - (s0 + .. + s3) is at most 2^-39.  11 pairs: all but (1,3) (3,1) (2,3)
+// (3,2) (3,3), at most 2^-35 in all, where the five bf16 slices drop 2^-35 and
+// have twice a residual of 2^-36.  The rest takes 8 pairs of the same sizes
+// instead of 12.  So no operand keeps fewer bits and no error is larger than
+// with the five slices, and 11 products do (rest's rms 2^-36 for K = 16, 2^-30.2
+// for 256).  Three fp16 slices with 12 bits in s1 (8 products) were faster and not
+// sound: level 1 then has up to 29 bits for the accumulator's 24, which shows
+// where level 0 cancels (K = 512, A alternating +-0.75 plus 2^-8: error 1.3e-6 of
+// the scales, 3e-8 with level 1 exact).
 //   Cr = Ar.Br + (-Ai).Bi   (the negation is the MMA's negate-A bit)
 //   Ci = Ar.Bi + Ai.Br
 //
@@ -64,8 +67,8 @@
 //                   tiles (TN = 128, or 64 / 32 / 16 for narrow pairs; a pair
 //                   whose A side is the narrow one runs as B x A):
 //     warp 0       producer: cp.async.bulk of B's plane tiles of one
-//                  16-deep K tile into the shared-memory ring;
-//     warp 1       TMEM owner and MMA issuer: 16 tcgen05.mma (kind::f16; 30
+//                  16-deep K tile into B's shared-memory ring;
+//     warp 1       TMEM owner and MMA issuer: 22 tcgen05.mma (kind::f16; 30
 //                  for five slices) per K tile into three TN-column
 //                  accumulators (levels 0, 1, rest); narrow tiles (TN <= 64)
 //                  alternate between two such sets, so a tile's MMAs do not
@@ -76,7 +79,7 @@
 //     8 or 12 warps A converters: gather A's 64 x 16 complex values of the K
 //                  tile through its index map straight from HBM (the group's
 //                  next K tile in flight while this one is sliced), slice
-//                  them and store the [Ar; Ai; -Ar] stacks into the ring (no
+//                  them and store the [Ar; Ai; -Ar] stacks into A's ring (no
 //                  slice planes of A ever reach HBM); for complex64 A two
 //                  groups of four warps take alternate K tiles, each thread
 //                  8 consecutive k of one row, so every store is a whole
@@ -114,24 +117,26 @@ constexpr int kExpZero = -4096;                  // exponent of an all-zero row
 constexpr int64_t kMaxK = 512;                   // exact level-0/1 sums up to this K
 
 // Tile width N: 128 for general pairs, 64 / 32 / 16 for narrow ones.
-// Split of a real value: kHalf for PQ_PREC_OZAKI with complex64 results (three
-// fp16 slices, the 8 pairs but (2,2)); bf16 slices for the others: 5 for
-// PQ_PREC_OZAKI with complex128 results (15 slice pairs, i + j <= 4), 4 for
-// PQ_PREC_OZAKI4 (10 pairs, i + j <= 3), 3 for PQ_PREC_3XBF16 (6 pairs,
-// i + j <= 2).
+// Split of a real value: kHalf for PQ_PREC_OZAKI with complex64 results and K <=
+// kHalfMaxK (four fp16 slices, 11 pairs); bf16 slices for the others: 5 for
+// PQ_PREC_OZAKI (15 slice pairs, i + j <= 4), 4 for PQ_PREC_OZAKI4 (10 pairs,
+// i + j <= 3), 3 for PQ_PREC_3XBF16 (6 pairs, i + j <= 2).
 constexpr int kHalf = 8;
+constexpr int64_t kHalfMaxK = 256;
 template <int S>
 struct Sl {
   static_assert(S == kHalf || S == 5 || S == 4 || S == 3, "split");
   static constexpr bool half = S == kHalf;
-  static constexpr int n = half ? 3 : S;      // slices
+  static constexpr int n = half ? 4 : S;      // slices
   static constexpr int planes = 2 * n;        // per operand: Re s0.., Im s0..
-  static constexpr int pairs = half ? 8 : (S == 5 ? 15 : (S == 4 ? 10 : 6));
+  static constexpr int pairs = half ? 11 : (S == 5 ? 15 : (S == 4 ? 10 : 6));
   // slices 0 .. met(i) - 1 of B meet slice i of A
-  __host__ __device__ static constexpr int met(int i) { return half ? (i < 2 ? 3 : 2) : n - i; }
+  __host__ __device__ static constexpr int met(int i) {
+    return half ? (i == 0 ? 4 : (i == 3 ? 1 : 3)) : n - i;
+  }
 };
 // Converter warps (the rest are epilogue warps): 12 for 16- and 32-wide tiles of
-// complex64 A in three slices, whose few MMAs wait for A's loads -- a third
+// complex64 A in fp16 slices, whose few MMAs wait for A's loads -- a third
 // group of converters keeps half as much again in flight (2^20 x 16 x 256: 0.9 ->
 // 0.7 ms; a second K tile per thread spilled) -- else 8.
 template <typename TA, int TN, int S>
@@ -139,14 +144,18 @@ __host__ __device__ constexpr int conv_warps() {
   return TN <= 32 && Sl<S>::half && sizeof(TA) == 8 ? 12 : 8;
 }
 // kHalf: scaled values are held times 2^kHalfUp, so that the lowest bits of
-// the third slice stay in fp16's range.
+// the last slice stay in fp16's range (its subnormals, 2^-24, are 2^-39).
 constexpr int kHalfUp = 15;
-// Bits of the first slice (a grid of 2^-bits): with a + b bits and K terms of
-// two real products, a level-0 sum is at most 2K on a grid of 2^-(a+b), which
-// fits the 24-bit significand while a + b + 1 + log2 K <= 24.
+// Bits of the first slice (a grid of 2^-bits) and how many more the second has.
+// With a and b first bits and K terms of two real products, a level-0 sum is at
+// most 2K on a grid of 2^-(a+b): 24 bits for a + b + 1 + log2 K <= 24, so 8 and 8
+// for K <= 128, 7 and 8 for K <= 256.  Level 1 is at most 2K (2^-(a+1) + 2^-(b+1))
+// on a grid of 2^-(a+b+more): 1 and 2^-24 for K <= 128 with 8 more bits, 3 and
+// 2^-22 for K <= 256 with 7 more.
 __host__ __device__ constexpr int first_bits(int64_t k, int side) { return k <= (side == 0 ? 128 : 256) ? 8 : 7; }
+__host__ __device__ constexpr int second_bits(int64_t k) { return k <= 128 ? 8 : 7; }
 
-// 128-wide tiles of three slices with complex64 results: the epilogue parks a
+// 128-wide tiles of kHalf or three slices with complex64 results: the epilogue parks a
 // tile's sums in shared memory (and stores whole complex values from there),
 // and the fourth TMEM block lets the next tile's MMAs of levels 2 and up start
 // before the epilogue has read this one.  Against parking in the fourth block
@@ -155,15 +164,21 @@ __host__ __device__ constexpr int first_bits(int64_t k, int side) { return k <= 
 // three.
 template <typename TC, int TN, int S>
 __host__ __device__ constexpr bool oz_park() {
-  return TN == 128 && Sl<S>::n == 3 && sizeof(TC) == 8;
+  return TN == 128 && (Sl<S>::half || S == 3) && sizeof(TC) == 8;
 }
 
 template <int TN, int S, bool PARK>
 struct OzCfg {
   static constexpr int kBTile = TN * TK;                                   // 16-bit values per B plane tile
   static constexpr uint32_t b_bytes = Sl<S>::planes * kBTile * 2;          // B planes of one K tile
-  static constexpr uint32_t stage_bytes = Sl<S>::n * kStackBytes + b_bytes;
-  static constexpr int stages = PARK ? 3 : (Sl<S>::half ? 6 : ((TN == 128 && S >= 4) ? 3 : 4));
+  static constexpr uint32_t a_bytes = Sl<S>::n * kStackBytes;              // A stacks of one K tile
+  // Rings of A stacks and of B planes.  Beside parked sums 227 KB hold two
+  // stages of four slices of A (24 KB) and three of B (32 KB): A's stores are
+  // short once a stage is free, B's copies take their time.
+  static constexpr int b_stages = PARK ? 3 : (Sl<S>::half ? (TN == 64 ? 5 : 6) : ((TN == 128 && S >= 4) ? 3 : 4));
+  static constexpr int a_stages = PARK && Sl<S>::half ? 2 : b_stages;
+  // rings of one length are one ring: a stage of both has one pair of barriers
+  static constexpr bool one_ring = a_stages == b_stages;
   // 16-wide tiles: one MMA per A slice i against B slices 0 .. met(i)-1 side
   // by side (N = 16 met(i)), every slice pair in its own TMEM region
   static constexpr bool narrow = TN == 16;
@@ -175,7 +190,7 @@ struct OzCfg {
   static constexpr int acc_sets = TN <= 64 ? 2 : 1;
   static constexpr uint32_t tmem_cols =
       TN == 128 ? 512 : (TN == 64 ? 512 : (TN == 32 ? 256 : (2 * set_cols > 256 ? 512 : 256)));
-  static_assert(acc_sets * set_cols <= (int)tmem_cols && stage_bytes % 1024 == 0, "tile width");
+  static_assert(acc_sets * set_cols <= (int)tmem_cols && a_bytes % 1024 == 0 && b_bytes % 1024 == 0, "tile width");
 };
 
 // First TMEM column of A slice i's region in a narrow tile.
@@ -200,19 +215,19 @@ __host__ __device__ constexpr int narrow_col(int i) {
 //   i: 0 0 1 0 1 2
 //   j: 0 1 0 2 1 0
 // kHalf:
-//   i: 0 0 1 1 2 0 2 1
-//   j: 0 1 0 2 1 2 0 1
+//   i: 0 0 1 2 3 0 2 1 2 0 1
+//   j: 0 1 0 2 0 3 1 2 0 2 1
 // (4-bit fields, pair p in bits [4p, 4p + 4))
 template <int S>
 __host__ __device__ constexpr int pair_i(int p) {
-  return (int)((S == kHalf ? 0x12021100ull
+  return (int)((S == kHalf ? 0x10212032100ull
                            : (S == 5 ? 0x210321043210100ull : (S == 4 ? 0x2103210100ull : 0x210100ull))) >>
                (4 * p)) &
          15;
 }
 template <int S>
 __host__ __device__ constexpr int pair_j(int p) {
-  return (int)((S == kHalf ? 0x10212010ull
+  return (int)((S == kHalf ? 0x12021302010ull
                            : (S == 5 ? 0x12012301234010ull : (S == 4 ? 0x0120123010ull : 0x12010ull))) >>
                (4 * p)) &
          15;
@@ -423,24 +438,35 @@ __device__ __forceinline__ void slices(R x, float* s) {
 // x rounded to a multiple of 2^e for |x| < 2^(e + 21), by adding and taking
 // off c = 1.5 2^(23 + e).
 __device__ __forceinline__ float round_grid(float x, float c) { return __fadd_rn(__fadd_rn(x, c), -c); }
-// The fp16 slices of x 2^kHalfUp (|x| < 1): s0 on the grid of c0, s1 on a grid
-// 2^-12 of it, s2 the rest (rounded to fp16's 11 bits when it is stored).
-// Exact but for that last rounding; |s1| is half a grid step of s0 (11 bits).
+// v rounded to fp16's 11 bits.
+__device__ __forceinline__ float round_half(float v) { return __half2float(__float2half_rn(v)); }
+// The fp16 slices of x 2^kHalfUp (|x| < 1): s0 on the grid of c0, s1 on the
+// grid of c1, s2 the remainder rounded to 11 bits, s3 the rest of that (rounded to
+// 11 bits, or multiples of 2^-24, when it is stored).  Exact but for that last
+// rounding; |s1| and |s2| are at most half a step of the slice before.
 __device__ __forceinline__ void half_slices(float x, float c0, float c1, float* s) {
   s[0] = round_grid(x, c0);
-  const float r = x - s[0];
+  float r = x - s[0];
   s[1] = round_grid(r, c1);
-  s[2] = r - s[1];
+  r -= s[1];
+  s[2] = round_half(r);
+  s[3] = r - s[2];
 }
 __device__ __forceinline__ void half_slices(double x, float c0, float c1, float* s) {
   s[0] = round_grid((float)x, c0);
-  const double r = x - (double)s[0];
+  double r = x - (double)s[0];
   s[1] = round_grid((float)r, c1);
-  s[2] = (float)(r - (double)s[1]);
+  r -= (double)s[1];
+  s[2] = round_half((float)r);
+  s[3] = (float)(r - (double)s[2]);
 }
-// The rounding constants of the first two slices for a first slice of `bits`.
-__device__ __forceinline__ float half_c0(int bits) { return 1.5f * __int_as_float((23 + kHalfUp - bits + 127) << 23); }
-__device__ __forceinline__ float half_c1(int bits) { return half_c0(bits) * (1.f / 4096.f); }
+// The rounding constants of the first two slices of rows (side 0) or columns.
+__device__ __forceinline__ float half_c0(int64_t k, int side) {
+  return 1.5f * __int_as_float((23 + kHalfUp - first_bits(k, side) + 127) << 23);
+}
+__device__ __forceinline__ float half_c1(int64_t k, int side) {
+  return half_c0(k, side) * __int_as_float((127 - second_bits(k)) << 23);
+}
 // A slice as the 16-bit operand value (exact, kHalf's last slice rounded).
 template <int S>
 __device__ __forceinline__ uint16_t slice_bits(float v) {
@@ -497,7 +523,7 @@ __global__ void __launch_bounds__(256) k_oz_pack(const T* __restrict__ X, uint16
   const int64_t zo = decode(z, d.nz, d.zdim, zstr);
   using R = typename Real<T>::R;
   uint16_t* tile = planes + (((z * rtiles + rt) * ktiles + kt) * Sl<S>::planes) * (int64_t)TILE;
-  const float c0 = half_c0(first_bits(d.K, side)), c1 = half_c1(first_bits(d.K, side));
+  const float c0 = half_c0(d.K, side), c1 = half_c1(d.K, side);
   for (int o = part * PER + threadIdx.x; o < (part + 1) * PER; o += blockDim.x) {
     // o = ((kc * GROUPS + g) * 8 + r8) * 8 + k8: core matrix (kc, g), row r8, K k8
     const int core = o >> 6, within = o & 63;
@@ -547,10 +573,13 @@ struct alignas(16) ParkCol {
 
 template <int TN, int S, bool PARK>
 struct alignas(1024) OzSmem {
-  unsigned char stage[OzCfg<TN, S, PARK>::stages][OzCfg<TN, S, PARK>::stage_bytes];  // A stacks, then B planes
+  unsigned char a[OzCfg<TN, S, PARK>::a_stages][OzCfg<TN, S, PARK>::a_bytes];  // ring of A stacks
+  unsigned char b[OzCfg<TN, S, PARK>::b_stages][OzCfg<TN, S, PARK>::b_bytes];  // ring of B planes
   int64_t koff[kMaxK];                                                        // A's K offsets
-  uint64_t full[OzCfg<TN, S, PARK>::stages];
-  uint64_t empty[OzCfg<TN, S, PARK>::stages];
+  uint64_t full_a[OzCfg<TN, S, PARK>::a_stages];
+  uint64_t empty_a[OzCfg<TN, S, PARK>::a_stages];
+  uint64_t full_b[OzCfg<TN, S, PARK>::one_ring ? 1 : OzCfg<TN, S, PARK>::b_stages];
+  uint64_t empty_b[OzCfg<TN, S, PARK>::one_ring ? 1 : OzCfg<TN, S, PARK>::b_stages];
   uint64_t accf[2];  // accumulator set b holds a finished tile
   uint64_t acce[2];  // the epilogue has read accumulator set b
   uint64_t drain;
@@ -643,7 +672,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   constexpr bool kPark = oz_park<TC, TN, S>();
   using CF = OzCfg<TN, S, kPark>;
   constexpr int kSlices = Sl<S>::n, kPlanes = Sl<S>::planes, kPairs = Sl<S>::pairs;
-  constexpr int kStages = CF::stages;
+  constexpr int kAStages = CF::a_stages, kBStages = CF::b_stages;
   constexpr uint32_t kTmemCols = CF::tmem_cols;
   constexpr int kSets = CF::acc_sets;
   constexpr int kConvWarps = conv_warps<TA, TN, S>(), kEpiWarps = kWorkWarps - kConvWarps;
@@ -653,13 +682,20 @@ __global__ void __launch_bounds__(kThreads, 1)
   OzSmem<TN, S, kPark>& sm = *reinterpret_cast<OzSmem<TN, S, kPark>*>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t ntot = ntiles * mtiles * d.Z;
+  uint64_t* const full_b = CF::one_ring ? sm.full_a : sm.full_b;
+  uint64_t* const empty_b = CF::one_ring ? sm.empty_a : sm.empty_b;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      // producer's expect_tx + one arrival per warp of the converter group of the K tile
-      mbar_init(&sm.full[s], 1 + kGroupThreads / 32);
-      mbar_init(&sm.empty[s], 1);
+    for (int s = 0; s < kAStages; ++s) {
+      // one arrival per warp of the converter group of the K tile (and the producer's)
+      mbar_init(&sm.full_a[s], kGroupThreads / 32 + (CF::one_ring ? 1 : 0));
+      mbar_init(&sm.empty_a[s], 1);
     }
+    if constexpr (!CF::one_ring)
+      for (int s = 0; s < kBStages; ++s) {
+        mbar_init(&sm.full_b[s], 1);  // the producer's expect_tx
+        mbar_init(&sm.empty_b[s], 1);
+      }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sm.accf[b], 1);
       mbar_init(&sm.acce[b], kEpiWarps);  // one arrival per epilogue warp
@@ -682,21 +718,20 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int64_t nt = tile % ntiles, z = tile / (ntiles * mtiles);
         const uint16_t* btile = pb + ((z * ntiles + nt) * ktiles) * (int64_t)(kPlanes * CF::kBTile);
         for (int64_t kt = 0; kt < ktiles; ++kt, ++g) {
-          const int s = (int)(g % kStages);
-          const uint32_t ph = (uint32_t)((g / kStages) & 1);
-          if (!mbar_wait(&sm.empty[s], ph ^ 1)) {
+          const int s = (int)(g % kBStages);
+          const uint32_t ph = (uint32_t)((g / kBStages) & 1);
+          if (!mbar_wait(&empty_b[s], ph ^ 1)) {
             ok = false;
             break;
           }
-          mbar_expect_tx(&sm.full[s], CF::b_bytes);
-          bulk_g2s(sm.stage[s] + kSlices * kStackBytes, btile + kt * (kPlanes * CF::kBTile), CF::b_bytes,
-                   &sm.full[s]);
+          mbar_expect_tx(&full_b[s], CF::b_bytes);
+          bulk_g2s(sm.b[s], btile + kt * (kPlanes * CF::kBTile), CF::b_bytes, &full_b[s]);
         }
       }
       // the copies of the last stages are in flight until their full barrier
       // completes: wait (bounded) so none lands after the CTA has exited
-      for (int64_t i = g - 1; i >= 0 && i >= g - kStages; --i)
-        if (!mbar_wait(&sm.full[i % kStages], (uint32_t)((i / kStages) & 1))) ok = false;
+      for (int64_t i = g - 1; i >= 0 && i >= g - kBStages; --i)
+        if (!mbar_wait(&full_b[i % kBStages], (uint32_t)((i / kBStages) & 1))) ok = false;
     }
   } else if (warp == 1) {
     // The whole warp runs the loop and waits, and one elected thread issues a
@@ -706,58 +741,73 @@ __global__ void __launch_bounds__(kThreads, 1)
     // (69 with this form).
     constexpr uint32_t idesc = idesc_f16(Sl<S>::half, 128, TN), idesc_neg = idesc_f16(Sl<S>::half, 128, TN, true);
     constexpr uint32_t ALBO = 24 * 128, BLBO = (TN / 8) * 128, SBO = 128;
-    int s = 0;       // ring stage and its phase
-    uint32_t ph = 0;
+    // positions in the rings of A and B, with their phases
+    struct Pos {
+      int a = 0, b = 0;
+      uint32_t pa = 0, pb = 0;
+    } at;
+    auto filled = [&](const Pos& p) {
+      return __all_sync(0xffffffffu, mbar_wait(&sm.full_a[p.a], p.pa) &&
+                                         (CF::one_ring || mbar_wait(&full_b[p.b], p.pb)));
+    };
+    auto advance = [&](Pos& p) {
+      next_stage<kAStages>(p.a, p.pa);
+      next_stage<kBStages>(p.b, p.pb);
+    };
+    // both stages are free once the MMAs issued so far have finished
+    auto release = [&](const Pos& p) {
+      mma_commit(&sm.empty_a[p.a]);
+      if constexpr (!CF::one_ring) mma_commit(&empty_b[p.b]);
+    };
     int64_t t = 0;   // tiles of this CTA
-    // The MMAs of the K tile in stage `st`, levels lo .. hi (2: the rest).
-    // kHalf: the MMAs of one A operand follow each other: the first fills the
-    // tensor core's A buffer from shared memory, the others use it (an M = N =
-    // 128 MMA reads 8 KB in its 64 cycles, all of the SM's shared-memory
-    // bandwidth; with A kept, kHalf reads 88 KB per K tile instead of 128 KB: 7 %
-    // of the wide pair's time).  bf16 slices: level by level (pair_i).  `first`
+    // The MMAs of the K tile at `p`, levels lo .. hi (2: the rest).  kHalf: the
+    // MMAs of one A operand follow each other, the last slices first: the first
+    // MMA fills the tensor core's A buffer from shared memory, the others use it
+    // (an M = N = 128 MMA reads 8 KB in its 64 cycles, all of the SM's
+    // shared-memory bandwidth).  bf16 slices: level by level (pair_i).  `first`
     // overwrites the levels; l2 is the column of level 2.
-    auto issue = [&](int st, int lo, int hi, bool first, uint32_t set, uint32_t l2) {
-      const uint32_t sa = smem_u32(sm.stage[st]) >> 4;
-      constexpr uint32_t BOFF = (kSlices * kStackBytes) >> 4;
-      if constexpr (!Sl<S>::half) {
+    auto issue = [&](const Pos& p, int lo, int hi, bool first, uint32_t set, uint32_t l2) {
+      const uint32_t sa = smem_u32(sm.a[p.a]) >> 4, sb = smem_u32(sm.b[p.b]) >> 4;
+      // part 0: [Ar; Ai] . Br = [Ar.Br ; Ai.Br]; part 1: [Ai; -Ar] with A
+      // negated . Bi = [-Ai.Bi ; Ar.Bi]
+      auto adesc = [&](int i, int part) { return desc_at(sa + ((i * kStackBytes + part * 8 * 128) >> 4), ALBO, SBO); };
+      auto bdesc = [&](int j, int part) {
+        return desc_at(sb + (((part * kSlices + j) * CF::kBTile * 2) >> 4), BLBO, SBO);
+      };
+      auto level = [&](int lv) { return tmem + (lv < 2 ? set + (uint32_t)(lv * TN) : l2); };
+      if constexpr (Sl<S>::half) {
+#pragma unroll
+        for (int i = kSlices - 1; i >= 0; --i) {
+#pragma unroll
+          for (int part = 0; part < 2; ++part) {
+            const uint64_t x = adesc(i, part);
+            const int j0 = i >= lo ? 0 : lo - i;  // B's slices j1 - 1 .. j0
+            const int j1 = hi < 2 && Sl<S>::met(i) > hi + 1 - i ? hi + 1 - i : Sl<S>::met(i);
+#pragma unroll
+            for (int j = Sl<S>::met(0) - 1; j >= 0; --j) {
+              if (j < j0 || j >= j1) continue;
+              // the first MMA into each level, pairs (0,0), (1,0) and (3,0), overwrites it
+              const uint32_t acc = (first && part == 0 && j == 0 && i != 2) ? 0u : 1u;
+              const uint32_t dl = level(i + j);
+              const uint64_t y = bdesc(j, part);
+              const uint32_t id = part ? idesc_neg : idesc;
+              if (j == j1 - 1)
+                mma_f16_a_fill(dl, x, y, id, acc);
+              else if (j > j0)
+                mma_f16_a_use(dl, x, y, id, acc);
+              else
+                mma_f16_a_lastuse(dl, x, y, id, acc);
+            }
+          }
+        }
+      } else {
 #pragma unroll
         for (int q = 0; q < kPairs; ++q) {
           const int i = pair_i<S>(q), j = pair_j<S>(q), lv = i + j < 2 ? i + j : 2;
           if (lv < lo || lv > hi) continue;
-          const uint32_t dl = tmem + (lv < 2 ? set + (uint32_t)(lv * TN) : l2);
-#pragma unroll
-          for (int part = 0; part < 2; ++part)  // the first pair of each level overwrites it
-            mma_f16(dl, desc_at(sa + ((i * kStackBytes + part * 8 * 128) >> 4), ALBO, SBO),
-                    desc_at(sa + BOFF + (((part * kSlices + j) * CF::kBTile * 2) >> 4), BLBO, SBO),
-                    part ? idesc_neg : idesc, first && part == 0 && (q < 2 || q == 3) ? 0u : 1u);
-        }
-        return;
-      }
-#pragma unroll
-      for (int i = 0; i < kSlices; ++i) {
-#pragma unroll
-        for (int part = 0; part < 2; ++part) {
-          // part 0: [Ar; Ai] . Br = [Ar.Br ; Ai.Br]; part 1: [Ai; -Ar]
-          // with A negated . Bi = [-Ai.Bi ; Ar.Bi]
-          const uint64_t x = desc_at(sa + ((i * kStackBytes + part * 8 * 128) >> 4), ALBO, SBO);
-          const int j0 = i >= lo ? 0 : lo - i;                              // first slice of B
-          const int j1 = hi < 2 && Sl<S>::met(i) > hi + 1 - i ? hi + 1 - i : Sl<S>::met(i);  // past the last
-#pragma unroll
-          for (int j = 0; j < Sl<S>::met(0); ++j) {
-            if (j < j0 || j >= j1) continue;
-            const int lv = i + j < 2 ? i + j : 2;
-            // the first MMA into each level overwrites it
-            const uint32_t acc = (first && i == 0 && part == 0 && j <= 2) ? 0u : 1u;
-            const uint32_t dl = tmem + (lv < 2 ? set + (uint32_t)(lv * TN) : l2);
-            const uint64_t y = desc_at(sa + BOFF + (((part * kSlices + j) * CF::kBTile * 2) >> 4), BLBO, SBO);
-            const uint32_t id = part ? idesc_neg : idesc;
-            if (j == j0)
-              mma_f16_a_fill(dl, x, y, id, acc);
-            else if (j + 1 < j1)
-              mma_f16_a_use(dl, x, y, id, acc);
-            else
-              mma_f16_a_lastuse(dl, x, y, id, acc);
-          }
+          // the first pair of each level overwrites it
+          mma_f16(level(lv), adesc(i, 0), bdesc(j, 0), idesc, first && (q < 2 || q == 3) ? 0u : 1u);
+          mma_f16(level(lv), adesc(i, 1), bdesc(j, 1), idesc_neg, 1u);
         }
       }
     };
@@ -766,18 +816,18 @@ __global__ void __launch_bounds__(kThreads, 1)
       int kt0 = 0;  // K tiles whose MMAs are all issued
       if constexpr (kPark) {
         // Level 2 alternates between TMEM blocks 2 and 3, so the first K tiles'
-        // level-2 MMAs (10 of 16) do not wait for the epilogue of the tile
+        // level-2 MMAs (16 of 22) do not wait for the epilogue of the tile
         // before; their level 0 and 1 MMAs follow once it has read its sums.
         const uint32_t l2 = (uint32_t)((2 + (t & 1)) * TN);
-        const int pre = (int)ktiles < kStages ? (int)ktiles : kStages;
-        int s1 = s;
-        uint32_t ph1 = ph;
+        static_assert(kAStages <= kBStages, "K tiles issued ahead");
+        const int pre = (int)ktiles < kAStages ? (int)ktiles : kAStages;
+        Pos ahead = at;
         for (int kt = 0; kt < pre && ok; ++kt) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&sm.full[s1], ph1))) ok = false;
+          if (!filled(ahead)) ok = false;
           fence_after();
-          if (ok && elect_one()) issue(s1, 2, 2, kt == 0, 0, l2);
+          if (ok && elect_one()) issue(ahead, 2, 2, kt == 0, 0, l2);
           __syncwarp();
-          next_stage<kStages>(s1, ph1);
+          advance(ahead);
         }
         if (!ok || !__all_sync(0xffffffffu, mbar_wait(&sm.acce[b], (uint32_t)((t & 1) ^ 1)))) {
           ok = false;
@@ -786,11 +836,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         fence_after();
         for (int kt = 0; kt < pre; ++kt) {
           if (elect_one()) {
-            issue(s, 0, 1, kt == 0, 0, l2);
-            mma_commit(&sm.empty[s]);  // smem stage free once these MMAs finish
+            issue(at, 0, 1, kt == 0, 0, l2);
+            release(at);
           }
           __syncwarp();
-          next_stage<kStages>(s, ph);
+          advance(at);
         }
         kt0 = pre;
       } else {
@@ -802,14 +852,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         fence_after();
       }
       for (int kt = kt0; kt < (int)ktiles; ++kt) {
-        if (!__all_sync(0xffffffffu, mbar_wait(&sm.full[s], ph))) {
+        if (!filled(at)) {
           ok = false;
           break;
         }
         fence_after();
         if constexpr (CF::narrow) {
-          const uint32_t sa = smem_u32(sm.stage[s]) >> 4;
-          constexpr uint32_t BOFF = (kSlices * kStackBytes) >> 4;
+          const uint32_t sa = smem_u32(sm.a[at.a]) >> 4, sb = smem_u32(sm.b[at.b]) >> 4;
           // B block per part: the slices x 2 row groups per K half
           constexpr uint32_t NLBO = kSlices * 2 * 128;
           if (elect_one()) {
@@ -818,26 +867,27 @@ __global__ void __launch_bounds__(kThreads, 1)
               const uint32_t dl = tmem + (uint32_t)(b * CF::set_cols + narrow_col<S>(i));
               const uint64_t x1 = desc_at(sa + ((i * kStackBytes) >> 4), ALBO, SBO);            // [Ar; Ai]
               const uint64_t x2 = desc_at(sa + ((i * kStackBytes + 8 * 128) >> 4), ALBO, SBO);  // [Ai; -Ar]
-              const uint64_t br = desc_at(sa + BOFF, NLBO, SBO);
-              const uint64_t bi = desc_at(sa + BOFF + ((kSlices * CF::kBTile * 2) >> 4), NLBO, SBO);
+              const uint64_t br = desc_at(sb, NLBO, SBO);
+              const uint64_t bi = desc_at(sb + ((kSlices * CF::kBTile * 2) >> 4), NLBO, SBO);
               // [Ar.Br ; Ai.Br], then [-Ai.Bi ; Ar.Bi], slices 0 .. met(i)-1 of B
               mma_f16(dl, x1, br, idesc_f16(Sl<S>::half, 128, 16 * Sl<S>::met(i)), kt == 0 ? 0u : 1u);
               mma_f16(dl, x2, bi, idesc_f16(Sl<S>::half, 128, 16 * Sl<S>::met(i), true), 1u);
             }
-            mma_commit(&sm.empty[s]);
+            release(at);
           }
-          next_stage<kStages>(s, ph);
+          __syncwarp();
+          advance(at);
           continue;
         }
         if (elect_one()) {
           if constexpr (kPark)
-            issue(s, 0, 2, false, 0, (uint32_t)((2 + (t & 1)) * TN));
+            issue(at, 0, 2, false, 0, (uint32_t)((2 + (t & 1)) * TN));
           else
-            issue(s, 0, 2, kt == 0, (uint32_t)(b * 3 * TN), (uint32_t)((b * 3 + 2) * TN));
-          mma_commit(&sm.empty[s]);  // smem stage free once these MMAs finish
+            issue(at, 0, 2, kt == 0, (uint32_t)(b * 3 * TN), (uint32_t)((b * 3 + 2) * TN));
+          release(at);
         }
         __syncwarp();
-        next_stage<kStages>(s, ph);
+        advance(at);
       }
       if (!ok) break;
       if (elect_one()) mma_commit(&sm.accf[b]);  // tile accumulators ready for the epilogue
@@ -853,14 +903,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     // core-matrix row per stack block, stored without bank conflicts;
     // complex128 A: NV = 4 (half rows; fewer registers), one group.
     constexpr int NV = conv_values<TA>(), GT = kGroupThreads, H = 32 * kConvWarps / GT;
-    static_assert(H <= kStages, "ring");
+    static_assert(H <= kAStages, "ring");
     const int c = threadIdx.x - 64;
     const int grp = c / GT, ch = c % GT;
     const int r = ch & (kRows - 1), kq = (ch >> 6) * NV;
     using R = typename Real<TA>::R;
     // byte offset of (slice 0, block 0, row r, K value kq) in the stacks
     const uint32_t row_off = (uint32_t)((((kq >> 3) * 24 + (r >> 3)) * 8 + (r & 7)) * 16 + (kq & 7) * 2);
-    const float hc0 = half_c0(first_bits(d.K, 0)), hc1 = half_c1(first_bits(d.K, 0));
+    const float hc0 = half_c0(d.K, 0), hc1 = half_c1(d.K, 0);
     // This CTA's K tiles form one sequence g = tile number * ktiles + kt; the
     // group takes g = grp, grp + H, ...  The next one's A values and row
     // exponent are loaded while this one is sliced, across tile boundaries
@@ -941,7 +991,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int up = Sl<S>::half ? kHalfUp : 0;
       const float2 f = inv_scale((e != kExpZero ? e : 0) - up);
       {
-        uint32_t pr[kSlices][NV / 2], pim[kSlices][NV / 2];  // bf16 pairs (k, k + 1) of Ar, Ai
+        uint32_t pr[kSlices][NV / 2], pim[kSlices][NV / 2];  // 16-bit pairs (k, k + 1) of Ar, Ai
 #pragma unroll
         for (int q = 0; q < NV; q += 2) {
           float a0[kSlices], b0[kSlices], a1[kSlices], b1[kSlices];
@@ -962,13 +1012,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             pim[i][q / 2] = pack_x2<S>(b0[i], b1[i]);
           }
         }
-        bool got = mbar_wait(&sm.empty[s], ph ^ 1);
+        bool got = mbar_wait(&sm.empty_a[s], ph ^ 1);
         got = __all_sync(0xffffffffu, got);
         if (!got) {
           ok = false;
           break;
         }
-        const uint32_t base = smem_u32(sm.stage[s]) + row_off;
+        const uint32_t base = smem_u32(sm.a[s]) + row_off;
 #pragma unroll
         for (int i = 0; i < kSlices; ++i) {
           const uint32_t slice = base + (uint32_t)(i * kStackBytes);
@@ -985,8 +1035,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.full[s]);
-        next_stage<kStages>(s, ph, H);
+        if (lane == 0) mbar_arrive(&sm.full_a[s]);
+        next_stage<kAStages>(s, ph, H);
       }
     }
   } else {
@@ -1402,14 +1452,17 @@ cudaError_t launch_oz(int slices, int ta, int tb, int tc, const void* A, const v
   const OzLayout L = layout(d, slices);
   if (!scratch || scratch_bytes < L.total) return cudaErrorInvalidValue;
   char* base = (char*)(((uintptr_t)scratch + 255) & ~(uintptr_t)255);
-  // Five slices stay for complex128 results, where the split's own error (about
-  // 2^-34 of the scales) is what the caller sees; in a complex64 result it is
-  // far below the 2^-25 of the storage rounding with either split, and kHalf
-  // takes 8 slice products instead of 15.
+  // Complex64 results up to K = kHalfMaxK take the fp16 split: no less exact than
+  // five bf16 slices (above), with 11 slice products instead of 15.  Past
+  // that its first slices would need 7 bits on both sides and the pairs (1,3) and
+  // (3,1) to drop no more than five slices do; complex128 results need the
+  // five slices' order of levels, whose rest is what their caller sees.
   const bool c128 = tc == PQ_C128;
-  if (slices == 5)
-    return c128 ? launch_oz_n<5, double2>(ta, tb, A, B, C, d, base, L, status, stream)
-                : launch_oz_n<kHalf, float2>(ta, tb, A, B, C, d, base, L, status, stream);
+  if (slices == 5) {
+    if (c128) return launch_oz_n<5, double2>(ta, tb, A, B, C, d, base, L, status, stream);
+    return d.K <= kHalfMaxK ? launch_oz_n<kHalf, float2>(ta, tb, A, B, C, d, base, L, status, stream)
+                            : launch_oz_n<5, float2>(ta, tb, A, B, C, d, base, L, status, stream);
+  }
   if (slices == 4)
     return c128 ? launch_oz_n<4, double2>(ta, tb, A, B, C, d, base, L, status, stream)
                 : launch_oz_n<4, float2>(ta, tb, A, B, C, d, base, L, status, stream);

@@ -638,3 +638,57 @@ def test_ozaki_bf16_small_products_first(pq, k, n):
         return np.sqrt(np.mean((np.abs(x - ref) / scale) ** 2))
 
     assert rms(got) <= 1.05 * rms(Z.accumulate(A, B, False))
+
+
+@pytest.mark.parametrize("k", [64, 128, 144, 256, 272, 512])
+@pytest.mark.parametrize("n", [128, 40, 16])
+def test_ozaki_cancelling_leading_level(pq, k, n):
+    """Rows whose leading slices cancel over K while the next ones add up
+    (+-0.75 alternating plus 0.95 2^-8, columns equal in pairs): level 1 is then
+    the result and has to be exact.  Either split, all tile widths, within the
+    scheme's bound (a second slice of 12 bits, whose level 1 does not fit, is at
+    ten times that for K = 512)."""
+    rng = np.random.default_rng(k + n)
+    m = max(1400, (1 << 21) // (k * n))
+    a = np.where(np.arange(k) % 2 == 0, 0.75, -0.75) + 0.95 * 2.0 ** -8
+    A = (np.tile(a, (m, 1)) * np.exp2(rng.integers(-20, 20, (m, 1)))).astype(np.complex64)
+    A[m // 2:] *= 1j
+    B = np.repeat(rng.uniform(0.9, 1.0, (k // 2, n)), 2, axis=0).astype(np.complex64)
+    be = ozaki_backend(pq)
+    got, nl = run(be, A, [-1, 1], B, [1, -2])
+    be.close()
+    assert nl == OZ_LAUNCHES
+    A, B = A.astype(np.complex128), B.astype(np.complex128)
+    ref = A @ B
+    assert np.all(np.abs(got - ref) <= ozaki_bound(A, B, ref))
+
+
+@pytest.mark.parametrize("k", [32, 128, 256])
+@pytest.mark.parametrize("n", [128, 40, 16])
+def test_ozaki_half_split_keeps_small_slices(pq, k, n):
+    """Results near 2^-20 of the scales (columns equal in pairs, rows that
+    nearly cancel over them), where the complex64 rounding hides nothing: the
+    rms error is that of the restated sums, with a factor of 2 for the adder's
+    own alignment.  Lost fp16 subnormals or a residual of 2^-33 (three slices)
+    would be 8 times that and more."""
+    from oracle import ozaki_oracle as Z
+
+    rng = np.random.default_rng(k + n)
+    m = max(1400, (1 << 21) // (k * n))
+    B = np.repeat(rng.uniform(0.5, 1, (k // 2, n)) * np.exp(2j * np.pi * rng.random((k // 2, n))), 2, axis=0)
+    a = rand(rng, (m, k // 2))
+    A = np.empty((m, k), dtype=np.complex128)
+    A[:, 0::2], A[:, 1::2] = a, -a + 1e-6 * rand(rng, a.shape)
+    A, B = A.astype(np.complex64), B.astype(np.complex64)
+    be = ozaki_backend(pq)
+    got, nl = run(be, A, [-1, 1], B, [1, -2])
+    be.close()
+    assert nl == OZ_LAUNCHES
+    A, B = A.astype(np.complex128)[:48], B.astype(np.complex128)
+    ref = A.astype(np.clongdouble) @ B.astype(np.clongdouble)
+    scale = np.exp2((Z.row_exponents(A)[:, None] + Z.row_exponents(B.T)[None, :]).astype(np.float64))
+
+    def rms(x):
+        return np.sqrt(np.mean((np.abs(x - ref) / scale) ** 2))
+
+    assert rms(got[:48].astype(np.clongdouble)) <= 2 * rms(Z.accumulate(A, B, True).astype(np.complex64))

@@ -130,7 +130,10 @@ __device__ __forceinline__ void sv_pass(float2* __restrict__ S, const ulonglong2
     // instead of being hoisted into registers
 #pragma unroll 1
     for (int c0 = 0; c0 < D; c0 += 2 * G) {
-      F2 rr[G], ii[G], ri[G];  // sums of re re, im im and re im + im re
+      // sums of re re, im im and re im + im re; up to two qubits re re - im im is
+      // one chain, as for the skinny pairs: with so few terms the rounding of
+      // a subtraction at the end would count
+      F2 rr[G], ii[G], ri[G];
 #pragma unroll
       for (int q = 0; q < G; ++q) rr[q] = ii[q] = ri[q] = 0;
 #pragma unroll
@@ -139,7 +142,10 @@ __device__ __forceinline__ void sv_pass(float2* __restrict__ S, const ulonglong2
         for (int q = 0; q < G; ++q) {
           const ulonglong2 u = U[ci * (D / 2) + c0 / 2 + q];
           rr[q] = f2_fma(ax[ci], u.x, rr[q]);
-          ii[q] = f2_fma(ay[ci], u.y, ii[q]);
+          if constexpr (D <= 4)
+            rr[q] = f2_fma(ay[ci] ^ 0x8000000080000000ull, u.y, rr[q]);
+          else
+            ii[q] = f2_fma(ay[ci], u.y, ii[q]);
           ri[q] = f2_fma(ax[ci], u.y, ri[q]);
           ri[q] = f2_fma(ay[ci], u.x, ri[q]);
         }

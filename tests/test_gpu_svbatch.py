@@ -123,3 +123,43 @@ def test_svbatch_block_positions(pq, n, qs):
     be.close()
     tol = 2.0 ** -24 * (2 * (len(qs) ** 2 + 2 ** len(qs) + 2) + 8 * n)
     assert np.linalg.norm(got - psi.reshape(-1)) <= tol
+
+
+@pytest.mark.parametrize("n,qs", [(3, [2]), (6, [1, 2]), (7, [1, 5]), (8, [3, 7])])
+def test_svbatch_small_blocks_are_one_chain(pq, n, qs):
+    """Blocks of one and two qubits add each output's real part up in one chain
+    of fused multiply-adds (a subtraction of two sums would round once more):
+    equal to that chain in FP32, bit for bit."""
+    from pqgb300.svbatch import StateVectorBatch
+
+    def fma(a, b, c):
+        return (np.asarray(a, np.longdouble) * np.longdouble(b) + np.asarray(c, np.longdouble)).astype(np.float32)
+
+    rng = np.random.default_rng(n + sum(qs))
+
+    def haar(d):
+        q, r = np.linalg.qr(rng.standard_normal((d, d)) + 1j * rng.standard_normal((d, d)))
+        return q * (np.diag(r) / np.abs(np.diag(r)))
+
+    blocks = [(haar(2), [q]) for q in range(1, n + 1)] + [(haar(1 << len(qs)), qs), (haar(2), [n])]
+    re, im = np.zeros(1 << n, np.float32), np.zeros(1 << n, np.float32)
+    re[0] = 1
+    index = np.arange(1 << n)
+    for U, b in blocks:
+        mask = sum(1 << (q - 1) for q in b)
+        base = index[(index & mask) == 0]
+        at = [base + sum(((c >> i) & 1) << (q - 1) for i, q in enumerate(b)) for c in range(1 << len(b))]
+        x, y = [re[a] for a in at], [im[a] for a in at]
+        for o, a in enumerate(at):
+            sr, si = np.float32(0), np.float32(0)
+            for c in range(1 << len(b)):
+                ux, uy = np.float32(U[o, c].real), np.float32(U[o, c].imag)
+                sr = fma(-y[c], uy, fma(x[c], ux, sr))
+                si = fma(y[c], ux, fma(x[c], uy, si))
+            re[a], im[a] = sr, si
+    be = pq.GB300Backend(pq.PREC_C64)
+    sb = StateVectorBatch(be, [(n, blocks, [format(i, f"0{n}b")[::-1] for i in range(1 << n)])])
+    got = sb.execute()[0]
+    sb.close()
+    be.close()
+    assert np.array_equal(got.real, re) and np.array_equal(got.imag, im)

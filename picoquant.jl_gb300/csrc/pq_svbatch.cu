@@ -168,9 +168,24 @@ __global__ void __launch_bounds__(kSvThreads, 6)
   __shared__ __align__(16) float U[kSvMaxDim * kSvMaxDim / 2][4];
   __shared__ SvOp s_op;
   __shared__ int64_t s_blk[2];
+  __shared__ int s_lo;
   // the entry owning this block: the one with blk[entry] <= blockIdx.x <
-  // blk[entry + 1], looked at by all threads at once
-  for (int t = threadIdx.x; t < nops; t += blockDim.x) {
+  // blk[entry + 1].  All threads look at one entry each; a longer table is first
+  // narrowed to the run of entries between two of 128 probes (one round to
+  // 2^14 entries): blocks are at least as many as entries, so a scan of the
+  // whole table by each would make a launch quadratic in the circuits.
+  int lo = 0, n = nops;
+  while (n > kSvThreads) {
+    const int run = (n + kSvThreads - 1) / kSvThreads;
+    const int t0 = lo + threadIdx.x * run, t1 = min(t0 + run, lo + n);
+    if (t0 < lo + n && blk[t0] <= (int64_t)blockIdx.x && (int64_t)blockIdx.x < blk[t1]) s_lo = t0;
+    __syncthreads();
+    n = min(run, lo + n - s_lo);
+    lo = s_lo;
+    __syncthreads();
+  }
+  if ((int)threadIdx.x < n) {
+    const int t = lo + threadIdx.x;
     const int64_t b0 = blk[t], b1 = blk[t + 1];
     if (b0 <= (int64_t)blockIdx.x && (int64_t)blockIdx.x < b1) {
       s_op = ops[t];

@@ -163,3 +163,23 @@ def test_svbatch_small_blocks_are_one_chain(pq, n, qs):
     sb.close()
     be.close()
     assert np.array_equal(got.real, re) and np.array_equal(got.imag, im)
+
+
+@pytest.mark.parametrize("count", [127, 128, 129, 16384, 16385, 20000])
+def test_svbatch_many_small_circuits(pq, count):
+    """Launch tables around 128 entries (one look by 128 threads) and 128^2 (two
+    rounds of narrowing): circuits of one and two qubits, each with a rotation
+    of its own, so that a block working on another's entry shows."""
+    from pqgb300.svbatch import StateVectorBatch
+
+    angle = np.random.default_rng(count).uniform(0, np.pi, count)
+    circs = []
+    for i, a in enumerate(angle):
+        R = np.array([[np.cos(a), -np.sin(a)], [np.sin(a), np.cos(a)]])
+        circs.append((1 + i % 2, [(R, [1 + i % 2])], ["01" if i % 2 else "1"]))
+    be = pq.GB300Backend(pq.PREC_C64)
+    sb = StateVectorBatch(be, circs)
+    got = np.concatenate(sb.execute())
+    sb.close()
+    be.close()
+    assert np.array_equal(got, np.sin(angle).astype(np.float32).astype(np.complex128))

@@ -293,12 +293,13 @@ struct pq_mlp {
   float* d_v = nullptr;
   int64_t step = 0;
   // workspace for a batch
-  int cap = 0;
+  int cap = 0;       // rows that the activations hold
+  int grad_cap = 0;  // rows that the gradient workspace holds
   std::vector<float*> act;  // act[0] = input, act[l+1] = output of layer l
   std::vector<float*> dact;
   float* d_t = nullptr;
   float* d_loss = nullptr;
-  float* d_part = nullptr;       // weight-gradient chunks (chunks(cap) x n_params)
+  float* d_part = nullptr;       // weight-gradient chunks (at most max_chunks x n_params)
   float* d_loss_part = nullptr;  // squared errors per k_head block
   __nv_bfloat16* d_wbf = nullptr;
   __nv_bfloat16* d_xb[2] = {nullptr, nullptr};
@@ -306,10 +307,17 @@ struct pq_mlp {
 
 namespace {
 
-// The batch in chunks of rows for the weight gradients: 128 rows each, and at
-// most 64 chunks.
-int chunk_rows(int n) { return std::max(128, ((n + 63) / 64 + GT - 1) / GT * GT); }
-int chunk_count(int n) { return (n + chunk_rows(n) - 1) / chunk_rows(n); }
+// The batch in chunks of rows for the weight gradients: 128 rows each, at most
+// 64 chunks and kPartBytes of partial gradients (a model whose gradients are
+// large has tiles for every SM without chunks).
+constexpr int64_t kPartBytes = 64 << 20;
+int max_chunks(int64_t n_params) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(64, kPartBytes / (n_params * (int64_t)sizeof(float))));
+}
+int chunk_rows(int n, int64_t n_params) {
+  const int c = max_chunks(n_params);
+  return std::max(128, ((n + c - 1) / c + GT - 1) / GT * GT);
+}
 
 void free_ws(pq_mlp* m) {
   for (auto p : m->act) cudaFree(p);
@@ -317,13 +325,17 @@ void free_ws(pq_mlp* m) {
   m->act.clear();
   m->dact.clear();
   cudaFree(m->d_t);
-  cudaFree(m->d_part);
-  cudaFree(m->d_loss_part);
   cudaFree(m->d_xb[0]);
   cudaFree(m->d_xb[1]);
-  m->d_t = m->d_part = m->d_loss_part = nullptr;
+  m->d_t = nullptr;
   m->d_xb[0] = m->d_xb[1] = nullptr;
   m->cap = 0;
+}
+void free_grad_ws(pq_mlp* m) {
+  cudaFree(m->d_part);
+  cudaFree(m->d_loss_part);
+  m->d_part = m->d_loss_part = nullptr;
+  m->grad_cap = 0;
 }
 
 int ensure_ws(pq_mlp* m, int n) {
@@ -340,10 +352,6 @@ int ensure_ws(pq_mlp* m, int n) {
   }
   int wmax = std::max(m->n_in, m->hidden);
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_t, sizeof(float) * (size_t)n);
-  // (a smaller batch has no more chunks than this one)
-  if (e == cudaSuccess)
-    e = cudaMalloc((void**)&m->d_part, sizeof(float) * (size_t)m->n_params * (size_t)std::min(64, (n + 127) / 128));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_loss_part, sizeof(float) * (size_t)((n + 7) / 8));
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_xb[0], sizeof(__nv_bfloat16) * (size_t)n * wmax);
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_xb[1], sizeof(__nv_bfloat16) * (size_t)n * wmax);
   if (e != cudaSuccess) {
@@ -351,6 +359,21 @@ int ensure_ws(pq_mlp* m, int n) {
     return cuda_fail(m->ctx, e, "mlp workspace");
   }
   m->cap = n;
+  return PQ_OK;
+}
+// What gradients of n rows need beside the activations (inference does not).
+int ensure_grad_ws(pq_mlp* m, int n) {
+  if (n <= m->grad_cap) return PQ_OK;
+  free_grad_ws(m);
+  // (a smaller batch has no more chunks than this)
+  const size_t chunks = (size_t)std::min(max_chunks(m->n_params), (n + 127) / 128);
+  cudaError_t e = cudaMalloc((void**)&m->d_part, sizeof(float) * (size_t)m->n_params * chunks);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_loss_part, sizeof(float) * (size_t)((n + 7) / 8));
+  if (e != cudaSuccess) {
+    free_grad_ws(m);
+    return cuda_fail(m->ctx, e, "mlp gradient workspace");
+  }
+  m->grad_cap = n;
   return PQ_OK;
 }
 
@@ -380,7 +403,7 @@ void backward(pq_mlp* m, int n) {
     k_layer<true><<<grid, 256, 0, s>>>(m->dact[l + 1], m->d_p + m->woff[l], nullptr, m->act[l], m->dact[l], n,
                                        m->din[l], m->dout[l]);
   }
-  const int chunks = chunk_count(n);
+  const int rows = chunk_rows(n, m->n_params), chunks = (n + rows - 1) / rows;
   for (int l0 = 0; l0 < L; l0 += kDwLayers) {
     DwTable d;
     d.layers = std::min(kDwLayers, L - l0);
@@ -395,7 +418,7 @@ void backward(pq_mlp* m, int n) {
       d.dy[i] = m->dact[l + 1];
       d.first[i + 1] = d.first[i] + ((d.M[i] + GT - 1) / GT) * ((d.N[i] + GT - 1) / GT);
     }
-    k_dw<<<dim3(d.first[d.layers], chunks), 256, 0, s>>>(d, n, chunk_rows(n), m->n_params, m->d_part);
+    k_dw<<<dim3(d.first[d.layers], chunks), 256, 0, s>>>(d, n, rows, m->n_params, m->d_part);
   }
   k_reduce_parts<<<(unsigned)((m->n_params + 255) / 256) + 1, 256, 0, s>>>(m->d_part, chunks, m->n_params, m->d_g,
                                                                          m->d_loss_part, (n + 7) / 8, n, m->d_loss);
@@ -461,6 +484,7 @@ int pq_mlp_destroy(pq_mlp* m) {
   if (!m) return PQ_ERR_INVALID;
   cudaStreamSynchronize(m->ctx->stream);
   free_ws(m);
+  free_grad_ws(m);
   cudaFree(m->d_p);
   cudaFree(m->d_g);
   cudaFree(m->d_m);
@@ -496,6 +520,7 @@ int pq_mlp_set_params(pq_mlp* m, const float* w, int64_t n) {
 int pq_mlp_gradients(pq_mlp* m, const float* X, const float* y, int64_t n, float* grad, float* loss) {
   if (!m || !X || !y || !grad || n < 1 || n > (1 << 24)) return PQ_ERR_INVALID;
   int st = ensure_ws(m, (int)n);
+  if (!st) st = ensure_grad_ws(m, (int)n);
   if (st) return st;
   cudaStream_t s = m->ctx->stream;
   cudaMemcpyAsync(m->act[0], X, sizeof(float) * n * m->n_in, cudaMemcpyHostToDevice, s);
@@ -532,6 +557,7 @@ int pq_mlp_train(pq_mlp* m, const float* X, const float* y, int64_t n, int epoch
   cudaMemcpyAsync(dY, y, sizeof(float) * n, cudaMemcpyHostToDevice, s);
   const int b = (int)std::min<int64_t>(batch, n);
   int st = ensure_ws(m, b);
+  if (!st) st = ensure_grad_ws(m, b);
   if (st) {
     cudaFree(dX);
     cudaFree(dY);

@@ -213,3 +213,44 @@ def test_mlp_gradients_shapes(pq, be, n, hidden, layers):
     assert abs(loss - lo) <= 1e-5 * max(1.0, abs(lo))
     assert np.max(np.abs(g - go)) <= 1.6e-4 * max(1.0, np.max(np.abs(go)))
     m.close()
+
+
+def test_mlp_workspace_of_large_models(pq, be):
+    """Inference takes no gradient workspace and gradients take a bounded one:
+    with 3 x 1024 hidden units and 8192 rows the activations and their
+    gradients (2 x 3078 floats per row) and two bf16 layers are 236 MB; 64 chunks
+    of weight gradients would be 539 MB more.  96 MB are left for
+    the allocator's blocks, and 64 MB are the bound on the chunks."""
+    import torch
+    from pqgb300.costmodel import CostModel
+
+    m = CostModel(be, hidden=1024, layers=3, seed=0)
+    X = np.random.default_rng(0).standard_normal((8192, 5)).astype(np.float32)
+    free = [torch.cuda.mem_get_info()[0]]
+    m.predict(X, bf16=False)
+    free.append(torch.cuda.mem_get_info()[0])
+    m.gradients(X, X[:, 0].copy())
+    free.append(torch.cuda.mem_get_info()[0])
+    m.close()
+    assert free[0] - free[1] < 332e6
+    assert free[1] - free[2] < 160e6
+
+
+@pytest.mark.parametrize("n,hidden,layers", [(8193, 600, 2), (1500, 1500, 2)])
+def test_mlp_gradients_few_chunks(pq, be, n, hidden, layers):
+    """Models whose gradients allow fewer than 64 chunks of rows (43 and 7), FP32
+    against FP64: at most 224 rows to a chunk, 1500-wide products twice through
+    2 layers and back and 43 chunks are under 6500 roundings, 3.9e-4 of sums of
+    absolute values of order the largest gradient."""
+    import mlp_oracle as MO
+    from pqgb300.costmodel import CostModel
+
+    m = CostModel(be, hidden=hidden, layers=layers, seed=n)
+    rng = np.random.default_rng(n)
+    X = rng.standard_normal((n, 5)).astype(np.float32)
+    y = rng.standard_normal(n).astype(np.float32)
+    g, loss = m.gradients(X, y)
+    lo, go = MO.loss_and_grad(m.params.astype(np.float64), X, y, 5, hidden, layers)
+    assert abs(loss - lo) <= 1e-5 * max(1.0, abs(lo))
+    assert np.max(np.abs(g - go)) <= 3.9e-4 * max(1.0, np.max(np.abs(go)))
+    m.close()

@@ -279,6 +279,13 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float
   p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
+
+// Gradients of up to this many bytes are read back through a pinned buffer of
+// the handle: a copy into the caller's pageable memory is staged and waited
+// for inside the driver (136 KB of gradients, batch of 1024: 92 -> 88 us).  Larger
+// ones, where the copy itself is the time, go straight to the caller.
+constexpr size_t kPinnedGrad = 1 << 20;
+
 }  // namespace
 
 struct pq_mlp {
@@ -289,6 +296,7 @@ struct pq_mlp {
   int64_t n_params = 0;
   float* d_p = nullptr;
   float* d_g = nullptr;  // gradients, then the loss (read together)
+  float* h_g = nullptr;  // pinned host copy of d_g (small models)
   float* d_m = nullptr;
   float* d_v = nullptr;
   int64_t step = 0;
@@ -464,6 +472,8 @@ int pq_mlp_create(pq_ctx* c, int n_in, int hidden, int hidden_layers, uint64_t s
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_v, sizeof(float) * m->n_params);
   if (e == cudaSuccess) m->d_loss = m->d_g + m->n_params;
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->d_wbf, sizeof(__nv_bfloat16) * m->n_params);
+  const size_t gbytes = sizeof(float) * ((size_t)m->n_params + 1);
+  if (e == cudaSuccess && gbytes <= kPinnedGrad) e = cudaHostAlloc((void**)&m->h_g, gbytes, cudaHostAllocDefault);
   if (e == cudaSuccess) e = cudaMemcpy(m->d_p, h.data(), sizeof(float) * m->n_params, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(m->d_m, 0, sizeof(float) * m->n_params);
   if (e == cudaSuccess) e = cudaMemset(m->d_v, 0, sizeof(float) * m->n_params);
@@ -473,6 +483,7 @@ int pq_mlp_create(pq_ctx* c, int n_in, int hidden, int hidden_layers, uint64_t s
     cudaFree(m->d_m);
     cudaFree(m->d_v);
     cudaFree(m->d_wbf);
+    if (m->h_g) cudaFreeHost(m->h_g);
     delete m;
     return cuda_fail(ctx, e, "mlp create");
   }
@@ -490,6 +501,7 @@ int pq_mlp_destroy(pq_mlp* m) {
   cudaFree(m->d_m);
   cudaFree(m->d_v);
   cudaFree(m->d_wbf);
+  if (m->h_g) cudaFreeHost(m->h_g);
   delete m;
   return PQ_OK;
 }
@@ -529,11 +541,23 @@ int pq_mlp_gradients(pq_mlp* m, const float* X, const float* y, int64_t n, float
   backward(m, (int)n);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(m->ctx, e, "mlp gradients");
-  std::vector<float> h((size_t)m->n_params + 1);
-  st = download(m->ctx, h.data(), m->d_g, sizeof(float) * h.size(), "mlp gradients");
+  // through the handle's pinned buffer where it has one (kPinnedGrad)
+  const size_t bytes = sizeof(float) * (size_t)m->n_params;
+  float l = 0;
+  if (m->h_g) {
+    e = cudaMemcpyAsync(m->h_g, m->d_g, bytes + sizeof(float), cudaMemcpyDeviceToHost, s);
+  } else {
+    e = cudaMemcpyAsync(grad, m->d_g, bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&l, m->d_loss, sizeof(float), cudaMemcpyDeviceToHost, s);
+  }
+  if (e != cudaSuccess) return cuda_fail(m->ctx, e, "mlp gradients");
+  st = check_status(m->ctx);
   if (st) return st;
-  std::memcpy(grad, h.data(), sizeof(float) * m->n_params);
-  if (loss) *loss = h[(size_t)m->n_params];
+  if (m->h_g) {
+    std::memcpy(grad, m->h_g, bytes);
+    l = m->h_g[m->n_params];
+  }
+  if (loss) *loss = l;
   return PQ_OK;
 }
 

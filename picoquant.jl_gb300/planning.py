@@ -377,10 +377,11 @@ def slice_range(total, rank, world):
 def bitstrings_to_index(bitstrings):
     """Column-major linear index of each bitstring (character i -> bit i)."""
     bitstrings = list(bitstrings)
-    n = len(bitstrings[0]) if bitstrings else 0
+    n = len(bitstrings[0]) if bitstrings and isinstance(bitstrings[0], str) else 0
     if 0 < n < 63 and all(isinstance(b, str) and len(b) == n for b in bitstrings):
         # one array pass (1024 strings of 20: 0.1 ms, character by character 0.9 ms)
-        ones = np.frombuffer("".join(bitstrings).encode("utf-32-le"), dtype="<u4").reshape(-1, n) == ord("1")
+        chars = np.frombuffer("".join(bitstrings).encode("utf-32-le", "surrogatepass"), dtype="<u4")
+        ones = chars.reshape(-1, n) == ord("1")
         return ones @ (np.int64(1) << np.arange(n, dtype=np.int64))
     out = np.empty(len(bitstrings), dtype=np.int64)
     for j, b in enumerate(bitstrings):

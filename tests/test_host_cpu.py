@@ -536,3 +536,15 @@ def test_backend_rejects_unknown_svd_mode(pq):
     refused before the library is touched."""
     with pytest.raises(ValueError):
         pq.GB300Backend(pq.PREC_C64, svd="gpu")
+
+
+def test_bitstrings_to_index_forms(pq):
+    """Every sequence of characters counts its "1"s, whatever else it holds: the
+    array pass over equal-length strings accepts what the loop over characters
+    does."""
+    f = pq.bitstrings_to_index
+    cases = [["0110", "1111"], ["01", "011", ""], [["0", "1"], ("1", "1")], ["x1\ud800", "1\u00e91"], ["1" * 62, "0" * 62],
+             ["1" * 63], [], ("10", "01"), np.array(["011", "110"])]
+    for c in cases:
+        assert f(c).tolist() == [sum(1 << i for i, ch in enumerate(b) if ch == "1") for b in c]
+    assert f([iter("01"), iter("11")]).tolist() == [2, 3]

@@ -692,3 +692,43 @@ def test_ozaki_half_split_keeps_small_slices(pq, k, n):
         return np.sqrt(np.mean((np.abs(x - ref) / scale) ** 2))
 
     assert rms(got[:48].astype(np.clongdouble)) <= 2 * rms(Z.accumulate(A, B, True).astype(np.complex64))
+
+
+@pytest.mark.parametrize("prec", [2, 4], ids=["3xtf32", "6xtf32"])
+@pytest.mark.parametrize("m,n,k,z", [
+    (300, 128, 36, 1),   # two whole column tiles, every row of C on a 32-byte boundary
+    (300, 127, 33, 1),   # rows of C on 8-byte boundaries only
+    (400, 68, 20, 3),    # a ragged column tile of four, batched
+    (400, 70, 20, 2),    # the last group of four half outside N; rows on 16-byte boundaries
+    (500, 65, 48, 2),    # one column past the tile
+])
+def test_tf32_columns_adjacent_in_result(pq, prec, m, n, k, z):
+    """The result stored with B's free index fastest (a plan's requested order),
+    where four adjacent columns leave as one 32-byte store if aligned.  An
+    element is within 2^-20 of |row of A| |column of B| (TF32 terms of an operand
+    are exact to 2^-22, a chunk of 16 takes a few truncations of 2^-23)."""
+    import ctypes as C
+    from pqgb300 import _lib as L
+
+    rng = np.random.default_rng(m + n + k + z)
+    A = rand(rng, (m, k, z)).astype(np.complex64)
+    B = rand(rng, (k, n, z)).astype(np.complex64)
+    be = pq.GB300Backend(prec, small_elems=0)
+    be.save_tensor_data("a", A)
+    be.save_tensor_data("b", B)
+    h = C.c_void_p()
+    rc = be.lib.pq_plan_create(be.ctx, 2, L.arr(C.c_int32, [3, 3]), L.arr(C.c_int32, [0, 1, 3, 1, 2, 3]), 4,
+                               L.arr(C.c_int64, [m, k, n, z]), 1, L.arr(C.c_int32, [0, 1]), 3,
+                               L.arr(C.c_int32, [2, 0, 3]), C.byref(h))
+    L.check(rc, be.ctx, "plan_create")
+    ids = L.arr(C.c_int64, [be.id_of("a"), be.id_of("b")])
+    n0 = be.launch_count()
+    L.check(be.lib.pq_plan_execute(h, ids, be.id_of("r")), be.ctx, "execute")
+    assert be.launch_count() - n0 == TC_LAUNCHES
+    got = be.load_tensor_data("r")
+    be.lib.pq_plan_destroy(h)
+    be.close()
+    A, B = A.astype(np.complex128), B.astype(np.complex128)
+    for iz in range(z):
+        bound = np.outer(np.linalg.norm(A[:, :, iz], axis=1), np.linalg.norm(B[:, :, iz], axis=0))
+        assert np.all(np.abs(got[:, :, iz].T - A[:, :, iz] @ B[:, :, iz]) <= 2.0 ** -20 * bound)

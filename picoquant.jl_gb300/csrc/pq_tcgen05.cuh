@@ -103,19 +103,10 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
-// Shared-memory matrix descriptor: no swizzle, K-major canonical layout
-// (8-row x 16-byte core matrices; lbo = K-adjacent core stride, sbo =
-// 8-row-group stride).  The start address field is the low 14 bits, so a
-// later byte offset o within shared memory is added as o >> 4.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
-  d |= (uint64_t)1 << 46;  // descriptor version for sm_100-family tcgen05
-  return d;                // base offset 0, no swizzle (layout type 0)
-}
-// The same from an address in 16-byte units, for the low word alone.
+// Shared-memory matrix descriptor from an address in 16-byte units: no
+// swizzle, K-major canonical layout (8-row x 16-byte core matrices; lbo =
+// K-adjacent core stride, sbo = 8-row-group stride, both in bytes), descriptor
+// version 1 (sm_100-family tcgen05) in bit 46.
 __device__ __forceinline__ uint64_t desc_at(uint32_t addr16, uint32_t lbo, uint32_t sbo) {
   const uint32_t lo = addr16 | (lbo >> 4) << 16, hi = (sbo >> 4) | 1u << 14;
   uint64_t d;

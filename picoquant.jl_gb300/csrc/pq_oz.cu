@@ -138,10 +138,12 @@ struct Sl {
 // Converter warps (the rest are epilogue warps): 12 for 16- and 32-wide tiles of
 // complex64 A in fp16 slices, whose few MMAs wait for A's loads -- a third
 // group of converters keeps half as much again in flight (2^20 x 16 x 256: 0.9 ->
-// 0.7 ms; a second K tile per thread spilled) -- else 8.
+// 0.7 ms; a second K tile per thread spilled) -- else 8.  Tiles of one or two K
+// tiles, whose stores are their time, keep 8 epilogue warps (2^18 x 32 x 32 in
+// 117 us, 169 with 4).
 template <typename TA, int TN, int S>
-__host__ __device__ constexpr int conv_warps() {
-  return TN <= 32 && Sl<S>::half && sizeof(TA) == 8 ? 12 : 8;
+__host__ __device__ constexpr bool many_converters() {
+  return TN <= 32 && Sl<S>::half && sizeof(TA) == 8;
 }
 // kHalf: scaled values are held times 2^kHalfUp, so that the lowest bits of
 // the last slice stay in fp16's range (its subnormals, 2^-24, are 2^-39).
@@ -663,7 +665,7 @@ __device__ __forceinline__ void next_stage(int& s, uint32_t& ph, int by = 1) {
   }
 }
 
-template <typename TA, typename TC, int TN, int S>
+template <typename TA, typename TC, int TN, int S, int CONV>
 __global__ void __launch_bounds__(kThreads, 1)
     k_oz_gemm(const TA* __restrict__ A, const uint16_t* __restrict__ pb, TC* __restrict__ C,
               const __grid_constant__ GemmDesc d, const int64_t* __restrict__ cm_tab,
@@ -675,7 +677,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   constexpr int kAStages = CF::a_stages, kBStages = CF::b_stages;
   constexpr uint32_t kTmemCols = CF::tmem_cols;
   constexpr int kSets = CF::acc_sets;
-  constexpr int kConvWarps = conv_warps<TA, TN, S>(), kEpiWarps = kWorkWarps - kConvWarps;
+  constexpr int kConvWarps = CONV, kEpiWarps = kWorkWarps - kConvWarps;
   constexpr int kGroupThreads = kRows * TK / conv_values<TA>();  // converters of one K tile
   static_assert(!kPark || kEpiWarps == 8, "epilogue_all counts 8 warps");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -1369,7 +1371,7 @@ void prep_b_tn(const void* X, int tn, uint16_t* planes, int* e, const GemmDesc& 
   else prep_b<T, 16, S>(X, planes, e, d, rtiles, kt, s);
 }
 
-template <typename TA, typename TC, int TN, int S>
+template <typename TA, typename TC, int TN, int S, int CONV>
 cudaError_t oz_gemm_launch(const void* A, const uint16_t* pb, void* C, const GemmDesc& d, const int64_t* cm,
                            const int64_t* cn, const int* ea, const int* eb, const OzLayout& L, int* status,
                            cudaStream_t s) {
@@ -1379,14 +1381,14 @@ cudaError_t oz_gemm_launch(const void* A, const uint16_t* pb, void* C, const Gem
   static bool attr = false;
   if (!attr) {
     cudaError_t e =
-        cudaFuncSetAttribute(k_oz_gemm<TA, TC, TN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_oz_gemm<TA, TC, TN, S, CONV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     attr = true;
   }
   const int64_t tiles = L.mt * L.nt * d.Z;
   const unsigned grid = (unsigned)std::min<int64_t>(tiles, sm_count());
-  k_oz_gemm<TA, TC, TN, S><<<grid, kThreads, smem, s>>>((const TA*)A, pb, (TC*)C, d, cm, cn, ea, eb, L.mt, L.nt, L.kt,
-                                                        k_vector(A, d) ? 1 : 0, status);
+  k_oz_gemm<TA, TC, TN, S, CONV><<<grid, kThreads, smem, s>>>((const TA*)A, pb, (TC*)C, d, cm, cn, ea, eb, L.mt, L.nt,
+                                                              L.kt, k_vector(A, d) ? 1 : 0, status);
   return cudaGetLastError();
 }
 
@@ -1394,10 +1396,16 @@ template <typename TA, typename TC, int S>
 cudaError_t oz_gemm_tn(const void* A, const uint16_t* pb, void* C, const GemmDesc& d, const int64_t* cm,
                        const int64_t* cn, const int* ea, const int* eb, const OzLayout& L, int* status,
                        cudaStream_t s) {
-  if (L.tn == 128) return oz_gemm_launch<TA, TC, 128, S>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
-  if (L.tn == 64) return oz_gemm_launch<TA, TC, 64, S>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
-  if (L.tn == 32) return oz_gemm_launch<TA, TC, 32, S>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
-  return oz_gemm_launch<TA, TC, 16, S>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+  if (L.tn == 128) return oz_gemm_launch<TA, TC, 128, S, 8>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+  if (L.tn == 64) return oz_gemm_launch<TA, TC, 64, S, 8>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+  constexpr int many = many_converters<TA, 32, S>() ? 12 : 8;
+  const bool few = L.kt <= 2;
+  if (L.tn == 32) {
+    if (few) return oz_gemm_launch<TA, TC, 32, S, 8>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+    return oz_gemm_launch<TA, TC, 32, S, many>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+  }
+  if (few) return oz_gemm_launch<TA, TC, 16, S, 8>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+  return oz_gemm_launch<TA, TC, 16, S, many>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
 }
 
 bool eligible_oriented(const GemmDesc& d) {

@@ -45,6 +45,7 @@ constexpr int kSkThreads64 = 64;
 struct SkinnyDesc {
   int64_t R, Z;
   int K, N, nr, nz;
+  int cols;                 // columns per block (blockIdx.z)
   int w64;                  // W is complex128
   int cvec;                 // columns 4i .. 4i + 3 are 32 aligned bytes of C (complex64)
   int64_t rdim[kMaxModes], rsx[kMaxModes], rsc[kMaxModes];
@@ -212,7 +213,8 @@ __global__ void __launch_bounds__(kSkThreads)
     k_skinny_w(const float2* __restrict__ X, const void* __restrict__ W, float2* __restrict__ C,
                const __grid_constant__ SkinnyDesc d) {
   extern __shared__ __align__(16) float w[];  // KMAX * np * 4, zero past K and N
-  const int np = (d.N + 3) / 4 * 2;
+  const int nb = blockIdx.z * d.cols, ne = min(d.N, nb + d.cols);  // this block's columns
+  const int np = (ne - nb + 3) / 4 * 2;
   const int64_t step = (int64_t)gridDim.x * kSkThreads;
   for (int64_t z = blockIdx.y; z < d.Z; z += gridDim.y) {
     int64_t zx, zw, zc;
@@ -220,7 +222,7 @@ __global__ void __launch_bounds__(kSkThreads)
     if (z != blockIdx.y) __syncthreads();  // the previous W has been read
     for (int t = threadIdx.x; t < KMAX * 2 * np; t += kSkThreads) {
       const int k = t / (2 * np), n = t - k * (2 * np);
-      w_store(w, np, k, n, w_value<float>(d, W, zw, k, n));
+      w_store(w, np, k, n, w_value<float>(d, W, zw, k, nb + n));
     }
     __syncthreads();
     for (int64_t r = (int64_t)blockIdx.x * kSkThreads + threadIdx.x; r < d.R; r += step) {
@@ -230,9 +232,9 @@ __global__ void __launch_bounds__(kSkThreads)
       load_row<KMAX, KV>(d, X + zx + xo, ax, ay);
       float2* c = C + zc + co;
 #pragma unroll 1
-      for (int n0 = 0; n0 < d.N; n0 += 4) {
+      for (int n0 = nb; n0 < ne; n0 += 4) {
         float2 o[4];
-        four_columns<KMAX>(ax, ay, w, np, n0, o);
+        four_columns<KMAX>(ax, ay, w, np, n0 - nb, o);
         if (d.cvec) {
           asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(c + d.cn[n0]), "f"(o[0].x), "f"(o[0].y),
                        "f"(o[1].x), "f"(o[1].y), "f"(o[2].x), "f"(o[2].y), "f"(o[3].x), "f"(o[3].y)
@@ -240,7 +242,7 @@ __global__ void __launch_bounds__(kSkThreads)
         } else {
 #pragma unroll
           for (int n = 0; n < 4; ++n)
-            if (n0 + n < d.N) c[d.cn[n0 + n]] = o[n];
+            if (n0 + n < ne) c[d.cn[n0 + n]] = o[n];
         }
       }
     }
@@ -254,16 +256,17 @@ __global__ void __launch_bounds__(kSkThreads64)
              const __grid_constant__ SkinnyDesc d) {
   using R = typename std::conditional<std::is_same<TC, double2>::value, double, float>::type;
   using R2 = typename Acc<R>::C;
-  // W[k][n] at w[k * nw + n], zero past K and N (nw a multiple of four)
+  // W[k][n] of this block's columns at w[k * nw + n], zero past K and N (nw a multiple of four)
   extern __shared__ __align__(16) unsigned char w_raw[];
   R2* w = reinterpret_cast<R2*>(w_raw);
-  const int nw = (d.N + 3) / 4 * 4;
+  const int nb = blockIdx.z * d.cols, ne = min(d.N, nb + d.cols);
+  const int nw = (ne - nb + 3) / 4 * 4;
   const int64_t step = (int64_t)gridDim.x * kSkThreads64;
   for (int64_t z = blockIdx.y; z < d.Z; z += gridDim.y) {
     int64_t zx, zw, zc;
     batch_offsets(d, z, zx, zw, zc);
     if (z != blockIdx.y) __syncthreads();  // the previous W has been read
-    for (int t = threadIdx.x; t < KMAX * nw; t += kSkThreads64) w[t] = w_value<R>(d, W, zw, t / nw, t % nw);
+    for (int t = threadIdx.x; t < KMAX * nw; t += kSkThreads64) w[t] = w_value<R>(d, W, zw, t / nw, nb + t % nw);
     __syncthreads();
     for (int64_t r = (int64_t)blockIdx.x * kSkThreads64 + threadIdx.x; r < d.R; r += step) {
       int64_t xo, co;
@@ -273,21 +276,22 @@ __global__ void __launch_bounds__(kSkThreads64)
       R2 a[KMAX];
 #pragma unroll
       for (int k = 0; k < KMAX; ++k) a[k] = k < d.K ? cvt<R>(__ldg(X + xo + d.kx[k])) : czero(R());
+      constexpr int CG = 4;
 #pragma unroll 1
-      for (int n0 = 0; n0 < d.N; n0 += 4) {
-        R2 acc[4];
+      for (int n0 = nb; n0 < ne; n0 += CG) {
+        R2 acc[CG];
 #pragma unroll
-        for (int n = 0; n < 4; ++n) acc[n] = czero(R());
+        for (int n = 0; n < CG; ++n) acc[n] = czero(R());
 #pragma unroll
         for (int k = 0; k < KMAX; ++k) {
           if (k < d.K) {  // (uniform: no FP64 time for padding)
 #pragma unroll
-            for (int n = 0; n < 4; ++n) cfma(acc[n], a[k], w[k * nw + n0 + n]);
+            for (int n = 0; n < CG; ++n) cfma(acc[n], a[k], w[k * nw + n0 - nb + n]);
           }
         }
 #pragma unroll
-        for (int n = 0; n < 4; ++n)
-          if (n0 + n < d.N) C[co + d.cn[n0 + n]] = store_as<TC>(acc[n]);
+        for (int n = 0; n < CG; ++n)
+          if (n0 + n < ne) C[co + d.cn[n0 + n]] = store_as<TC>(acc[n]);
       }
     }
   }
@@ -404,29 +408,45 @@ dim3 sk_grid(const SkinnyDesc& d, int per_sm, int threads = kSkThreads) {
   const int64_t x = std::max<int64_t>(1, 152 * per_sm / y);
   return dim3((unsigned)std::min<int64_t>((d.R + threads - 1) / threads, x), (unsigned)y);
 }
+// The columns, `unit` at a time, in as many groups as leave every SM four blocks
+// where the rows alone do not (4096 rows, N = 128, K = 16: 43 us on 32 blocks, 11
+// on 1024).
+dim3 split_columns(SkinnyDesc& d, dim3 g, int unit) {
+  const int units = (d.N + unit - 1) / unit;
+  const int64_t want = std::max<int64_t>(1, 4 * 152 / ((int64_t)g.x * g.y));
+  const int per = (int)std::max<int64_t>(1, units / std::min<int64_t>(units, want));
+  d.cols = unit * per;
+  g.z = (unsigned)((units + per - 1) / per);
+  return g;
+}
 
-template <typename TX, typename TC>
-cudaError_t launch_mixed(const void* X, const void* W, void* C, const SkinnyDesc& d, cudaStream_t s) {
-  const size_t col = (size_t)((d.N + 3) / 4 * 4) * (std::is_same<TC, double2>::value ? 16 : 8);
-  if (d.K <= 4)
-    k_skinny<TX, TC, 4><<<sk_grid(d, 18, kSkThreads64), kSkThreads64, 4 * col, s>>>((const TX*)X, W, (TC*)C, d);
-  else
-    k_skinny<TX, TC, 16><<<sk_grid(d, 9, kSkThreads64), kSkThreads64, 16 * col, s>>>((const TX*)X, W, (TC*)C, d);
+template <typename TX, typename TC, int KMAX>
+cudaError_t launch_mixed_k(const void* X, const void* W, void* C, SkinnyDesc& d, int per_sm, cudaStream_t s) {
+  dim3 grid = sk_grid(d, per_sm, kSkThreads64);
+  grid = split_columns(d, grid, 4);
+  const size_t smem = (size_t)KMAX * ((d.cols + 3) / 4 * 4) * (std::is_same<TC, double2>::value ? 16 : 8);
+  k_skinny<TX, TC, KMAX><<<grid, kSkThreads64, smem, s>>>((const TX*)X, W, (TC*)C, d);
   return cudaGetLastError();
+}
+template <typename TX, typename TC>
+cudaError_t launch_mixed(const void* X, const void* W, void* C, SkinnyDesc& d, cudaStream_t s) {
+  return d.K <= 4 ? launch_mixed_k<TX, TC, 4>(X, W, C, d, 18, s) : launch_mixed_k<TX, TC, 16>(X, W, C, d, 9, s);
 }
 
 template <int KMAX, int KV>
-cudaError_t launch_kv(const void* X, const void* W, void* C, const SkinnyDesc& d, cudaStream_t s) {
-  const dim3 grid = sk_grid(d, KMAX == 16 ? 8 : 10);
-  if (d.N <= 16 && d.Z == 1 && !d.cvec)
+cudaError_t launch_kv(const void* X, const void* W, void* C, SkinnyDesc& d, cudaStream_t s) {
+  dim3 grid = sk_grid(d, KMAX == 16 ? 8 : 10);
+  if (d.N <= 16 && d.Z == 1 && !d.cvec) {
     k_skinny_f<KMAX, KV><<<grid, kSkThreads, 0, s>>>((const float2*)X, W, (float2*)C, d);
-  else
-    k_skinny_w<KMAX, KV><<<grid, kSkThreads, (size_t)KMAX * ((d.N + 3) / 4 * 2) * 16, s>>>((const float2*)X, W,
-                                                                                             (float2*)C, d);
+  } else {
+    grid = split_columns(d, grid, 4);
+    const size_t smem = (size_t)KMAX * (d.cols / 2) * 16;
+    k_skinny_w<KMAX, KV><<<grid, kSkThreads, smem, s>>>((const float2*)X, W, (float2*)C, d);
+  }
   return cudaGetLastError();
 }
 template <int KMAX>
-cudaError_t launch_k(int kv, const void* X, const void* W, void* C, const SkinnyDesc& d, cudaStream_t s) {
+cudaError_t launch_k(int kv, const void* X, const void* W, void* C, SkinnyDesc& d, cudaStream_t s) {
   if (kv == 4) return launch_kv<KMAX, 4>(X, W, C, d, s);
   if (kv == 2) return launch_kv<KMAX, 2>(X, W, C, d, s);
   return launch_kv<KMAX, 1>(X, W, C, d, s);

@@ -287,3 +287,36 @@ def test_skinny_wide_and_batched(pq, m, k, n, z, order, swap):
     ref = np.einsum(expr, X.astype(np.complex128), W.astype(np.complex128))
     bound = 2 * (k + 2) * 2.0 ** -24 * np.einsum(expr, np.abs(X), np.abs(W))
     assert np.all(np.abs(got - ref) <= bound)
+
+
+@pytest.mark.parametrize("m,k,n,z", [(4096, 16, 128, 1), (4100, 7, 127, 1), (4097, 1, 66, 1), (130, 16, 5, 40), (512, 16, 18, 8),
+                                     (33000, 3, 1, 2), (70001, 16, 3, 1), (150000, 9, 8, 1), (2050, 4, 6, 2)])
+@pytest.mark.parametrize("small", [0, 1 << 62], ids=["c64", "c128"])
+def test_skinny_column_groups(pq, m, k, n, z, small):
+    """Few rows against many columns (the columns split over blocks), groups whose
+    last has fewer than four columns, and rows that the blocks take in equal
+    rounds; complex64 and complex128 operands and results.  Bound as for single
+    pairs, with the unit roundoff of the results' type."""
+    from pqgb300 import _lib as L
+
+    rng = np.random.default_rng(m + k + n + z)
+    dt = np.complex128 if small else np.complex64
+    X = (rng.standard_normal((m, k, z)) + 1j * rng.standard_normal((m, k, z))).astype(dt)
+    W = (rng.standard_normal((k, n, z)) + 1j * rng.standard_normal((k, n, z))).astype(dt)
+    be = pq.GB300Backend(pq.PREC_C64, small_elems=small)
+    be.save_tensor_data("a", X)
+    be.save_tensor_data("b", W)
+    h = C.c_void_p()
+    L.check(be.lib.pq_plan_create(be.ctx, 2, L.arr(C.c_int32, [3, 3]), L.arr(C.c_int32, [0, 1, 3, 1, 2, 3]), 4,
+                                  L.arr(C.c_int64, [m, k, n, z]), 1, L.arr(C.c_int32, [0, 1]), 3,
+                                  L.arr(C.c_int32, [0, 2, 3]), C.byref(h)), be.ctx, "plan_create")
+    f = (C.c_double * 8)()
+    L.check(be.lib.pq_plan_step_features(h, f), be.ctx, "features")
+    assert int(f[6]) == KC_SKINNY
+    L.check(be.lib.pq_plan_execute(h, L.arr(C.c_int64, [be.id_of("a"), be.id_of("b")]), be.id_of("r")), be.ctx, "run")
+    got = be.load_tensor_data("r", dtype=dt)
+    be.lib.pq_plan_destroy(h)
+    be.close()
+    ref = np.einsum("mkz,knz->mnz", X.astype(np.complex128), W.astype(np.complex128))
+    bound = 2 * (k + 2) * (2.0 ** -53 if small else 2.0 ** -24) * np.einsum("mkz,knz->mnz", np.abs(X), np.abs(W))
+    assert np.all(np.abs(got - ref) <= 2 * bound if small else np.abs(got - ref) <= bound)

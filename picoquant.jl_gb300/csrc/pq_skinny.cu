@@ -249,8 +249,9 @@ __global__ void __launch_bounds__(kSkThreads)
   }
 }
 
-// Every other mix of element types (complex128 results in FP64).
-template <typename TX, typename TC, int KMAX>
+// Every other mix of element types (complex128 results in FP64).  ONE: a column
+// at a time, else four (padded: 2^18 rows, N = 1, K = 4 in 35 us so, 13 with ONE).
+template <typename TX, typename TC, int KMAX, bool ONE>
 __global__ void __launch_bounds__(kSkThreads64)
     k_skinny(const TX* __restrict__ X, const void* __restrict__ W, TC* __restrict__ C,
              const __grid_constant__ SkinnyDesc d) {
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(kSkThreads64)
       R2 a[KMAX];
 #pragma unroll
       for (int k = 0; k < KMAX; ++k) a[k] = k < d.K ? cvt<R>(__ldg(X + xo + d.kx[k])) : czero(R());
-      constexpr int CG = 4;
+      constexpr int CG = ONE ? 1 : 4;
 #pragma unroll 1
       for (int n0 = nb; n0 < ne; n0 += CG) {
         R2 acc[CG];
@@ -423,9 +424,15 @@ dim3 split_columns(SkinnyDesc& d, dim3 g, int unit) {
 template <typename TX, typename TC, int KMAX>
 cudaError_t launch_mixed_k(const void* X, const void* W, void* C, SkinnyDesc& d, int per_sm, cudaStream_t s) {
   dim3 grid = sk_grid(d, per_sm, kSkThreads64);
-  grid = split_columns(d, grid, 4);
+  // single columns where four would be padded, and where the rows are few (4096,
+  // N = 4, K = 16: 14 -> 10 us)
+  const bool one = d.N < 4 || (d.N < 16 && (int64_t)grid.x * grid.y <= 152);
+  grid = split_columns(d, grid, one ? 1 : 4);
   const size_t smem = (size_t)KMAX * ((d.cols + 3) / 4 * 4) * (std::is_same<TC, double2>::value ? 16 : 8);
-  k_skinny<TX, TC, KMAX><<<grid, kSkThreads64, smem, s>>>((const TX*)X, W, (TC*)C, d);
+  if (one)
+    k_skinny<TX, TC, KMAX, true><<<grid, kSkThreads64, smem, s>>>((const TX*)X, W, (TC*)C, d);
+  else
+    k_skinny<TX, TC, KMAX, false><<<grid, kSkThreads64, smem, s>>>((const TX*)X, W, (TC*)C, d);
   return cudaGetLastError();
 }
 template <typename TX, typename TC>

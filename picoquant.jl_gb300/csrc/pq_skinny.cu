@@ -406,7 +406,10 @@ cudaError_t launch_tall_kv(const void* X, const void* W, void* C, const TallDesc
 // below; FP64: 96).
 dim3 sk_grid(const SkinnyDesc& d, int per_sm, int threads = kSkThreads) {
   const int64_t y = std::min<int64_t>(d.Z, 65535);
-  const int64_t x = std::max<int64_t>(1, 152 * per_sm / y);
+  // (a few blocks per batch index would leave a part of the chip out or over:
+  // four rounds of smaller ones; 2^15 rows, N = 1, K = 2, Z = 512: 157
+  // -> 129 us)
+  const int64_t fit = 152 * per_sm / y, x = std::max<int64_t>(1, fit >= 8 ? fit : 4 * 152 * per_sm / y);
   return dim3((unsigned)std::min<int64_t>((d.R + threads - 1) / threads, x), (unsigned)y);
 }
 // The columns, `unit` at a time, in as many groups as leave every SM four blocks

@@ -81,9 +81,9 @@
 //                  next K tile in flight while this one is sliced), slice
 //                  them and store the [Ar; Ai; -Ar] stacks into A's ring (no
 //                  slice planes of A ever reach HBM); for complex64 A two
-//                  groups of four warps take alternate K tiles, each thread
-//                  8 consecutive k of one row, so every store is a whole
-//                  16-byte core-matrix row;
+//                  or three groups of four warps take K tiles in turn, each
+//                  thread 8 consecutive k of one row, so every store is a
+//                  whole 16-byte core-matrix row;
 //     8 or 4 warps  epilogue, once per tile: Cr from TMEM lanes 0-63, Ci from
 //                  lanes 64-127; the levels are combined with an error-free
 //                  two-sum (128-wide complex64 tiles park the sums, in shared
@@ -135,15 +135,16 @@ struct Sl {
     return half ? (i == 0 ? 4 : (i == 3 ? 1 : 3)) : n - i;
   }
 };
-// Converter warps (the rest are epilogue warps): 12 for 16- and 32-wide tiles of
-// complex64 A in fp16 slices, whose few MMAs wait for A's loads -- a third
-// group of converters keeps half as much again in flight (2^20 x 16 x 256: 0.9 ->
-// 0.7 ms; a second K tile per thread spilled) -- else 8.  Tiles of one or two K
-// tiles, whose stores are their time, keep 8 epilogue warps (2^18 x 32 x 32 in
-// 117 us, 169 with 4).
+// Converter warps (the rest are epilogue warps): 8; 12 for 16-wide tiles of more
+// than six K tiles of complex64 A in fp16 slices, whose few MMAs wait for A's
+// loads -- a third group of converters keeps half as much again in flight
+// (2^18 rows, N = 16, K = 256: 337 -> 306 us; a second K tile per thread
+// spilled).  Shorter tiles wait for their stores (K = 64: 142 us with 12, 125
+// with 8), 32-wide ones for their MMAs (K = 48: 180 and 134 us, K = 256: 357 and
+// 354).
 template <typename TA, int TN, int S>
 __host__ __device__ constexpr bool many_converters() {
-  return TN <= 32 && Sl<S>::half && sizeof(TA) == 8;
+  return TN == 16 && Sl<S>::half && sizeof(TA) == 8;
 }
 // kHalf: scaled values are held times 2^kHalfUp, so that the lowest bits of
 // the last slice stay in fp16's range (its subnormals, 2^-24, are 2^-39).
@@ -1398,14 +1399,10 @@ cudaError_t oz_gemm_tn(const void* A, const uint16_t* pb, void* C, const GemmDes
                        cudaStream_t s) {
   if (L.tn == 128) return oz_gemm_launch<TA, TC, 128, S, 8>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
   if (L.tn == 64) return oz_gemm_launch<TA, TC, 64, S, 8>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
-  constexpr int many = many_converters<TA, 32, S>() ? 12 : 8;
-  const bool few = L.kt <= 2;
-  if (L.tn == 32) {
-    if (few) return oz_gemm_launch<TA, TC, 32, S, 8>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
-    return oz_gemm_launch<TA, TC, 32, S, many>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
-  }
-  if (few) return oz_gemm_launch<TA, TC, 16, S, 8>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
-  return oz_gemm_launch<TA, TC, 16, S, many>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+  if (L.tn == 32) return oz_gemm_launch<TA, TC, 32, S, 8>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+  if (many_converters<TA, 16, S>() && L.kt > 6)
+    return oz_gemm_launch<TA, TC, 16, S, many_converters<TA, 16, S>() ? 12 : 8>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
+  return oz_gemm_launch<TA, TC, 16, S, 8>(A, pb, C, d, cm, cn, ea, eb, L, status, s);
 }
 
 bool eligible_oriented(const GemmDesc& d) {

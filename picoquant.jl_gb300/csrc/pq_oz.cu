@@ -158,13 +158,13 @@ constexpr int kHalfUp = 15;
 __host__ __device__ constexpr int first_bits(int64_t k, int side) { return k <= (side == 0 ? 128 : 256) ? 8 : 7; }
 __host__ __device__ constexpr int second_bits(int64_t k) { return k <= 128 ? 8 : 7; }
 
-// 128-wide tiles of kHalf or three slices with complex64 results: the epilogue parks a
-// tile's sums in shared memory (and stores whole complex values from there),
-// and the fourth TMEM block lets the next tile's MMAs of levels 2 and up start
-// before the epilogue has read this one.  Against parking in the fourth block
-// the issuer's wait for the epilogue fell from 17 % of its time to 1 %: 24.3k ->
-// 21.6k cycles per 64 x 128 x 256 tile, with the ring cut from five stages to
-// three.
+// 128-wide tiles of kHalf or three slices with complex64 results: the epilogue
+// parks a tile's sums in shared memory (and stores whole complex values from
+// there), and the fourth TMEM block lets the next tile's MMAs of levels 2 and up
+// start before the epilogue has read this one.  Against parking in the fourth
+// block with a ring of three stages (kHalf): 2^20 x 256 x 16 in 1.44 instead of
+// 2.36 ms, 2^18 x 128 x 64 in 0.27 instead of 0.39; K = 256, where two stages of
+// A are the price, 4.26 instead of 4.17.
 template <typename TC, int TN, int S>
 __host__ __device__ constexpr bool oz_park() {
   return TN == 128 && (Sl<S>::half || S == 3) && sizeof(TC) == 8;
@@ -207,7 +207,7 @@ __host__ __device__ constexpr int narrow_col(int i) {
 // Slice pairs, level 0 first, then level 1, then the rest with the smallest
 // first.  The order in which the bf16 splits issue them (the truncating rest
 // accumulator then takes the fewest additions at full size: by slice of A from
-// the first its rms error is 5 to 20 % larger, K = 512 to 32), and in which the
+// the first its rms error is 5 to 17 % larger, K = 512 to 64), and in which the
 // epilogue of 16-wide tiles adds the pairs' regions up.  Five slices:
 //   i: 0 0 1 0 1 2 3 4 0 1 2 3 0 1 2
 //   j: 0 1 0 4 3 2 1 0 3 2 1 0 2 1 0
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(256) k_oz_exp_k(const T* __restrict__ X, const
 // value, which coalesces over rows when A's first M mode has stride 1; over rows
 // 128 bytes apart it costs the converters a wavefront of the L1 per row and
 // value, 88 % of its rate (2^20 x 256 x 256 with runs of 16, exponent pass
-// included: 3.35 ms value by value, 2.75 so).
+// included: 3.35 ms value by value, 2.75 so, with 8 products per pair).
 bool k_vector(const void* A, const GemmDesc& d) {
   if (((uintptr_t)A & 31) || d.nk < 1 || d.ksa[0] != 1) return false;
   int64_t run = d.kdim[0];
@@ -1147,7 +1147,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // without a branch, so that the columns' loads and stores overlap: with
         // two branches per column (zero row, scale outside the normal range)
         // this phase took 275 cycles per column and 82 % of a tile of one K tile
-        // (2^20 x 256 x 16 with the exponent pass: 1.31 -> 0.77 ms).
+        // (2^20 x 256 x 16 with the exponent pass, 8 products: 1.31 -> 0.77 ms).
         const int emin = __reduce_min_sync(0xffffffffu, M.ebl[0]), emax = __reduce_max_sync(0xffffffffu, M.ebl[0]);
         const bool plain = !mrow || (exa + emin - kDown >= -126 && exa + emax - kDown <= 127);
         if (__all_sync(0xffffffffu, plain && ncol == SW)) {
